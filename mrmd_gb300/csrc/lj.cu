@@ -1,9 +1,9 @@
 // action::LennardJones: capped, optionally shifted LJ on a half Verlet list.
 //
-// FP64 form: one thread per local atom i (atoms are cell-sorted by the
-// stepper, so a warp's neighbours share cache lines), i-force in registers,
-// j-force scattered with FP64 atomics into the 32-byte atom sector, energy
-// and virial reduced per block and added once per block.
+// FP64 form: the j-force is scattered with FP64 atomics into the 32-byte atom
+// sector (atoms are cell-sorted by the stepper, so a warp's neighbours share
+// cache lines), energy and virial are reduced per block and added once per
+// block.
 #include <cmath>
 #include <vector>
 
@@ -70,60 +70,266 @@ void lj_table_host(mrmd_lj_params* out, int64_t numTypes, const double* cap, con
 namespace
 {
 constexpr int LJ_TB = 128;
+constexpr int LJ_CHUNK = 64;  // list entries of a row scanned at a time
+constexpr int LJ_BLOCKS = 5;  // resident blocks per SM: with 6 or 7 the segments take the L1's room
+                              // (4,000,000 atoms: 4.83 ms with 5, 4.89 with 6, 5.03 with 7)
 
-template <bool PRED, bool MULTI>
-__global__ void __launch_bounds__(LJ_TB) k_lj_fp64(
+// Pair force on the half list in two phases per warp, R list rows per warp.
+//
+// The kernel is bound by the FP64 pipe (2 lanes per SM and clock on GB300),
+// so it is laid out to issue as few FP64 instructions as possible, with all
+// 32 lanes busy in each:
+//  1. Scan: the rows' entries are tested against the cutoff in FP32 from the
+//     high words of the coordinates (a lower bound of r^2, half_list_far);
+//     the ones that may be in range (71% with a skin of 0.3 at 2.5) are
+//     appended to their row's segment in shared memory.
+//  2. Evaluation: the segments' pairs, numbered row after row, are dealt out
+//     evenly, so that every lane evaluates the same number of pairs (+-1)
+//     whatever the rows' lengths; a lane keeps the force of its current row
+//     in registers and adds it to the row's atom when it moves on.
+// A pair takes 22 FP64 instructions: distance 3, r^2 3, reciprocal 3, force
+// factor 5, energy and virial sums 2 (of u^3 and u^6; E and W are formed once
+// per lane), forces 6.  The comparisons are integer ones on the bits.
+// One lane per row with all entries in FP64 and a correctly rounded
+// reciprocal took ~35 instructions per entry and, with rows of unequal
+// length, 47 rounds for 38 entries.  At 256,000 atoms 4.91e6 FP64 warp
+// instructions (22 per pair in range are 4.85e6), FP64 pipe 76% active.
+// Measured times: lj_rows_per_warp.
+//
+// The double's leading bits as a float, truncated to 20 fraction bits: below
+// 2^-126 zero, beyond FP32 (and NaN, infinity) NaN.
+__device__ __forceinline__ float hi_word_f32(double x)
+{
+    const uint32_t h = (uint32_t)__double2hiint(x), m = h & 0x7fffffffu;
+    uint32_t b = (m - 0x38000000u) << 3;
+    b = m < 0x38100000u ? 0u : b;
+    b = m >= 0x47f00000u ? 0x7fc00000u : b;
+    return __uint_as_float((h & 0x80000000u) | b);
+}
+
+// True when the pair is certainly beyond the cutoff: per axis the distance
+// of the truncated coordinates less 2^-19 of their magnitudes (the two
+// truncations, 2^-20 each, and the FP32 rounding) bounds the true one from
+// below.  NaN coordinates are never far.
+__device__ __forceinline__ bool half_list_far(float3 a, const double4& pj, float rcSqrUp)
+{
+    constexpr float E = 1.9073486328125e-6f;  // 2^-19
+    const float bx = hi_word_f32(pj.x), by = hi_word_f32(pj.y), bz = hi_word_f32(pj.z);
+    const float dx = fmaxf(__fmaf_rn(-E, fabsf(a.x) + fabsf(bx), fabsf(a.x - bx)), 0.f);
+    const float dy = fmaxf(__fmaf_rn(-E, fabsf(a.y) + fabsf(by), fabsf(a.y - by)), 0.f);
+    const float dz = fmaxf(__fmaf_rn(-E, fabsf(a.z) + fabsf(bz), fabsf(a.z - bz)), 0.f);
+    return __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz)) > rcSqrUp;
+}
+
+// 1/x to about an ulp for x in [2^-340, 2^1000]: the hardware's approximate
+// reciprocal y (relative error below 2^-20) and the geometric series of
+// 1/(1 - e), e = 1 - x y, up to e^2; the rest, e^3, is below 2^-60.
+__device__ __forceinline__ double rcp_series(double x)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = __fma_rn(-x, y, 1.0);
+    return __fma_rn(y, __fma_rn(e, e, e), y);
+}
+
+template <bool PRED, bool MULTI, int R>
+__global__ void __launch_bounds__(LJ_TB, LJ_BLOCKS) k_lj_fp64(
     const double4* __restrict__ pos, double* __restrict__ force, const int32_t* __restrict__ type,
-    const LJDev p0, const LJDev* __restrict__ table, int32_t numTypesIndex, double rcSqr,
+    const LJDev p0, const LJDev* __restrict__ table, int32_t numTypesIndex, double rcSqr, float rcSqrUp,
     const int32_t* __restrict__ counts, const int32_t* __restrict__ nbrs, int64_t cap, int64_t n,
     int64_t begin, int64_t nAll, mrmd_dev::Pred pred, double* __restrict__ ev)
 {
+    constexpr int G = 32 / R;  // lanes scanning one row
+    constexpr unsigned ALL = 0xffffffffu;
+    constexpr unsigned ROW0 = R == 2 ? 0x55555555u : R == 4 ? 0x11111111u : R == 8 ? 0x01010101u : 0x00010001u;  // row 0's lanes
+    static_assert(R == 2 || R == 4 || R == 8 || R == 16, "rows per warp");
+    __shared__ int32_t segS[LJ_TB / 32][LJ_CHUNK * R];
+    __shared__ int32_t endS[LJ_TB / 32][R];
     __shared__ double red[64];
-    double energy = 0.0, virial = 0.0;
-    const int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (row < n)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int32_t* seg = segS[warp];  // entry q of row r: seg[q * R + r]
+    int32_t* ends = endS[warp];
+    // sums over the lane's pairs: u^3, u^6 and the number of uncapped pairs;
+    // energies and force factor * r^2 of the others
+    double s3 = 0.0, s6 = 0.0, sE = 0.0, sW = 0.0;
+    int32_t num = 0;
+    const unsigned long long rcBits = (unsigned long long)__double_as_longlong(rcSqr);
+    const int r = lane % R, g = lane / R;
+    // a warp takes every (number of warps)-th group of R rows
+    for (int64_t row0 = (blockIdx.x * (int64_t)(LJ_TB / 32) + warp) * R; row0 < n;
+         row0 += (int64_t)gridDim.x * (LJ_TB / 32) * R)
     {
-        // list row `row` belongs to particle begin + row (the list's range)
-        const int64_t i = begin + row;
-        const double4 pi = pos[i];
-        double fx = 0.0, fy = 0.0, fz = 0.0;
-        const int32_t cnt = counts[row];
-        const int32_t ti = MULTI ? type[i] * numTypesIndex : 0;
+        const int64_t row = row0 + r;
+        const int32_t cnt = row < n ? counts[row] : 0;
+        int32_t maxCnt = cnt;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) maxCnt = max(maxCnt, __shfl_xor_sync(ALL, maxCnt, o));
+        double4 pr = make_double4(0.0, 0.0, 0.0, 0.0);
+        if (cnt > 0) pr = pos[begin + row];
+        const float3 pf = make_float3(hi_word_f32(pr.x), hi_word_f32(pr.y), hi_word_f32(pr.z));
         const int32_t* __restrict__ col = nbrs + mrmd_dev::nbr_row(row, cap);
-        for (int32_t k = 0; k < cnt; ++k)
+        for (int32_t k0 = 0; k0 < maxCnt; k0 += LJ_CHUNK)
         {
-            const int32_t j = __ldg(col + 32 * (int64_t)k);
-            if (!MRMD_IN_BOUNDS(j, nAll)) continue;
-            const double4 pj = mrmd_dev::ldg4(pos + j);
-            if (PRED && !mrmd_dev::pred2(pred, pi.x, pi.y, pi.z, pj.x, pj.y, pj.z)) continue;
-            const double dx = pi.x - pj.x;
-            const double dy = pi.y - pj.y;
-            const double dz = pi.z - pj.z;
-            const double distSqr = dx * dx + dy * dy + dz * dz;
-            if (distSqr > rcSqr) continue;
-            const LJDev& p = MULTI ? table[ti + type[j]] : p0;
-            double ff, e;
-            lj_eval_fp64(p, distSqr, ff, e);
-            energy += e;
-            virial -= 0.5 * ff * distSqr;
-            const double gx = dx * ff, gy = dy * ff, gz = dz * ff;
-            fx += gx;
-            fy += gy;
-            fz += gz;
-            atomicAdd(force + 4 * (int64_t)j + 0, -gx);
-            atomicAdd(force + 4 * (int64_t)j + 1, -gy);
-            atomicAdd(force + 4 * (int64_t)j + 2, -gz);
+            // 1. scan
+            int32_t c = 0;  // entries of the row kept so far (the same in its G lanes)
+            const int32_t kEnd = min(k0 + LJ_CHUNK, maxCnt);
+#pragma unroll 4
+            for (int32_t kk = k0; kk < kEnd; kk += G)
+            {
+                const int32_t k = kk + g;
+                bool keep = k < cnt;
+                int32_t j = 0;
+                if (keep)
+                {
+                    j = __ldg(col + 32 * (int64_t)k);
+                    keep = MRMD_IN_BOUNDS(j, nAll);
+                    if (keep)
+                    {
+                        const double4 pj = mrmd_dev::ldg4(pos + j);
+                        keep = !half_list_far(pf, pj, rcSqrUp);
+                        if (PRED) keep = keep && mrmd_dev::pred2(pred, pr.x, pr.y, pr.z, pj.x, pj.y, pj.z);
+                    }
+                }
+                const unsigned m = __ballot_sync(ALL, keep) & (ROW0 << r);
+                if (keep) seg[(c + __popc(m & ((1u << lane) - 1u))) * R + r] = j;
+                c += __popc(m);
+            }
+            // 2. evaluation: row r's pairs are numbers [incl - c, incl)
+            int32_t incl = c;
+#pragma unroll
+            for (int o = 1; o < R; o <<= 1)
+            {
+                const int32_t t = __shfl_up_sync(ALL, incl, o, R);
+                if (r >= o) incl += t;
+            }
+            if (g == 0) ends[r] = incl;
+            __syncwarp();
+            const int32_t total = ends[R - 1];
+            int32_t t = (total * lane) >> 5;  // total <= R * LJ_CHUNK
+            const int32_t tEnd = (total * (lane + 1)) >> 5;
+            if (t < tEnd)
+            {
+                int32_t q = 0, qStart = 0, qEnd;  // current row and its numbers
+                {
+                    int lo = 0, hi = R - 1;  // first row that ends above t
+                    while (lo < hi)
+                    {
+                        const int mid = (lo + hi) >> 1;
+                        if (ends[mid] > t) hi = mid;
+                        else lo = mid + 1;
+                    }
+                    q = lo;
+                    qStart = q > 0 ? ends[q - 1] : 0;
+                    qEnd = ends[q];
+                }
+                int64_t i = begin + row0 + q;
+                double4 pi = mrmd_dev::ldg4(pos + i);
+                int32_t ti = MULTI ? type[i] * numTypesIndex : 0;
+                double fx = 0.0, fy = 0.0, fz = 0.0;
+                for (; t < tEnd; ++t)
+                {
+                    if (t >= qEnd)
+                    {
+                        atomicAdd(force + 4 * i + 0, fx);
+                        atomicAdd(force + 4 * i + 1, fy);
+                        atomicAdd(force + 4 * i + 2, fz);
+                        fx = fy = fz = 0.0;
+                        do
+                        {
+                            ++q;
+                            qStart = qEnd;
+                            qEnd = ends[q];
+                        } while (t >= qEnd);
+                        i = begin + row0 + q;
+                        pi = mrmd_dev::ldg4(pos + i);
+                        if (MULTI) ti = type[i] * numTypesIndex;
+                    }
+                    const int64_t j = seg[(t - qStart) * R + q];
+                    const double4 pj = mrmd_dev::ldg4(pos + j);
+                    const double dx = pi.x - pj.x;
+                    const double dy = pi.y - pj.y;
+                    const double dz = pi.z - pj.z;
+                    const double r2 = __fma_rn(dz, dz, __fma_rn(dy, dy, __dmul_rn(dx, dx)));
+                    // bits of a non-negative double order as the value; a NaN's
+                    // lie above infinity's and are not skipped
+                    const unsigned long long b = (unsigned long long)__double_as_longlong(r2);
+                    if (b > rcBits && b <= 0x7ff0000000000000ull) continue;
+                    const LJDev& p = MULTI ? table[ti + type[j]] : p0;
+                    double ff;
+                    if (b >= (unsigned long long)__double_as_longlong(p.capSqr) && b >= 0x2ab0000000000000ull)  // 2^-340
+                    {
+                        const double u = rcp_series(r2);
+                        const double u3 = __dmul_rn(__dmul_rn(u, u), u);
+                        ff = __dmul_rn(__dmul_rn(u3, __fma_rn(p.ff1, u3, -p.ff2)), u);
+                        if (MULTI)
+                        {
+                            sE += __fma_rn(u3, __fma_rn(p.ef1, u3, -p.ef2), -p.shift);
+                            sW = __fma_rn(ff, r2, sW);
+                        }
+                        else
+                        {
+                            s3 += u3;
+                            s6 = __fma_rn(u3, u3, s6);
+                            ++num;
+                        }
+                    }
+                    else
+                    {
+                        double e;
+                        lj_eval_fp64(p, r2, ff, e);
+                        sE += e;
+                        sW = __fma_rn(ff, r2, sW);
+                    }
+                    const double gx = __dmul_rn(dx, -ff), gy = __dmul_rn(dy, -ff), gz = __dmul_rn(dz, -ff);
+                    fx -= gx;
+                    fy -= gy;
+                    fz -= gz;
+                    atomicAdd(force + 4 * j + 0, gx);
+                    atomicAdd(force + 4 * j + 1, gy);
+                    atomicAdd(force + 4 * j + 2, gz);
+                }
+                atomicAdd(force + 4 * i + 0, fx);
+                atomicAdd(force + 4 * i + 1, fy);
+                atomicAdd(force + 4 * i + 2, fz);
+            }
+            __syncwarp();  // the next chunk overwrites the segments
         }
-        atomicAdd(force + 4 * i + 0, fx);
-        atomicAdd(force + 4 * i + 1, fy);
-        atomicAdd(force + 4 * i + 2, fz);
     }
-    mrmd_dev::block_sum2(energy, virial, red);
+    if (!MULTI)
+    {
+        // E = sum ef1 u^6 - ef2 u^3 - shift, -2 W = sum ff1 u^6 - ff2 u^3
+        // (action/LennardJones.hpp:52-78: forceFactor r^2 = ff1 u^6 - ff2 u^3)
+        sE += __fma_rn(p0.ef1, s6, -__fma_rn(p0.ef2, s3, __dmul_rn(p0.shift, (double)num)));
+        sW += __fma_rn(p0.ff1, s6, -__dmul_rn(p0.ff2, s3));
+    }
+    mrmd_dev::block_sum2(sE, sW, red);
     if (threadIdx.x == 0)
     {
-        atomicAdd(ev + 0, energy);
-        atomicAdd(ev + 1, virial);
+        atomicAdd(ev + 0, sE);
+        atomicAdd(ev + 1, -0.5 * sW);
     }
+}
+
+// Rows per warp.  Few rows give a small system enough warps; many rows make
+// the evaluation's rounds full (27.6 pairs in range per row at density
+// 0.8442 against 32 lanes) and amortise the force additions at row changes.
+// Kernel times in us for 2 / 4 / 8 / 16 rows (one lane per row, all entries
+// in FP64, before), dense fluid:
+//       2,048 atoms   10.6 / 12.6 / 18.8 / 29.1   (76)
+//       4,000         16.6 / 14.6 / 18.6 / 29.0   (76)
+//      10,976         28.9 / 26.9 / 29.0 / 39.0
+//      32,000         59.6 / 57.5 / 55.6 / 63.7   (120)
+//     256,000          377 /  363 /  330 /  330   (782)
+//   4,000,000         5640 / 5430 / 4930 / 4830   (11332)
+// (1 row: 12.7 us at 2,048; 32 rows: 4900 us at 4,000,000).  The FP64
+// instructions of the pairs alone take 3.86 ms at 4,000,000 atoms.
+int lj_rows_per_warp(const mrmd_ctx* ctx, int64_t n)
+{
+    const int64_t sms = ctx->numSMs;
+    if (n >= 16 * 96 * sms) return 16;  // 96 warps per SM and more
+    if (n >= 8 * 16 * sms) return 8;
+    if (n >= 4 * 5 * sms) return 4;
+    return 2;
 }
 }  // namespace
 
@@ -135,17 +341,28 @@ int lj_apply_fp64(mrmd_ctx* ctx, const mrmd_lj* lj, mrmd_atoms* a, const mrmd_nl
     const bool usePred = pred != nullptr && pred->kind != MRMD_PRED_ALWAYS;
     const bool multi = lj->numTypes > 1;
     const mrmd_dev::Pred dp = to_dev_pred(pred);
-    const unsigned grid = (unsigned)div_up(n, LJ_TB);
     const double4* pos = reinterpret_cast<const double4*>(a->pos);
-#define LJ_LAUNCH(P, M)                                                                                \
-    k_lj_fp64<P, M><<<grid, LJ_TB, 0, ctx->stream>>>(pos, a->force, a->type, lj->p0, lj->dTable,         \
-                                                     (int32_t)lj->numTypesIndex, lj->rcSqr, nl->counts, \
-                                                     nl->nbrs, nl->maxNeighbors, n, nl->begin, a->numLocal + a->numGhost, dp, ev)
-    if (usePred && multi) LJ_LAUNCH(true, true);
-    else if (usePred) LJ_LAUNCH(true, false);
-    else if (multi) LJ_LAUNCH(false, true);
-    else LJ_LAUNCH(false, false);
-#undef LJ_LAUNCH
+    const float rcSqrUp = (float)(lj->rcSqr * (1.0 + 1e-6));
+    auto launch = [&](auto kernel, int R) {
+        const int64_t groups = div_up(n, (int64_t)(LJ_TB / 32) * R), most = (int64_t)ctx->numSMs * LJ_BLOCKS;
+        const unsigned grid = (unsigned)(groups < most ? groups : most);
+        kernel<<<grid, LJ_TB, 0, ctx->stream>>>(pos, a->force, a->type, lj->p0, lj->dTable, (int32_t)lj->numTypesIndex,
+                                                lj->rcSqr, rcSqrUp, nl->counts, nl->nbrs, nl->maxNeighbors, n,
+                                                nl->begin, a->numLocal + a->numGhost, dp, ev);
+    };
+#define LJ_ROWS(R)                                              \
+    if (usePred && multi) launch(k_lj_fp64<true, true, R>, R);  \
+    else if (usePred) launch(k_lj_fp64<true, false, R>, R);     \
+    else if (multi) launch(k_lj_fp64<false, true, R>, R);       \
+    else launch(k_lj_fp64<false, false, R>, R)
+    switch (lj_rows_per_warp(ctx, n))
+    {
+        case 16: LJ_ROWS(16); break;
+        case 8: LJ_ROWS(8); break;
+        case 4: LJ_ROWS(4); break;
+        default: LJ_ROWS(2); break;
+    }
+#undef LJ_ROWS
     return after_launch(ctx, "lj_fp64");
 }
 }  // namespace mrmd_impl

@@ -1,0 +1,91 @@
+"""The half-list pair kernels at the sizes where their split of the work
+changes (rows per warp, list chunks, ragged last groups), against the oracle."""
+import numpy as np
+import pytest
+
+from conftest import assert_fp64_forces
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def M():
+    import mrmd_gb300 as m
+
+    return m
+
+
+def fluid(cells, drop, rho, seed, lo):
+    """Lattice sites with displacements of 0.08 sigma, `drop` of them vacant,
+    in a box with its lower corner at lo."""
+    rng = np.random.default_rng(seed)
+    a = (4.0 / rho) ** (1.0 / 3.0)
+    base = np.array([[0, 0, 0], [0.5, 0.5, 0], [0.5, 0, 0.5], [0, 0.5, 0.5]])
+    g = np.stack(np.meshgrid(*[np.arange(cells)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    pos = ((g[:, None, :] + base[None, :, :]).reshape(-1, 3) + 0.25) * a
+    pos = np.delete(pos, rng.choice(len(pos), drop, replace=False), axis=0)
+    L = cells * a
+    return np.mod(pos + rng.normal(0, 0.08, pos.shape), L) + np.asarray(lo), L
+
+
+def both(M, orc, pos, lo, L, rc, table, pred=None, types=None):
+    """(forces, energy, virial) of the oracle and a function giving those of a
+    precision on the GPU, before the ghosts' forces are folded back."""
+    hi = [x + L for x in lo]
+    rl = rc + 0.3
+    sd_o, sd_g = orc.subdomain(lo, hi, rl), M.Subdomain(lo, hi, rl)
+    cap = int(len(pos) * (1 + 2.1 * rl / L) ** 3) + 256
+    ao = orc.Atoms.from_positions(pos, capacity=cap)
+    if types is not None:
+        ao.type[: len(pos)] = types
+    orc.create_ghosts(ao, sd_o)
+    most = int(4.5 * rl ** 3) + 32
+    co, no = orc.build_half_list(ao.pos, ao.n, 0, ao.numLocal, rl, sd_o.minGhostCorner, sd_o.maxGhostCorner, 1.0, most)
+    ao.force[:] = 0
+    kinds = {None: None, "either": (orc.PRED_EITHER_IN_SLAB, M.PRED_EITHER_IN_SLAB),
+             "both": (orc.PRED_BOTH_IN_SLAB, M.PRED_BOTH_IN_SLAB)}[pred]
+    args = (0, lo[0] + L / 2, 0.0, L / 4)
+    Eo, Wo = orc.lj_apply(table, rc * rc, ao, co, no, None if kinds is None else orc.pred(kinds[0], *args),
+                          1 if types is None else 2)
+    ag = M.Atoms.from_arrays(pos, type=types, capacity=cap)
+    M.GhostLayer().createGhostAtoms(ag, sd_g)
+    vl = M.HalfVerletList()
+    vl.build(ag, 0, ag.numLocalAtoms, rl, 1.0, sd_g.minGhostCorner, sd_g.maxGhostCorner, 60)
+    assert vl.total_pairs == int(co.sum())
+
+    def gpu(lj, precision):
+        ag.setForce(0.0)
+        lj.apply_if(ag, vl, None if kinds is None else M.pred(kinds[1], *args), precision)
+        return ag.getForce(), lj.getEnergy(), lj.getVirial()
+
+    return (ao.force[: ao.n], Eo, Wo), gpu
+
+
+# Rows per warp change at 3,040, 19,456 and 233,472 atoms on 152 SMs; rc 4
+# gives rows of more than 64 entries (several chunks).
+@pytest.mark.parametrize("cells,drop,rc,cap,pred,lo,types", [
+    (4, 255, 2.5, 0.0, None, [0.0, 0.0, 0.0], False),              # a single atom
+    (5, 3, 2.5, 0.95, None, [-3.0, 2.5, 0.0], False),
+    (9, 1, 4.0, 0.0, "either", [0.0, 0.0, 0.0], False),
+    (10, 961, 2.5, 0.0, None, [0.0, 0.0, 0.0], False),             # 3,039
+    (10, 959, 2.5, 0.95, "both", [5000.0, -70000.0, 0.1], False),  # 3,041, far from the origin
+    (10, 5, 4.0, 0.9, None, [0.0, 0.0, 0.0], True),
+    (17, 197, 2.5, 0.95, None, [0.0, 0.0, 0.0], False),            # 19,455
+    (17, 195, 4.0, 0.0, "either", [-10.0, -10.0, -10.0], True),    # 19,457
+    (39, 3800, 2.5, 0.0, None, [0.0, 0.0, 1000.0], False),         # 233,476
+    (39, 3790, 3.2, 0.95, "both", [0.0, 0.0, 0.0], False),
+])
+def test_fp64_rows_per_warp(M, orc, cells, drop, rc, cap, pred, lo, types):
+    pos, L = fluid(cells, drop, 0.8 if cells > 4 else 0.4, cells + drop, lo)
+    t = np.random.default_rng(cells).integers(0, 2, len(pos)) if types else None
+    sig, eps = (np.array([1.0, 0.95, 0.95, 0.9]), np.array([1.0, 0.8, 0.8, 1.3])) if types else (1.0, 1.0)
+    k = 2 if types else 1
+    caps, rcs = (np.full(4, cap), np.full(4, rc)) if types else (cap, rc)
+    (Fo, Eo, Wo), gpu = both(M, orc, pos, lo, L, rc, orc.lj_table(caps, rcs, sig, eps, k, True), pred, t)
+    F, E, W = gpu(M.LennardJones(rcs, sig, eps, caps, num_types=k, is_shifted=True, num_types_index=k), M.PREC_FP64)
+    if not np.any(Fo):
+        assert not np.any(F) and E == Eo == 0.0 and W == Wo == 0.0
+        return
+    assert_fp64_forces(F, Fo)
+    assert abs(E - Eo) <= 1e-10 * max(abs(Eo), 1.0)
+    assert abs(W - Wo) <= 1e-10 * max(abs(Wo), 1.0)
