@@ -1140,8 +1140,11 @@ class DiffSystem:
         c.tfBinWidth, c.tfTargetDensity, c.tfModulation = tf_bin_width, 0.5, 1.0
         c.tfSmoothingSigma, c.tfSmoothingRange = 1.0, 1.0
         c.tfSampleInterval, c.tfUpdateInterval = 1, int(steps) + 1
-        c.tuning = _tuning_struct(dict(threads_per_row=1, block_size=128, rebuild_interval=rebuild_interval,
-                                       sort_every=0, graph_steps=0))
+        # several lanes per row where one would leave the GPU with few warps
+        # (the rows of the coarse-grained region are empty)
+        self.threads_per_row = 8 if self.n < 20000 else 4 if self.n < 200000 else 1
+        c.tuning = _tuning_struct(dict(threads_per_row=self.threads_per_row, block_size=128,
+                                       rebuild_interval=rebuild_interval, sort_every=0, graph_steps=0))
         dc = _abi.DiffConfigS(int(steps), int(window), int(checkpoint_interval), int(loss_bins), float(loss_sigma))
         h = C.c_void_p()
         self.ctx.check(self.ctx.lib.mrmd_diff_create(self.ctx.h, C.byref(h), C.byref(c), C.byref(replica._struct()),

@@ -163,6 +163,25 @@ int ad_capture(mrmd_ctx* ctx, mrmd_adress* s, int64_t st0, int64_t count, int64_
     s->graphSteps = count;
     return MRMD_OK;
 }
+// Lanes per row of the one-replica engine: several where one lane per row
+// would leave the GPU with few warps and long serial rows (rows outside the
+// slab are empty), one where there are rows enough.  us per step with
+// 1 / 2 / 4 / 8 lanes (slab half the box, fluid after 300 steps):
+//                 FP64                       mixed
+//      5,184   211 / 141 / 102 /  82     143 / 104 /  80 /  69
+//     12,960   186 / 133 / 104 /  98     141 / 106 /  85 /  75
+//     34,560   169 / 123 / 107 / 117     133 / 100 /  86 /  90
+//    129,600   235 / 217 / 206 / 248     154 / 128 / 135 / 170
+//    276,480   377 / 323 / 340 / 448     195 / 198 / 206 / 287
+//    504,600   569 / 537 / 584 / 764
+//    985,680   944 / 969 / 1060 / 1417   582 / 581 / 642 / 934
+int row_lanes_for(int64_t n, bool mixed)
+{
+    if (n < 20000) return 8;
+    if (n < (mixed ? 100000 : 230000)) return 4;
+    if (n < 700000) return 2;
+    return 1;
+}
 }  // namespace
 
 extern "C" {
@@ -206,8 +225,9 @@ int mrmd_adress_create(mrmd_ctx* ctx, mrmd_adress** out, const mrmd_adress_confi
         // million molecules the steps between rebuilds as one persistent
         // launch (4,000,000 molecules: 2.01 against 2.33 ms per step mixed,
         // 5.13 against 5.25 FP64; 34,560: 6% slower)
-        bc.tuning.threadsPerRow = 1;
-        bc.tuning.blockSize = 128;
+        const int lanes = row_lanes_for(n, cfg->precision == MRMD_PREC_MIXED);
+        bc.tuning.threadsPerRow = lanes;
+        bc.tuning.blockSize = lanes == 8 ? 256 : 128;  // blocks of a multiple of 32 rows (rowOrderEnergy)
         bc.tuning.rebuildInterval = cfg->rebuildInterval;
         bc.tuning.sortEvery = 5;
         bc.tuning.graphSteps = cfg->useGraph ? 5 * cfg->rebuildInterval : 0;
@@ -225,6 +245,7 @@ int mrmd_adress_create(mrmd_ctx* ctx, mrmd_adress** out, const mrmd_adress_confi
         rd.seed = cfg->seed;
         mrmd_batch* b = nullptr;
         MRMD_TRY(mrmd_batch_create(ctx, &b, &bc, 1, &rd, pos3, vel3));
+        b->B.rowOrderEnergy = 1;  // the FP32 energies do not depend on the number of lanes
         mrmd_adress* s = new mrmd_adress();
         s->cfg = *cfg;
         s->n = n;

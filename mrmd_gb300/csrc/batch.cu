@@ -609,12 +609,33 @@ struct RowOut
     float fenergy;      // the same in the mixed form (FP32 pair energies)
 };
 
-// One row (local molecule i), lanes `sub` of TPR.  Returns this lane's
-// partial sums.  CL: the row is row `lane >> 2` of i-cluster c (-1: none) and
-// the lane takes slot `sub` of each j-cluster whose mask has bit `lane`.
+// FP64 rows: entries scanned at a time (their positions in the chunk are
+// kept in shared memory, SCAN_CHUNK bytes per row; 1,024 rows, the largest
+// block with one lane per row, stay below the 48 KB that need no opt-in)
+constexpr int SCAN_CHUNK = 40;
+
+// The row's lanes and the lanes before this one among them.
+template <int TPR>
+__device__ __forceinline__ unsigned row_lanes(int lane)
+{
+    return (TPR == 32 ? 0xffffffffu : ((1u << TPR) - 1u)) << (lane & ~(TPR - 1));
+}
+
+// One row (local molecule i; valid = false: none), lanes `sub` of TPR.
+// Returns this lane's partial sums, reduced over the row's lanes.  CL: the
+// row is row `lane >> 2` of i-cluster c (-1: none) and the lane takes slot
+// `sub` of each j-cluster whose mask has bit `lane`.
+//
+// FP64 rows go in two phases, because the kernel is bound by the FP64 pipe:
+// the row's entries are tested in FP32 first (pairs of two coarse-grained
+// molecules, and pairs surely beyond the cutoff: 29% at a skin of 0.3), and
+// the rest, in entry order, is dealt to the row's lanes.  A pair then takes
+// 22 FP64 instructions (distance 3, r^2 3, force factor and energy 10,
+// weight 2, forces 3, energy 1; the comparisons are integer ones) against
+// ~40 for every entry before.
 template <bool MIXED, int TPR, bool CL = false>
-__device__ __forceinline__ RowOut row_force(const BDev& B, int32_t i, int sub, bool sampling, int32_t c = -1,
-                                            int lane = 0)
+__device__ __forceinline__ RowOut row_force(const BDev& B, int32_t i, bool valid, int sub, bool sampling, int32_t c,
+                                            int lane, uint8_t* seg)
 {
     const RepDev& R = B.reps[B.slotRep[i]];
     const double4 la = B.lam[i];  // lambda, modulated, grad x
@@ -645,7 +666,9 @@ __device__ __forceinline__ RowOut row_force(const BDev& B, int32_t i, int sub, b
     float fenergy = 0.0f;
     const int binAlpha = is_hy(la.y) ? comp_bin(la.x) : -1;
     float ffx = 0.0f, ffy = 0.0f, ffz = 0.0f, vsF = 0.0f, csF = 0.0f;  // FP32 sums of the far pairs
-    auto pair_entry = [&](const int32_t entry) {
+    // one list entry; returns the mixed form's (e, w) of the pair's energy e w
+    const float2 none = make_float2(0.f, 0.f);
+    auto pair_entry = [&](const int32_t entry) -> float2 {
         const bool rev = entry < 0;
         const int32_t j = entry & 0x7fffffff;
         // own slot (the molecule or one of its images) and partner slot weights
@@ -707,7 +730,7 @@ __device__ __forceinline__ RowOut row_force(const BDev& B, int32_t i, int sub, b
         if (MIXED)
         {
             const float2 ownF = ownImgF;
-            if (ownF.x <= 0.0f && partModF.x <= 0.0f) return;  // both coarse grained: ideal gas
+            if (ownF.x <= 0.0f && partModF.x <= 0.0f) return none;  // both coarse grained: ideal gas
             const float4 hj = B.hi[j], lj = B.lo[j];
             if (B.farF32 && ownIsSelf)
             {
@@ -718,7 +741,7 @@ __device__ __forceinline__ RowOut row_force(const BDev& B, int32_t i, int sub, b
                 const float dy = (hi_i.y - hj.y) + (lo_i.y - lj.y);
                 const float dz = (hi_i.z - hj.z) + (lo_i.z - lj.z);
                 const float r2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
-                if (r2 > B.rc2.h * 1.0000005f) return;
+                if (r2 > B.rc2.h * 1.0000005f) return none;
                 if (r2 >= B.rsplitSq && r2 < B.rc2.h * 0.9999995f)
                 {
                     const float u = __fdividef(1.0f, r2);
@@ -738,12 +761,11 @@ __device__ __forceinline__ RowOut row_force(const BDev& B, int32_t i, int sub, b
                         vsF += V;
                         if (sampling && binAlpha != -1) csF += V;
                     }
-                    fenergy = __fmaf_rn(e, w, fenergy);
-                    return;
+                    return make_float2(e, w);
                 }
             }
             PairMixed q;
-            if (!pair_mixed(hi_i, lo_i, hj, lj, B.lj, B.rc2, q)) return;
+            if (!pair_mixed(hi_i, lo_i, hj, lj, B.lj, B.rc2, q)) return none;
             const bool hyPair = is_hy_df(ownF) || is_hy_df(partModF);
             // weighting = (lambda~_own + lambda~_partner) / 2 as a double-float
             const bool bothAT = ownF.x == 1.0f && ownF.y == 0.0f && partModF.x == 1.0f && partModF.y == 0.0f;
@@ -777,36 +799,37 @@ __device__ __forceinline__ RowOut row_force(const BDev& B, int32_t i, int sub, b
                     vImgP = df_add(vImgP, V);
                 }
             }
-            fenergy = __fmaf_rn(q.e, bothAT ? 1.0f : 0.5f * (ownF.x + partModF.x), fenergy);
+            return make_float2(q.e, bothAT ? 1.0f : 0.5f * (ownF.x + partModF.x));
         }
         else
         {
-            if (ownMod <= 0.0 && partMod <= 0.0) return;  // both coarse grained: ideal gas
+            if (le_zero(ownMod) && le_zero(partMod)) return none;  // both coarse grained: ideal gas
             const double4 pj = B.pos[j];
             const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
             // explicit roundings: the same bits in every kernel that inlines
             // this body
             const double distSqr = __fma_rn(dx, dx, __fma_rn(dy, dy, __dmul_rn(dz, dz)));
-            if (distSqr > B.rcSqr) return;
-            const bool hyPair = is_hy(ownMod) || is_hy(partMod);
+            if (gt_nonneg(distSqr, B.rcSqr)) return none;
+            const bool hyPair = !(ge_one(ownMod) || le_zero(ownMod)) || !(ge_one(partMod) || le_zero(partMod));
             double ff, e;
-            lj_eval_fp64(B.lj, distSqr, ff, e);
-            const double weighting = 0.5 * (ownMod + partMod);
-            const double ffactor = ff * weighting;
+            lj_eval_series(B.lj, distSqr, ff, e);
+            // twice the weight: the sums are halved once per row (exact)
+            const double weighting = __dadd_rn(ownMod, partMod);
+            const double ffactor = __dmul_rn(ff, weighting);
             dfx = fma(dx, ffactor, dfx);
             dfy = fma(dy, ffactor, dfy);
             dfz = fma(dz, ffactor, dfz);
             energy = fma(e, weighting, energy);
             if (hyPair)
             {
-                const double Vij = 0.5 * e;
                 if (ownIsSelf)
                 {
-                    dvs += Vij;
-                    if (sampling && binAlpha != -1) dcs += Vij;
+                    dvs += e;  // V_ij = e/2: halved once per row
+                    if (sampling && binAlpha != -1) dcs += e;
                 }
                 else
                 {
+                    const double Vij = 0.5 * e;
                     imgFx = fma(-Vij, ownGx, imgFx);
                     if (sampling && is_hy(ownMod))
                     {
@@ -818,7 +841,8 @@ __device__ __forceinline__ RowOut row_force(const BDev& B, int32_t i, int sub, b
                 }
             }
         }
-        };
+        return none;
+    };
     if (CL)
     {
         // every lane walks the cluster's row (uniform loop, broadcast loads)
@@ -830,21 +854,88 @@ __device__ __forceinline__ RowOut row_force(const BDev& B, int32_t i, int sub, b
             if (((uint32_t)e.y >> lane) & 1u)
             {
                 const int32_t j = B.sorted[e.x + sub];
-                pair_entry((((uint32_t)e.z >> lane) & 1u) ? (j | REVERSED) : j);
+                const float2 ew = pair_entry((((uint32_t)e.z >> lane) & 1u) ? (j | REVERSED) : j);
+                fenergy = __fmaf_rn(ew.x, ew.y, fenergy);
             }
         }
     }
+    else if (MIXED)
+    {
+        auto row = [&](const int32_t* nbrs, const int32_t* counts, int32_t cap) {
+            const int cnt = valid ? counts[i] : 0;
+            const int32_t* col = nbrs + mrmd_dev::nbr_row(i, cap);
+            if (TPR == 1 || !B.rowOrderEnergy)
+            {
+                for (int k = sub; k < cnt; k += TPR)
+                {
+                    const float2 ew = pair_entry(col[32 * (int64_t)k]);
+                    fenergy = __fmaf_rn(ew.x, ew.y, fenergy);
+                }
+                return;
+            }
+            // the pairs' energies added in entry order, whatever the number
+            // of lanes: every lane of the row forms the same FP32 chain
+            int most = cnt;
+#pragma unroll
+            for (int off = 16; off >= TPR; off >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, off));
+            for (int k0 = 0; k0 < most; k0 += TPR)
+            {
+                float2 ew = none;
+                if (k0 + sub < cnt) ew = pair_entry(col[32 * (int64_t)(k0 + sub)]);
+#pragma unroll
+                for (int q = 0; q < TPR; ++q)
+                    fenergy = __fmaf_rn(__shfl_sync(0xffffffffu, ew.x, q, TPR), __shfl_sync(0xffffffffu, ew.y, q, TPR),
+                                        fenergy);
+            }
+        };
+        row(B.nbrs, B.counts, B.listCap);
+        if (B.split) row(B.nbrsF, B.countsF, B.listCapF);
+    }
     else
     {
-        const int cnt = B.counts[i];
-        const int64_t rowBase = mrmd_dev::nbr_row(i, B.listCap);
-        for (int k = sub; k < cnt; k += TPR) pair_entry(B.nbrs[rowBase + 32 * (int64_t)k]);
+        const int cnt = valid ? B.counts[i] : 0;
+        const int32_t* col = B.nbrs + mrmd_dev::nbr_row(i, B.listCap);
+        const float3 pf = make_float3(hi_word_f32(pi.x), hi_word_f32(pi.y), hi_word_f32(pi.z));
+        const float rcUp = (float)B.rcSqr * 1.000001f;
+        const bool ownCG = le_zero(la.y);
+        const unsigned mine = row_lanes<TPR>(lane), before = mine & ((1u << lane) - 1u);
+        uint8_t* rowSeg = seg + (threadIdx.x / TPR) * SCAN_CHUNK;
+        int most = cnt;
+#pragma unroll
+        for (int off = 16; off >= TPR; off >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, off));
+        for (int k0 = 0; k0 < most; k0 += SCAN_CHUNK)
+        {
+            int kept = 0;
+            const int kEnd = min(k0 + SCAN_CHUNK, most);
+#pragma unroll 2
+            for (int kk = k0; kk < kEnd; kk += TPR)
+            {
+                const int k = kk + sub;
+                bool keep = k < cnt;
+                if (keep)
+                {
+                    const int32_t entry = col[32 * (int64_t)k], j = entry & 0x7fffffff;
+                    // a reversed instance may act with other weights
+                    if (ownCG && (entry >= 0 || R.consistent)) keep = !le_zero(B.lamt[j]);
+                    if (keep) keep = !surely_beyond(pf, mrmd_dev::ldg4(B.pos + j), rcUp);
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, keep);
+                if (keep) rowSeg[kept + __popc(m & before)] = (uint8_t)(k - k0);
+                kept += __popc(m & mine);
+            }
+            __syncwarp();
+            for (int q = sub; q < kept; q += TPR) pair_entry(col[32 * (int64_t)(k0 + rowSeg[q])]);
+            __syncwarp();
+        }
     }
-    if (MIXED && B.split)
+    if (!MIXED)
     {
-        const int cntF = B.countsF[i];
-        const int64_t rowBaseF = mrmd_dev::nbr_row(i, B.listCapF);
-        for (int k = sub; k < cntF; k += TPR) pair_entry(B.nbrsF[rowBaseF + 32 * (int64_t)k]);
+        dfx *= 0.5;
+        dfy *= 0.5;
+        dfz *= 0.5;
+        dvs *= 0.5;
+        dcs *= 0.5;
+        energy *= 0.5;
     }
     if (MIXED)
     {
@@ -900,6 +991,8 @@ __device__ __forceinline__ RowOut row_force(const BDev& B, int32_t i, int sub, b
     for (int off = 1; off < TPR; off <<= 1)
     {
         imgFx += __shfl_xor_sync(0xffffffffu, imgFx, off);
+        if (MIXED && !CL && B.rowOrderEnergy)
+            continue;  // every lane has the row's sum
         if (MIXED)
             fenergy += __shfl_xor_sync(0xffffffffu, fenergy, off);
         else
@@ -919,7 +1012,7 @@ __device__ __forceinline__ RowOut row_force(const BDev& B, int32_t i, int sub, b
 // One thread's share of the force for global thread index gtid (a warp's
 // 32 lanes take 32 consecutive indices, aligned to 32).
 template <bool MIXED, int TPR, bool CL>
-__device__ __forceinline__ void force_body(const BDev& B, int64_t gtid)
+__device__ __forceinline__ void force_body(const BDev& B, int64_t gtid, uint8_t* seg)
 {
     static_assert(!CL || TPR == CLUSTER_J, "the cluster layout has CLUSTER_J lanes per row");
     const bool sampling = B.sc->sampleComp != 0;
@@ -937,7 +1030,7 @@ __device__ __forceinline__ void force_body(const BDev& B, int64_t gtid)
         valid = c >= 0 && a < cl.y;
         i = valid ? cl.x + a : cl.x;
     }
-    RowOut o = row_force<MIXED, TPR, CL>(B, valid ? i : 0, sub, sampling && valid, c, threadIdx.x & 31);
+    RowOut o = row_force<MIXED, TPR, CL>(B, valid ? i : 0, valid, sub, sampling && valid, c, threadIdx.x & 31, seg);
     int32_t r = valid ? B.slotRep[i] : -1;
     if (valid && sub == 0)
     {
@@ -997,10 +1090,39 @@ __device__ __forceinline__ void force_body(const BDev& B, int64_t gtid)
         B.vel[i] = v;
         B.force[i] = f;
     }
+    double* ring = B.energyRing + (int64_t)B.sc->ringSlot * B.R;
+    if (MIXED && !CL && TPR > 1 && B.rowOrderEnergy)
+    {
+        // the sums of one lane per row: a tree over 32 consecutive rows (the
+        // block holds a multiple of 32), one atomic per 32 rows of a replica
+        __shared__ float rowE[1024 / TPR];
+        __shared__ int32_t rowR[1024 / TPR];
+        __syncthreads();  // read by the previous call
+        if (sub == 0)
+        {
+            rowE[threadIdx.x / TPR] = valid ? 0.5f * o.fenergy : 0.0f;
+            rowR[threadIdx.x / TPR] = r;
+        }
+        __syncthreads();
+        if (threadIdx.x < blockDim.x / TPR)
+        {
+            float e = rowE[threadIdx.x];
+            const int32_t rr = rowR[threadIdx.x];
+            const int32_t r0 = __shfl_sync(0xffffffffu, rr, 0);
+            if (__all_sync(0xffffffffu, rr == r0 || rr == -1))
+            {
+#pragma unroll
+                for (int off = 16; off > 0; off >>= 1) e += __shfl_down_sync(0xffffffffu, e, off);
+                if ((threadIdx.x & 31) == 0 && r0 >= 0) atomicAdd(ring + r0, (double)e);
+            }
+            else if (rr >= 0 && e != 0.0f)
+                atomicAdd(ring + rr, (double)e);
+        }
+        return;
+    }
     // energy per replica: one atomic per warp when the warp's rows share a replica
     const int lane = threadIdx.x & 31;
     const int32_t r0 = __shfl_sync(0xffffffffu, r, 0);
-    double* ring = B.energyRing + (int64_t)B.sc->ringSlot * B.R;
     const bool oneReplica = __all_sync(0xffffffffu, r == r0 || r == -1);
     if (MIXED)
     {
@@ -1036,7 +1158,15 @@ __device__ __forceinline__ void force_body(const BDev& B, int64_t gtid)
 template <bool MIXED, int TPR, bool CL>
 __global__ void __maxnreg__(80) k_b_force(BDev B)
 {
-    force_body<MIXED, TPR, CL>(B, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
+    extern __shared__ uint8_t seg[];
+    force_body<MIXED, TPR, CL>(B, blockIdx.x * (int64_t)blockDim.x + threadIdx.x, seg);
+}
+
+// dynamic shared memory of force_body for blocks of bs threads
+template <bool MIXED, int TPR, bool CL>
+size_t force_smem(int bs)
+{
+    return MIXED || CL ? 0 : (size_t)(bs / TPR) * SCAN_CHUNK;
 }
 
 // pairs (mask bits) and cluster pairs of the cluster layout's rows
@@ -1235,6 +1365,7 @@ __device__ bool grid_sync(const GridBar& gb, bool skip = false)
 template <bool MIXED, int TPR, bool CL>
 __global__ void __maxnreg__(80) k_b_steps(BDev B, int count, GridBar gb)
 {
+    extern __shared__ uint8_t seg[];
     __shared__ TailShared t;
     const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -1246,7 +1377,7 @@ __global__ void __maxnreg__(80) k_b_steps(BDev B, int count, GridBar gb)
         ghost_update_body<MIXED>(B, tid, stride);
         if (!grid_sync(gb)) return;
         for (int64_t base = blockIdx.x * (int64_t)blockDim.x; base < threads; base += stride)
-            force_body<MIXED, TPR, CL>(B, base + threadIdx.x);
+            force_body<MIXED, TPR, CL>(B, base + threadIdx.x, seg);
         if (!grid_sync(gb)) return;
         if (threadIdx.x == 0) tail_read(B, t);
         __syncthreads();
@@ -1401,7 +1532,7 @@ int force_t(mrmd_ctx* ctx, mrmd_batch* b)
 {
     const int bs = b->cfg.tuning.blockSize;
     const int64_t threads = CL ? (int64_t)b->B.numClusters * 32 : (int64_t)b->N * TPR;
-    k_b_force<M, TPR, CL><<<(unsigned)div_up(threads, bs), bs, 0, ctx->stream>>>(b->B);
+    k_b_force<M, TPR, CL><<<(unsigned)div_up(threads, bs), bs, force_smem<M, TPR, CL>(bs), ctx->stream>>>(b->B);
     return after_launch(ctx, "batch force");
 }
 
@@ -1569,15 +1700,15 @@ constexpr unsigned long long SYNC_LIMIT_NS = 2000000000ull;
 // A cooperative launch of the kernel with every block resident (blocks per
 // SM from the occupancy calculator), captured like any launch.
 template <typename... A>
-int cooperative_launch(mrmd_ctx* ctx, void (*kernel)(A...), int blockSize, const char* what, A... args)
+int cooperative_launch(mrmd_ctx* ctx, void (*kernel)(A...), int blockSize, size_t smem, const char* what, A... args)
 {
     int perSM = 0;
-    MRMD_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kernel, blockSize, 0));
+    MRMD_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kernel, blockSize, smem));
     if (perSM < 1) return set_error(ctx, MRMD_ERR_CAPACITY, "%s: no block of %d threads fits an SM", what, blockSize);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(perSM * ctx->numSMs));
     cfg.blockDim = dim3((unsigned)blockSize);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeCooperative;
@@ -1595,8 +1726,9 @@ int persistent_t(mrmd_ctx* ctx, mrmd_batch* b, int count)
     // host before each graph launch and read after it
     MRMD_CUDA(ctx, cudaMemsetAsync(b->dSync, 0, 2 * sizeof(unsigned), ctx->stream));
     const GridBar gb{b->dSync, b->dSync + 1, reinterpret_cast<int32_t*>(b->dSync + 2), SYNC_LIMIT_NS};
-    return cooperative_launch(ctx, k_b_steps<M, TPR, CL>, b->cfg.tuning.blockSize, "batch persistent steps", b->B,
-                              count, gb);
+    const int bs = b->cfg.tuning.blockSize;
+    return cooperative_launch(ctx, k_b_steps<M, TPR, CL>, bs, force_smem<M, TPR, CL>(bs), "batch persistent steps",
+                              b->B, count, gb);
 }
 
 template <bool M>
@@ -2258,7 +2390,7 @@ int mrmd_grid_sync_selftest(mrmd_ctx* ctx, int32_t rounds, int32_t skipBlock, do
     int rc = check_cuda(ctx, cudaMemsetAsync(d, 0, 4 * sizeof(unsigned), ctx->stream), "memset");
     const GridBar gb{d, d + 1, reinterpret_cast<int32_t*>(d + 2), (unsigned long long)(limitMs * 1e6)};
     if (rc == MRMD_OK)
-        rc = cooperative_launch(ctx, k_grid_sync_test, 128, "grid sync selftest", gb, (int)rounds, (int)skipBlock);
+        rc = cooperative_launch(ctx, k_grid_sync_test, 128, 0, "grid sync selftest", gb, (int)rounds, (int)skipBlock);
     unsigned err = 0;
     if (rc == MRMD_OK) rc = d2h(ctx, &err, d + 2, sizeof(unsigned));
     cudaStreamSynchronize(ctx->stream);

@@ -132,6 +132,7 @@ struct BDev
     int32_t* nbrsF;
     int32_t listCapF;
     int32_t split;      // 1: near/far rows (mixed form only)
+    int32_t rowOrderEnergy;  // mixed form, several lanes per row: FP32 energies summed as by one lane per row
     int32_t farF32;     // mixed form: pairs at and beyond r_split in FP32 (near/far and cluster layouts)
     // cluster layout: i-cluster c holds the locals [clusters[c].x, clusters[c].x
     // + clusters[c].y), at most CLUSTER_I of one replica, aligned to the

@@ -80,7 +80,7 @@ constexpr int LJ_BLOCKS = 5;  // resident blocks per SM: with 6 or 7 the segment
 // so it is laid out to issue as few FP64 instructions as possible, with all
 // 32 lanes busy in each:
 //  1. Scan: the rows' entries are tested against the cutoff in FP32 from the
-//     high words of the coordinates (a lower bound of r^2, half_list_far);
+//     high words of the coordinates (a lower bound of r^2, surely_beyond);
 //     the ones that may be in range (71% with a skin of 0.3 at 2.5) are
 //     appended to their row's segment in shared memory.
 //  2. Evaluation: the segments' pairs, numbered row after row, are dealt out
@@ -95,43 +95,6 @@ constexpr int LJ_BLOCKS = 5;  // resident blocks per SM: with 6 or 7 the segment
 // length, 47 rounds for 38 entries.  At 256,000 atoms 4.91e6 FP64 warp
 // instructions (22 per pair in range are 4.85e6), FP64 pipe 76% active.
 // Measured times: lj_rows_per_warp.
-//
-// The double's leading bits as a float, truncated to 20 fraction bits: below
-// 2^-126 zero, beyond FP32 (and NaN, infinity) NaN.
-__device__ __forceinline__ float hi_word_f32(double x)
-{
-    const uint32_t h = (uint32_t)__double2hiint(x), m = h & 0x7fffffffu;
-    uint32_t b = (m - 0x38000000u) << 3;
-    b = m < 0x38100000u ? 0u : b;
-    b = m >= 0x47f00000u ? 0x7fc00000u : b;
-    return __uint_as_float((h & 0x80000000u) | b);
-}
-
-// True when the pair is certainly beyond the cutoff: per axis the distance
-// of the truncated coordinates less 2^-19 of their magnitudes (the two
-// truncations, 2^-20 each, and the FP32 rounding) bounds the true one from
-// below.  NaN coordinates are never far.
-__device__ __forceinline__ bool half_list_far(float3 a, const double4& pj, float rcSqrUp)
-{
-    constexpr float E = 1.9073486328125e-6f;  // 2^-19
-    const float bx = hi_word_f32(pj.x), by = hi_word_f32(pj.y), bz = hi_word_f32(pj.z);
-    const float dx = fmaxf(__fmaf_rn(-E, fabsf(a.x) + fabsf(bx), fabsf(a.x - bx)), 0.f);
-    const float dy = fmaxf(__fmaf_rn(-E, fabsf(a.y) + fabsf(by), fabsf(a.y - by)), 0.f);
-    const float dz = fmaxf(__fmaf_rn(-E, fabsf(a.z) + fabsf(bz), fabsf(a.z - bz)), 0.f);
-    return __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz)) > rcSqrUp;
-}
-
-// 1/x to about an ulp for x in [2^-340, 2^1000]: the hardware's approximate
-// reciprocal y (relative error below 2^-20) and the geometric series of
-// 1/(1 - e), e = 1 - x y, up to e^2; the rest, e^3, is below 2^-60.
-__device__ __forceinline__ double rcp_series(double x)
-{
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = __fma_rn(-x, y, 1.0);
-    return __fma_rn(y, __fma_rn(e, e, e), y);
-}
-
 template <bool PRED, bool MULTI, int R>
 __global__ void __launch_bounds__(LJ_TB, LJ_BLOCKS) k_lj_fp64(
     const double4* __restrict__ pos, double* __restrict__ force, const int32_t* __restrict__ type,
@@ -186,7 +149,7 @@ __global__ void __launch_bounds__(LJ_TB, LJ_BLOCKS) k_lj_fp64(
                     if (keep)
                     {
                         const double4 pj = mrmd_dev::ldg4(pos + j);
-                        keep = !half_list_far(pf, pj, rcSqrUp);
+                        keep = !surely_beyond(pf, pj, rcSqrUp);
                         if (PRED) keep = keep && mrmd_dev::pred2(pred, pr.x, pr.y, pr.z, pj.x, pj.y, pj.z);
                     }
                 }

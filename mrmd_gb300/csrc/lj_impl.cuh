@@ -80,6 +80,82 @@ __device__ __forceinline__ void lj_eval_fp64(const LJDev& p, double distSqr, dou
     e = __dsub_rn(__fma_rn(-__dsub_rn(dist, p.capDist), p.capCoeff, p.eCap), p.shift);
 }
 
+// The double's leading bits as a float, truncated to 20 fraction bits: below
+// 2^-126 zero, beyond FP32 (and NaN, infinity) NaN.
+__device__ __forceinline__ float hi_word_f32(double x)
+{
+    const uint32_t h = (uint32_t)__double2hiint(x), m = h & 0x7fffffffu;
+    uint32_t b = (m - 0x38000000u) << 3;
+    b = m < 0x38100000u ? 0u : b;
+    b = m >= 0x47f00000u ? 0x7fc00000u : b;
+    return __uint_as_float((h & 0x80000000u) | b);
+}
+
+// True when the pair is certainly beyond the cutoff: per axis the distance
+// of the truncated coordinates less 2^-19 of their magnitudes (the two
+// truncations, 2^-20 each, and the FP32 rounding) bounds the true one from
+// below.  NaN coordinates are never far.
+__device__ __forceinline__ bool surely_beyond(float3 a, const double4& pj, float rcSqrUp)
+{
+    constexpr float E = 1.9073486328125e-6f;  // 2^-19
+    const float bx = hi_word_f32(pj.x), by = hi_word_f32(pj.y), bz = hi_word_f32(pj.z);
+    auto least = [](float u, float v) {
+        const float d = __fmaf_rn(-E, fabsf(u) + fabsf(v), fabsf(u - v));
+        return d < 0.f ? 0.f : d;  // NaN stays NaN
+    };
+    const float dx = least(a.x, bx), dy = least(a.y, by), dz = least(a.z, bz);
+    return __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz)) > rcSqrUp;
+}
+
+// 1/x to about an ulp for x in [2^-340, 2^1000]: the hardware's approximate
+// reciprocal y (relative error below 2^-20) and the geometric series of
+// 1/(1 - e), e = 1 - x y, up to e^2; the rest, e^3, is below 2^-60.
+__device__ __forceinline__ double rcp_series(double x)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = __fma_rn(-x, y, 1.0);
+    return __fma_rn(y, __fma_rn(e, e, e), y);
+}
+
+// Comparisons of doubles on the integer pipe (FP64 comparisons run on the
+// FP64 pipe), with the outcome of the FP64 ones for NaN too.
+__device__ __forceinline__ bool le_zero(double x)
+{
+    const long long b = __double_as_longlong(x);
+    return b == 0 || (b < 0 && (unsigned long long)b <= 0xfff0000000000000ull);
+}
+
+__device__ __forceinline__ bool ge_one(double x)
+{
+    const long long b = __double_as_longlong(x);
+    return b >= 0x3ff0000000000000ll && b <= 0x7ff0000000000000ll;
+}
+
+// a > b for a >= 0 or NaN, b >= 0
+__device__ __forceinline__ bool gt_nonneg(double a, double b)
+{
+    const unsigned long long u = (unsigned long long)__double_as_longlong(a);
+    return u > (unsigned long long)__double_as_longlong(b) && u <= 0x7ff0000000000000ull;
+}
+
+// LJ force factor and energy of one pair (the formulae of lj_eval_fp64 with
+// the reciprocal of rcp_series, 10 FP64 instructions): the general form
+// inside the cap and for r^2 below 2^-340.
+__device__ __forceinline__ void lj_eval_series(const LJDev& p, double r2, double& ff, double& e)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(r2);
+    if (b < (unsigned long long)__double_as_longlong(p.capSqr) || b < 0x2ab0000000000000ull)
+    {
+        lj_eval_fp64(p, r2, ff, e);
+        return;
+    }
+    const double u = rcp_series(r2);
+    const double u3 = __dmul_rn(__dmul_rn(u, u), u);
+    ff = __dmul_rn(__dmul_rn(u3, __fma_rn(p.ff1, u3, -p.ff2)), u);
+    e = __fma_rn(u3, __fma_rn(p.ef1, u3, -p.ef2), -p.shift);
+}
+
 void lj_force_energy_host(const mrmd_lj_params* t, double distSqr, int64_t typeIdx, double* ff, double* e);
 void lj_table_host(mrmd_lj_params* out, int64_t numTypes, const double* cap, const double* rc,
                    const double* sigma, const double* epsilon, int isShifted);

@@ -43,13 +43,14 @@ class ThermoForceFit:
                                tf_bin_width=tf_bin_width, ctx=self.ctx, **physics)
         self.num_bins = self.diff.num_bins
         # the batched engine on the same trajectory: same replica (noise
-        # seed), slot order, rebuild interval and frozen compensation, with
+        # seed), slot order, lanes per row, rebuild interval and frozen compensation, with
         # the density sampled every step and one table update at its end
         self._batch_args = dict(hybrid_diameter=hybrid_diameter, tf=True, tf_bin_width=tf_bin_width,
                                 tf_target_density=tf_target_density, tf_modulation=tf_modulation,
                                 tf_sigma=tf_sigma, tf_range=tf_range, tf_sample_interval=1,
-                                tf_update_interval=self.steps, comp_frozen=True, threads_per_row=1,
-                                block_size=128, sort_every=0, graph_steps=0, list_layout=0, **physics)
+                                tf_update_interval=self.steps, comp_frozen=True,
+                                threads_per_row=self.diff.threads_per_row, block_size=128, sort_every=0,
+                                graph_steps=0, list_layout=0, **physics)
 
     def grid(self):
         """Bin centres of the table, min + (i + 0.5) (max - min) / numBins

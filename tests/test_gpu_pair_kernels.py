@@ -89,3 +89,49 @@ def test_fp64_rows_per_warp(M, orc, cells, drop, rc, cap, pred, lo, types):
     assert_fp64_forces(F, Fo)
     assert abs(E - Eo) <= 1e-10 * max(abs(Eo), 1.0)
     assert abs(W - Wo) <= 1e-10 * max(abs(Wo), 1.0)
+
+
+# The AdResS stepper takes 8, 4, 2 or 1 lanes per row by size and form; the
+# batched engine with one lane per row is the same system.
+LANES = [((36, 6, 6), 20.0), ((31, 13, 13), 20.0), ((60, 21, 21), 30.0), ((61, 31, 31), 60.0)]
+
+
+def gas(M, cells, at, precision):
+    """(AdResS stepper, one-lane batch) of one density-0.5 system."""
+    rng = np.random.default_rng(cells[0])
+    base = np.array([[0, 0, 0], [0.5, 0.5, 0], [0.5, 0, 0.5], [0, 0.5, 0.5]])
+    g = np.stack(np.meshgrid(*[np.arange(c) for c in cells], indexing="ij"), -1).reshape(-1, 3)
+    L = 2.0 * np.array(cells)
+    pos = np.mod(((g[:, None, :] + base).reshape(-1, 3) + 0.25) * 2.0 + rng.normal(0, 0.1, (4 * len(g), 3)), L)[:-3]
+    vel = rng.normal(0, 1, pos.shape)
+    kw = dict(rc=2.5, skin=0.3, capping_distance=0.7842, precision=precision, dt=0.005)
+    return (M.AdResSSystem(pos, vel, [0, 0, 0], list(L), list(L / 2), at, 10.0, seed=7, **kw),
+            M.BatchSystem([M.Replica(len(pos), [0, 0, 0], list(L), list(L / 2), at, 7)], pos, vel, 10.0, **kw))
+
+
+@pytest.mark.parametrize("cells,at", LANES)
+def test_adress_lanes_per_row_fp64(M, cells, at):
+    """Sums of some hundred doubles in another order: 1e-12 of the rms force."""
+    a, b = gas(M, cells, at, M.PREC_FP64)
+    ea, eb = a.run(1)[0], b.run(1)[0, 0]
+    (pa, va, fa), (pb, vb, fb) = a.state(), b.state()
+    assert np.array_equal(pa, pb)
+    assert np.abs(fa - fb).max() <= 1e-12 * np.sqrt((fb ** 2).sum(1).mean())
+    assert abs(ea - eb) <= 1e-12 * abs(eb)
+    ea, eb = a.run(49), b.run(49)[:, 0]
+    np.testing.assert_allclose(a.state()[0], b.state()[0], rtol=0, atol=1e-9)
+    np.testing.assert_allclose(ea, eb, rtol=1e-9)
+
+
+@pytest.mark.parametrize("cells,at", LANES)
+def test_adress_lanes_per_row_mixed(M, cells, at):
+    """The FP32 energies are summed in the order of one lane per row: equal
+    but for the FP64 additions across rows.  Forces within the mixed form's
+    bar of the FP64 ones (1e-6 of the rms force)."""
+    a, b = gas(M, cells, at, M.PREC_MIXED)
+    f64 = gas(M, cells, at, M.PREC_FP64)[1]
+    ea, eb = a.run(1)[0], b.run(1)[0, 0]
+    f64.run(1)
+    fa, f = a.state()[2], f64.state()[2]
+    assert np.abs(fa - f).max() <= 1e-6 * np.sqrt((f ** 2).sum(1).mean())
+    assert abs(ea - eb) <= 1e-12 * abs(eb)
