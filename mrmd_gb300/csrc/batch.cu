@@ -337,6 +337,13 @@ __global__ void k_b_ghost_update(BDev B)
 }
 
 // ------------------------------------------------------------ list build --
+// The lanes (TPR consecutive ones) that share this lane's row.
+template <int TPR>
+__device__ __forceinline__ unsigned row_lanes(int lane)
+{
+    return (TPR == 32 ? 0xffffffffu : ((1u << TPR) - 1u)) << (lane & ~(TPR - 1));
+}
+
 // Cabana's half-list discriminator (lexicographic x, y, z): b above a
 __device__ __forceinline__ bool lex_above(const double4& a, const double4& b)
 {
@@ -347,10 +354,26 @@ __device__ __forceinline__ bool lex_above(const double4& a, const double4& b)
 // local molecule, 27-cell stencil walked as contiguous z-column spans of the
 // replica's cell-sorted FP32 coordinates; an FP32 prefilter settles the
 // clear cases and FP64 positions decide inside its error band.
+//
+// LANES lanes of a warp walk a row together, consecutive candidates side by
+// side; ballots give every kept one its place, so the entries are in scan
+// order whatever LANES is.  The walk is bound by the latency of its loads
+// and by idle lanes (rows of unequal spans, coarse-grained rows that keep
+// nothing), not by bandwidth.  A row that stays coarse grained skips the
+// columns whose cells all do: for most of them that is the whole stencil.
+template <int LANES>
 __global__ void __launch_bounds__(128) k_b_build_list(BDev B)
 {
-    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < B.N; i += gridDim.x * blockDim.x)
+    constexpr unsigned ALL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, sub = lane % LANES;
+    const unsigned mine = row_lanes<LANES>(lane), before = mine & ((1u << lane) - 1u);
+    const int64_t step = (int64_t)gridDim.x * blockDim.x / LANES;
+    const int64_t warpRow = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane) / LANES;
+    for (int64_t w0 = warpRow; w0 < B.N; w0 += step)  // the same rounds in every lane of a warp
     {
+        const int64_t row = w0 + lane / LANES;
+        const bool live = row < B.N;
+        const int32_t i = (int32_t)(live ? row : w0);
         const RepDev& R = B.reps[B.slotRep[i]];
         const double4 pi = B.pos[i];
         const float xi = (float)(pi.x - R.gmn[0]), yi = (float)(pi.y - R.gmn[1]), zi = (float)(pi.z - R.gmn[2]);
@@ -361,65 +384,103 @@ __global__ void __launch_bounds__(128) k_b_build_list(BDev B)
         const float cxRel = (float)(R.slab.cx - R.gmn[0]);
         const bool prune = R.consistent != 0;
         const bool rowCG = prune && fabsf(xi - cxRel) > deepCG;
+        // a column of cells lies wholly beyond deepCG: with a margin far above
+        // the FP32 error of the coordinates compared below
+        const float cellX = 1.0f / (float)R.grdx[0], deepCol = deepCG + 1e-3f + 1e-5f * (xi + cellX * R.gn[0]);
         const int32_t ci = B.cellOf[i] - R.cellBase;
         const int cz = ci % R.gn[2];
         const int cy = (ci / R.gn[2]) % R.gn[1];
         const int cx = ci / (R.gn[2] * R.gn[1]);
         int32_t cnt = 0, cntF = 0;
         const int az0 = max(cz - 1, 0), az1 = min(cz + 1, R.gn[2] - 1);
-        for (int ax = max(cx - 1, 0); ax <= min(cx + 1, R.gn[0] - 1); ++ax)
+        for (int col = 0; col < 9; ++col)
         {
-            for (int ay = max(cy - 1, 0); ay <= min(cy + 1, R.gn[1] - 1); ++ay)
+            const int ax = cx - 1 + col / 3, ay = cy - 1 + col % 3;
+            int32_t s0 = 0, len = 0;
+            if (live && ax >= 0 && ax < R.gn[0] && ay >= 0 && ay < R.gn[1])
             {
-                const int32_t c0 = R.cellBase + (ax * R.gn[1] + ay) * R.gn[2];
-                const int32_t s0 = B.cellStart[c0 + az0], s1 = B.cellStart[c0 + az1 + 1];
-                for (int32_t s = s0; s < s1; ++s)
+                const float left = ax * cellX - cxRel, right = left + cellX;
+                if (!(rowCG && (left > deepCol || right < -deepCol)))
                 {
-                    const float4 q = B.spos[s];
+                    const int32_t c0 = R.cellBase + (ax * R.gn[1] + ay) * R.gn[2];
+                    s0 = B.cellStart[c0 + az0];
+                    len = B.cellStart[c0 + az1 + 1] - s0;
+                }
+            }
+            const int32_t rounds = LANES == 1 ? len : __reduce_max_sync(ALL, len);
+            for (int32_t t = 0; t < rounds; t += LANES)
+            {
+                bool keep = false, far = false;
+                int32_t entry = 0;
+                if (t + sub < len)
+                {
+                    const float4 q = B.spos[s0 + t + sub];
                     const int32_t j = __float_as_int(q.w);
-                    if (j == i) continue;
-                    if (rowCG && fabsf(q.x - cxRel) > deepCG) continue;
                     const float dx = xi - q.x, dy = yi - q.y, dz = zi - q.z;
                     const float d2f = dx * dx + dy * dy + dz * dz;
-                    if (d2f > B.listRsqHi) continue;
-                    bool keep = d2f < B.listRsqLo;
-                    if (!keep)
+                    if (j != i && !(rowCG && fabsf(q.x - cxRel) > deepCG) && !(d2f > B.listRsqHi))
                     {
-                        const double4 pj = B.pos[j];
-                        const double ddx = pi.x - pj.x, ddy = pi.y - pj.y, ddz = pi.z - pj.z;
-                        const double d2 =
-                            __dadd_rn(__dadd_rn(__dmul_rn(ddx, ddx), __dmul_rn(ddy, ddy)), __dmul_rn(ddz, ddz));
-                        keep = d2 <= B.listRsq;
-                    }
-                    if (!keep) continue;
-                    int32_t entry = j;
-                    if (j >= B.N && !lex_above(pi, B.pos[j]))
-                    {
-                        // Cabana's half list keeps (source, image of i) instead of
-                        // (i, ghost): i must have that image, or the pair is absent
-                        const uint32_t code = B.gShift[j - B.N];
-                        bool has = true;
-#pragma unroll
-                        for (int d = 0; d < 3; ++d)
+                        keep = d2f < B.listRsqLo;
+                        if (!keep)
                         {
-                            const uint32_t c = (code >> (2 * d)) & 3u;
-                            if (c == 1) has = has && (myImg & (2u << (2 * d)));  // ghost +L: i needs a -L image
-                            if (c == 2) has = has && (myImg & (1u << (2 * d)));  // ghost -L: i needs a +L image
+                            const double4 pj = B.pos[j];
+                            const double ddx = pi.x - pj.x, ddy = pi.y - pj.y, ddz = pi.z - pj.z;
+                            const double d2 =
+                                __dadd_rn(__dadd_rn(__dmul_rn(ddx, ddx), __dmul_rn(ddy, ddy)), __dmul_rn(ddz, ddz));
+                            keep = d2 <= B.listRsq;
                         }
-                        if (!has) continue;
-                        entry = j | REVERSED;
+                        entry = j;
+                        if (keep && j >= B.N && !lex_above(pi, B.pos[j]))
+                        {
+                            // Cabana's half list keeps (source, image of i) instead of
+                            // (i, ghost): i must have that image, or the pair is absent
+                            const uint32_t code = B.gShift[j - B.N];
+#pragma unroll
+                            for (int d = 0; d < 3; ++d)
+                            {
+                                const uint32_t c = (code >> (2 * d)) & 3u;
+                                if (c == 1) keep = keep && (myImg & (2u << (2 * d)));  // ghost +L: i needs a -L image
+                                if (c == 2) keep = keep && (myImg & (1u << (2 * d)));  // ghost -L: i needs a +L image
+                            }
+                            entry = j | REVERSED;
+                        }
+                        far = B.split && d2f >= B.nearSqF;
                     }
-                    if (B.split && d2f >= B.nearSqF)
+                }
+                if (LANES == 1)
+                {
+                    if (keep && far)
                     {
                         if (cntF < B.listCapF) B.nbrsF[mrmd_dev::nbr_row(i, B.listCapF) + 32 * (int64_t)cntF] = entry;
                         ++cntF;
-                        continue;
                     }
-                    if (cnt < B.listCap) B.nbrs[mrmd_dev::nbr_row(i, B.listCap) + 32 * (int64_t)cnt] = entry;
-                    ++cnt;
+                    else if (keep)
+                    {
+                        if (cnt < B.listCap) B.nbrs[mrmd_dev::nbr_row(i, B.listCap) + 32 * (int64_t)cnt] = entry;
+                        ++cnt;
+                    }
+                    continue;
+                }
+                const unsigned m = __ballot_sync(ALL, keep && !far);
+                if (keep && !far)
+                {
+                    const int32_t k = cnt + __popc(m & before);
+                    if (k < B.listCap) B.nbrs[mrmd_dev::nbr_row(i, B.listCap) + 32 * (int64_t)k] = entry;
+                }
+                cnt += __popc(m & mine);
+                if (B.split)
+                {
+                    const unsigned mF = __ballot_sync(ALL, keep && far);
+                    if (keep && far)
+                    {
+                        const int32_t k = cntF + __popc(mF & before);
+                        if (k < B.listCapF) B.nbrsF[mrmd_dev::nbr_row(i, B.listCapF) + 32 * (int64_t)k] = entry;
+                    }
+                    cntF += __popc(mF & mine);
                 }
             }
         }
+        if (!live || sub != 0) continue;
         B.counts[i] = cnt < B.listCap ? cnt : B.listCap;
         if (cnt > B.listCap)
         {
@@ -613,13 +674,6 @@ struct RowOut
 // kept in shared memory, SCAN_CHUNK bytes per row; 1,024 rows, the largest
 // block with one lane per row, stay below the 48 KB that need no opt-in)
 constexpr int SCAN_CHUNK = 40;
-
-// The row's lanes and the lanes before this one among them.
-template <int TPR>
-__device__ __forceinline__ unsigned row_lanes(int lane)
-{
-    return (TPR == 32 ? 0xffffffffu : ((1u << TPR) - 1u)) << (lane & ~(TPR - 1));
-}
 
 // One row (local molecule i; valid = false: none), lanes `sub` of TPR.
 // Returns this lane's partial sums, reduced over the row's lanes.  CL: the
@@ -1518,7 +1572,16 @@ int rebuild_t(mrmd_ctx* ctx, mrmd_batch* b, bool sort)
         k_b_build_clusters<<<grid_for(ctx, (int64_t)B.numClusters * 32, 128, 16), 128, 0, ctx->stream>>>(B);
         return after_launch(ctx, "batch build_clusters");
     }
-    k_b_build_list<<<grid_for(ctx, b->N, 128, 16), 128, 0, ctx->stream>>>(B);
+    // eight lanes per row below ~2,600 rows per SM, where one lane per row
+    // waits for its loads: us per launch with 1 / 4 / 8 / 16 / 32 lanes
+    // 159 / 61 / 44 / 49 / 60 at 34,560 molecules; one lane above, where the
+    // ballots cost more than the idle lanes: 465 / 530 / 592 / 681 / 1049 at
+    // 1.04 million (us per step 158.7 / 153.0 / 152.7 at 192,000, equal
+    // within noise at 500,000)
+    if ((int64_t)b->N < 2600 * (int64_t)ctx->numSMs)
+        k_b_build_list<8><<<grid_for(ctx, (int64_t)b->N * 8, 128, 16), 128, 0, ctx->stream>>>(B);
+    else
+        k_b_build_list<1><<<grid_for(ctx, b->N, 128, 16), 128, 0, ctx->stream>>>(B);
     return after_launch(ctx, "batch build_list");
 }
 

@@ -135,3 +135,28 @@ def test_adress_lanes_per_row_mixed(M, cells, at):
     fa, f = a.state()[2], f64.state()[2]
     assert np.abs(fa - f).max() <= 1e-6 * np.sqrt((f ** 2).sum(1).mean())
     assert abs(ea - eb) <= 1e-12 * abs(eb)
+
+
+def test_list_order_does_not_depend_on_lanes(M):
+    """Small batches build their rows with eight lanes each, large ones with
+    one: the entries come in the same order, so that a replica run in a
+    large batch (near/far rows, FP32 far sums) is bitwise the one run alone."""
+    rng = np.random.default_rng(5)
+    reps, pos, vel = [], [], []
+    for k, (c, at) in enumerate([((120, 30, 30), 60.0), ((30, 6, 7), 14.0)]):
+        base = np.array([[0, 0, 0], [0.5, 0.5, 0], [0.5, 0, 0.5], [0, 0.5, 0.5]])
+        g = np.stack(np.meshgrid(*[np.arange(m) for m in c], indexing="ij"), -1).reshape(-1, 3)
+        L = 2.0 * np.array(c)
+        x = np.mod(((g[:, None, :] + base).reshape(-1, 3) + 0.25) * 2.0 + rng.normal(0, 0.1, (4 * len(g), 3)), L)
+        reps.append(M.Replica(len(x), [0, 0, 0], list(L), list(L / 2), at, 50 + k))
+        pos.append(x)
+        vel.append(rng.normal(0, 1, x.shape))
+    kw = dict(hybrid_diameter=8.0, capping_distance=0.7842, precision=M.PREC_MIXED, rebuild_interval=5,
+              sort_every=1, graph_steps=10, list_layout=1)
+    b = M.BatchSystem(reps, np.concatenate(pos), np.concatenate(vel), **kw)
+    b.run(20)
+    sl = b.replica_slice(1)
+    alone = M.BatchSystem(reps[1:], pos[1], vel[1], **kw)
+    alone.run(20)
+    for x, y in zip(b.state(), alone.state()):
+        assert np.array_equal(x[sl], y)
