@@ -16,6 +16,8 @@ struct SlabDev
     double cx;
     double atHalf;  // atomisticRegionHalfDiameter
     double hy;      // hybridRegionDiameter
+    double outer;   // atHalf + hy
+    double k;       // pi / (2 hy)
     int64_t exponent;
     int32_t abrupt;
 };
@@ -35,17 +37,21 @@ __device__ __forceinline__ double pow_int(double x, int64_t n)
 __device__ __forceinline__ void slab_eval(const SlabDev& s, double x, double& lambda, double& modLambda,
                                           double& gx)
 {
-    // weighting_function/Slab.hpp:161-187 (+ setSmoothWeightInHY :96-120)
-    const double pi = 3.141592653589793238462643383279502884;
+    // weighting_function/Slab.hpp:161-187 (+ setSmoothWeightInHY :96-120).
+    // Outside the hybrid regions this is one FP64 operation: the comparisons
+    // are integer ones on the bits of |dx| (a NaN's lie above infinity's and
+    // go on to the weights, like the FP64 comparisons'), and k and outer are
+    // the host's, of the same roundings.  The gradient's dx / |dx| is a sign.
     const double dx = x - s.cx;
     const double absDx = fabs(dx);
+    const long long b = __double_as_longlong(absDx);
     gx = 0.0;
-    if (absDx < s.atHalf)
+    if (b < __double_as_longlong(s.atHalf))
     {
         lambda = 1.0;
         modLambda = 1.0;
     }
-    else if (absDx > s.atHalf + s.hy)
+    else if (b > __double_as_longlong(s.outer) && b <= 0x7ff0000000000000ll)
     {
         lambda = 0.0;
         modLambda = 0.0;
@@ -57,13 +63,12 @@ __device__ __forceinline__ void slab_eval(const SlabDev& s, double x, double& la
     }
     else
     {
-        const double arg = pi / (2.0 * s.hy) * (absDx - s.atHalf);
-        const double base = cos(arg);
+        double sn, base;
+        sincos(s.k * (absDx - s.atHalf), &sn, &base);
         lambda = base * base;
         modLambda = pow_int(base, s.exponent);
-        const double factor =
-            -pi / (2.0 * s.hy) * (double)s.exponent * sin(arg) * pow_int(base, s.exponent - 1) / absDx;
-        gx = factor * dx;
+        const double slope = s.k * (double)s.exponent * sn * pow_int(base, s.exponent - 1);
+        gx = __double_as_longlong(dx) < 0 ? slope : -slope;
     }
 }
 
@@ -88,6 +93,8 @@ inline SlabDev to_slab(const mrmd_slab* s)
     d.cx = s->center[0];
     d.atHalf = 0.5 * s->atomisticRegionDiameter;
     d.hy = s->hybridRegionDiameter;
+    d.outer = d.atHalf + d.hy;
+    d.k = 3.141592653589793238462643383279502884 / (2.0 * d.hy);
     d.exponent = 2 * s->nu;
     d.abrupt = s->interfaceType == 1;
     return d;

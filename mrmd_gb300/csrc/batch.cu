@@ -45,11 +45,32 @@ using namespace mrmd_batch_impl;
 namespace
 {
 // ------------------------------------------------------------------ pre --
+// Ghost g of a molecule at x with derived values `own`: its position, and the
+// derived values of the axes it is shifted along anew.
+template <bool MIXED>
+__device__ __forceinline__ void ghost_follow(const BDev& B, const RepDev& R, int32_t g, const double4& x,
+                                             const Derived& own)
+{
+    const uint32_t code = B.gShift[g];
+    const int64_t s = (int64_t)B.N + g;
+    const double4 p = make_double4(shifted(x.x, code & 3u, R.L[0]), shifted(x.y, (code >> 2) & 3u, R.L[1]),
+                                   shifted(x.z, (code >> 4) & 3u, R.L[2]), 0.0);
+    Derived d = own;
+    if (code & 3u) derive_x<MIXED>(R, p.x, d);
+    if (code & 12u) derive_y<MIXED>(R, p.y, d);
+    if (code & 48u) derive_z<MIXED>(R, p.z, d);
+    B.pos[s] = p;
+    derived_store<MIXED>(B, s, d);
+}
+
 // B(dt/2) A(dt/2) O(dt) A(dt/2) (VelocityVerletLangevinThermostat.hpp:64-113)
 // with noise keyed by (replica seed, step, the molecule's input index inside
 // the replica: the noise follows the molecule through cell sorts); on a
 // rebuild step the molecule is then wrapped into its box by the
 // MultiResRealAtomsExchange rule (MultiResRealAtomsExchange.cpp:23-73).
+// On a step without rebuild the molecule's ghosts follow it here: they are
+// neighbours in the ghost slots, share its weights unless shifted in x, and
+// take no kernel (and no second pass over positions) of their own.
 // The body over molecules tid, tid + stride, ... (every thread of the grid
 // calls it: the displacement maximum ends in a warp reduction).
 template <bool MIXED>
@@ -77,17 +98,29 @@ __device__ __forceinline__ void pre_body(const BDev& B, int rebuild, int64_t tid
         // Verlet criterion: displacement since the list was built (FP32; the
         // bound it is compared with, skin/2, is far above the rounding)
         const float4 r0 = B.ref[i];
-        if (MIXED && !rebuild)
+        if (!rebuild)
         {
-            // r0 is relative to gmn, the split coordinates to the split
-            // origin, soff below it
             B.pos[i] = x;
             B.vel[i] = v;
-            float4 h, l;
-            slot_derived<MIXED>(B, R, i, x, &h, &l);
-            const float dx = ((h.x - r0.x) + l.x) - R.soff[0], dy = ((h.y - r0.y) + l.y) - R.soff[1],
-                        dz = ((h.z - r0.z) + l.z) - R.soff[2];
+            const Derived own = slot_derived<MIXED>(B, R, i, x);
+            float dx, dy, dz;
+            if (MIXED)
+            {
+                // r0 is relative to gmn, the split coordinates to the split
+                // origin, soff below it
+                dx = ((own.hv.x - r0.x) + own.lv.x) - R.soff[0];
+                dy = ((own.hv.y - r0.y) + own.lv.y) - R.soff[1];
+                dz = ((own.hv.z - r0.z) + own.lv.z) - R.soff[2];
+            }
+            else
+            {
+                dx = f64_to_f32_rn(x.x - R.gmn[0]) - r0.x;
+                dy = f64_to_f32_rn(x.y - R.gmn[1]) - r0.y;
+                dz = f64_to_f32_rn(x.z - R.gmn[2]) - r0.z;
+            }
             m2 = fmaxf(m2, __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz))));
+            const int32_t gEnd = i + 1 < B.N ? B.gCount[i + 1] : B.sc->numGhost;
+            for (int32_t g = B.gCount[i]; g < gEnd && g < B.gCap; ++g) ghost_follow<MIXED>(B, R, g, x, own);
             continue;
         }
         {
@@ -114,8 +147,12 @@ __device__ __forceinline__ void pre_body(const BDev& B, int rebuild, int64_t tid
     if ((threadIdx.x & 31) == 0) mrmd_dev::atomic_max_nonneg(&B.sc->dispStep, (double)m2);
 }
 
+// small blocks end evenly (128 threads: 87 us, 64: 85; 256: 97)
+constexpr int PRE_TB = 64;
+constexpr int PRE_B = 14;
+
 template <bool MIXED>
-__global__ void k_b_pre(BDev B, int rebuild)
+__global__ void __launch_bounds__(PRE_TB, PRE_B) k_b_pre(BDev B, int rebuild)
 {
     pre_body<MIXED>(B, rebuild, blockIdx.x * (int64_t)blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
 }
@@ -305,7 +342,7 @@ __global__ void k_b_ghost_write(BDev B)
     }
 }
 
-// ghost position = real position +- L (UpdateGhostAtoms.cpp:31-68)
+// every ghost from its source's position (the adjoint's steps)
 template <bool MIXED>
 __device__ __forceinline__ void ghost_update_body(const BDev& B, int64_t tid, int64_t stride)
 {
@@ -315,15 +352,9 @@ __device__ __forceinline__ void ghost_update_body(const BDev& B, int64_t tid, in
         const int32_t i = B.gSrc[g];
         const uint32_t code = B.gShift[g];
         const RepDev& R = B.reps[B.slotRep[i]];
-        double4 p = B.pos[i];
-#pragma unroll
-        for (int d = 0; d < 3; ++d)
-        {
-            const uint32_t c = (code >> (2 * d)) & 3u;
-            if (c == 1) set_coord(p, d, __dadd_rn(coord(p, d), R.L[d]));
-            if (c == 2) set_coord(p, d, __dsub_rn(coord(p, d), R.L[d]));
-        }
-        p.w = 0.0;
+        const double4 x = B.pos[i];
+        const double4 p = make_double4(shifted(x.x, code & 3u, R.L[0]), shifted(x.y, (code >> 2) & 3u, R.L[1]),
+                                       shifted(x.z, (code >> 4) & 3u, R.L[2]), 0.0);
         const int64_t s = (int64_t)B.N + g;
         B.pos[s] = p;
         slot_derived<MIXED>(B, R, s, p);
@@ -1413,8 +1444,8 @@ __device__ bool grid_sync(const GridBar& gb, bool skip = false)
     return ok != 0;
 }
 
-// `count` steps without rebuild in one cooperative launch: the four phases
-// of step() (pre, ghost update, force, tail) separated by grid barriers,
+// `count` steps without rebuild in one cooperative launch: the three phases
+// of step() (pre with the ghosts, force, tail) separated by grid barriers,
 // the same arithmetic per molecule, ghost, row and replica.
 template <bool MIXED, int TPR, bool CL>
 __global__ void __maxnreg__(80) k_b_steps(BDev B, int count, GridBar gb)
@@ -1427,8 +1458,6 @@ __global__ void __maxnreg__(80) k_b_steps(BDev B, int count, GridBar gb)
     for (int k = 0; k < count; ++k)
     {
         pre_body<MIXED>(B, 0, tid, stride);
-        if (!grid_sync(gb)) return;
-        ghost_update_body<MIXED>(B, tid, stride);
         if (!grid_sync(gb)) return;
         for (int64_t base = blockIdx.x * (int64_t)blockDim.x; base < threads; base += stride)
             force_body<MIXED, TPR, CL>(B, base + threadIdx.x, seg);
@@ -1679,11 +1708,15 @@ int step(mrmd_ctx* ctx, mrmd_batch* b, int64_t st, bool checkRebuild)
     const bool M = b->cfg.precision == MRMD_PREC_MIXED;
     const bool reb = is_rebuild(b, st) || b->needRebuild;
     b->needRebuild = false;
-    const unsigned gN = grid_for(ctx, b->N, TB);
+    // one molecule per thread up to a few million: the hybrid regions'
+    // molecules take several times longer than the others, so that blocks
+    // with several strided molecules per thread end unevenly (1.04 million:
+    // 103 us with 8 blocks of 256 per SM)
+    const unsigned gN = grid_for(ctx, b->N, PRE_TB, 256);
     if (M)
-        k_b_pre<true><<<gN, TB, 0, ctx->stream>>>(B, reb ? 1 : 0);
+        k_b_pre<true><<<gN, PRE_TB, 0, ctx->stream>>>(B, reb ? 1 : 0);
     else
-        k_b_pre<false><<<gN, TB, 0, ctx->stream>>>(B, reb ? 1 : 0);
+        k_b_pre<false><<<gN, PRE_TB, 0, ctx->stream>>>(B, reb ? 1 : 0);
     MRMD_TRY(after_launch(ctx, "batch pre"));
     if (reb)
     {
@@ -1692,14 +1725,6 @@ int step(mrmd_ctx* ctx, mrmd_batch* b, int64_t st, bool checkRebuild)
         else
             MRMD_TRY(rebuild(ctx, b, is_sort(b, st)));
         b->rebuilds++;
-    }
-    else
-    {
-        if (M)
-            k_b_ghost_update<true><<<grid_for(ctx, B.gCap, TB), TB, 0, ctx->stream>>>(B);
-        else
-            k_b_ghost_update<false><<<grid_for(ctx, B.gCap, TB), TB, 0, ctx->stream>>>(B);
-        MRMD_TRY(after_launch(ctx, "batch ghost_update"));
     }
     MRMD_TRY(M ? force_m<true>(ctx, b) : force_m<false>(ctx, b));
     k_b_tail<<<(unsigned)b->R, TB, 0, ctx->stream>>>(B, reb ? 1 : 0);

@@ -195,34 +195,74 @@ __device__ __forceinline__ void set_coord(double4& p, int d, double v)
 // velocity-Verlet kick and drift: kick_fma / drift_fma (integrate_impl.cuh),
 // the reference's v += dt/2m F and x += dt v, each rounded once
 
-// lambda, modulated lambda and grad lambda (x) of one slot, plus the mixed
-// form's split coordinates (UpdateMolecules.hpp:39-69 for a single site).
-template <bool MIXED>
-__device__ __forceinline__ void slot_derived(const BDev& B, const RepDev& R, int64_t s, const double4& x,
-                                             float4* hiOut = nullptr, float4* loOut = nullptr)
+// What a slot's position gives: lambda, modulated lambda and grad lambda (x),
+// and the mixed form's double-float weight and split coordinates
+// (UpdateMolecules.hpp:39-69 for a single site).
+struct Derived
 {
     double l, m, g;
-    slab_eval(R.slab, x.x, l, m, g);
-    B.lam[s] = make_double4(l, m, g, 0.0);
-    B.lamt[s] = m;
+    float2 mf;
+    float4 hv, lv;
+};
+
+template <bool MIXED>
+__device__ __forceinline__ void derive_x(const RepDev& R, double x, Derived& d)
+{
+    slab_eval(R.slab, x, d.l, d.m, d.g);
     if (MIXED)
     {
         // the conversions on the integer pipe (the same values as the FP64
-        // conversions: this kernel is bound by the FP64 pipe)
-        const float h = f64_to_f32_rn(m);
-        B.lamtf[s] = make_float2(h, f64_to_f32_rn(__dsub_rn(m, f32_to_f64(h))));
-        const float invQ = (float)R.splitInv;
-        float4 hv, lv;
-        split_bits(x.x, R.sko[0], R.sq, invQ, hv.x, lv.x);
-        split_bits(x.y, R.sko[1], R.sq, invQ, hv.y, lv.y);
-        split_bits(x.z, R.sko[2], R.sq, invQ, hv.z, lv.z);
-        hv.w = 0.0f;
-        lv.w = 0.0f;
-        B.hi[s] = hv;
-        B.lo[s] = lv;
-        if (hiOut) *hiOut = hv;
-        if (loOut) *loOut = lv;
+        // conversions: the kernels that call this are bound by the FP64 pipe;
+        // outside the hybrid regions the weight, 0 or 1, has no low part)
+        const float h = f64_to_f32_rn(d.m);
+        const double hd = f32_to_f64(h);
+        const bool exact = __double_as_longlong(hd) == __double_as_longlong(d.m);
+        d.mf = make_float2(h, exact ? 0.0f : f64_to_f32_rn(__dsub_rn(d.m, hd)));
+        split_bits(x, R.sko[0], R.sq, (float)R.splitInv, d.hv.x, d.lv.x);
     }
+}
+
+template <bool MIXED>
+__device__ __forceinline__ void derive_y(const RepDev& R, double y, Derived& d)
+{
+    if (MIXED) split_bits(y, R.sko[1], R.sq, (float)R.splitInv, d.hv.y, d.lv.y);
+}
+
+template <bool MIXED>
+__device__ __forceinline__ void derive_z(const RepDev& R, double z, Derived& d)
+{
+    if (MIXED) split_bits(z, R.sko[2], R.sq, (float)R.splitInv, d.hv.z, d.lv.z);
+}
+
+template <bool MIXED>
+__device__ __forceinline__ void derived_store(const BDev& B, int64_t s, const Derived& d)
+{
+    B.lam[s] = make_double4(d.l, d.m, d.g, 0.0);
+    B.lamt[s] = d.m;
+    if (MIXED)
+    {
+        B.lamtf[s] = d.mf;
+        B.hi[s] = make_float4(d.hv.x, d.hv.y, d.hv.z, 0.0f);
+        B.lo[s] = make_float4(d.lv.x, d.lv.y, d.lv.z, 0.0f);
+    }
+}
+
+// Weights (and split coordinates) of slot s at x.
+template <bool MIXED>
+__device__ __forceinline__ Derived slot_derived(const BDev& B, const RepDev& R, int64_t s, const double4& x)
+{
+    Derived d;
+    derive_x<MIXED>(R, x.x, d);
+    derive_y<MIXED>(R, x.y, d);
+    derive_z<MIXED>(R, x.z, d);
+    derived_store<MIXED>(B, s, d);
+    return d;
+}
+
+// c +- L by a ghost's shift code of one axis (UpdateGhostAtoms.cpp:31-68)
+__device__ __forceinline__ double shifted(double c, uint32_t code, double L)
+{
+    return code == 1 ? __dadd_rn(c, L) : code == 2 ? __dsub_rn(c, L) : c;
 }
 
 // Everything a step changes (positions, velocities, forces, the order of
