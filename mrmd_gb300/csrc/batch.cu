@@ -1483,6 +1483,23 @@ __global__ void k_grid_sync_test(GridBar gb, int rounds, int skipBlock)
 }
 }  // namespace
 
+namespace
+{
+// out[orig[i]] = v[i], three components, for the n locals
+__global__ void k_b_input_order(const double4* __restrict__ v, const int32_t* __restrict__ orig, int64_t n,
+                                double* __restrict__ out3)
+{
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    {
+        const double4 x = v[i];
+        double* o = out3 + 3 * (int64_t)orig[i];
+        o[0] = x.x;
+        o[1] = x.y;
+        o[2] = x.z;
+    }
+}
+}  // namespace
+
 // ================================================================== host ==
 
 namespace mrmd_batch_impl
@@ -2346,26 +2363,22 @@ int mrmd_batch_run(mrmd_ctx* ctx, mrmd_batch* b, int64_t nsteps, double* energie
 int mrmd_batch_get_state(mrmd_ctx* ctx, mrmd_batch* b, double* pos3, double* vel3, double* force3)
 {
     if (!ctx || !b) return MRMD_ERR_ARG;
-    const size_t N = (size_t)b->N;
-    std::vector<double4> h(N);
-    std::vector<int32_t> orig(N);
-    MRMD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    MRMD_TRY(d2h(ctx, orig.data(), b->B.orig, sizeof(int32_t) * N));
+    // put into input order on the device, in the sort's shadow buffer (free
+    // between runs), and copied straight into the caller's arrays: the host
+    // loop over N scattered 24-byte records took 20 of the 43 ms of a 50-step
+    // pass with 1.05 million molecules
+    double* stage = reinterpret_cast<double*>(b->B.sPos);
+    const int64_t N = b->N;
     double* outs[3] = {pos3, vel3, force3};
     const double4* src[3] = {b->B.pos, b->B.vel, b->B.force};
     for (int q = 0; q < 3; ++q)
     {
         if (!outs[q]) continue;
-        MRMD_TRY(d2h(ctx, h.data(), src[q], sizeof(double4) * N));
-        for (size_t i = 0; i < N; ++i)
-        {
-            const size_t o = (size_t)orig[i];
-            outs[q][3 * o] = h[i].x;
-            outs[q][3 * o + 1] = h[i].y;
-            outs[q][3 * o + 2] = h[i].z;
-        }
+        k_b_input_order<<<grid_for(ctx, N, TB), TB, 0, ctx->stream>>>(src[q], b->B.orig, N, stage);
+        MRMD_TRY(after_launch(ctx, "batch input_order"));
+        MRMD_TRY(d2h(ctx, outs[q], stage, sizeof(double) * 3 * (size_t)N));
     }
-    return MRMD_OK;
+    return check_cuda(ctx, cudaStreamSynchronize(ctx->stream), "batch state");
 }
 
 int mrmd_batch_get_tf(mrmd_ctx* ctx, mrmd_batch* b, double* force, double* density, int64_t* binOffsets)

@@ -700,9 +700,7 @@ int mrmd_md_get_state(mrmd_ctx* ctx, mrmd_md* md, double* pos3, double* vel3, do
         k_unpermute3<<<grid_for(ctx, n, TB), TB, 0, ctx->stream>>>(reinterpret_cast<const double4*>(src), md->orig, n,
                                                                     stage);
         MRMD_TRY(after_launch(ctx, "unpermute"));
-        MRMD_CUDA(ctx, cudaMemcpyAsync(hostOut[w], stage, sizeof(double) * 3 * (size_t)n, cudaMemcpyDeviceToHost,
-                                       ctx->stream));
-        MRMD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        MRMD_TRY(d2h(ctx, hostOut[w], stage, sizeof(double) * 3 * (size_t)n));
     }
     return MRMD_OK;
 }
