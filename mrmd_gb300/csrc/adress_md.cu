@@ -266,7 +266,7 @@ int mrmd_adress_create(mrmd_ctx* ctx, mrmd_adress** out, const mrmd_adress_confi
         if (!(s->sd.diameter[d] > rlist)) rc = set_error(ctx, MRMD_ERR_ARG, "box must exceed the list radius");
     if (rc == MRMD_OK)
     {
-        s->grid = make_grid(s->sd.minGhostCorner, s->sd.maxGhostCorner, rlist);
+        s->grid = make_list_grid(s->sd.minGhostCorner, s->sd.maxGhostCorner, rlist, n);
         for (int d = 0; d < 3; ++d) s->slab.center[d] = cfg->slabCenter[d];
         s->slab.atomisticRegionDiameter = cfg->atomisticDiameter;
         s->slab.hybridRegionDiameter = cfg->hybridDiameter;

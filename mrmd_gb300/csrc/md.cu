@@ -480,8 +480,9 @@ int mrmd_md_create(mrmd_ctx* ctx, mrmd_md** out, const mrmd_md_config* cfg, int6
     {
         // mixed form: cells of half the list radius (5^3 cells searched: 42%
         // fewer candidates than 3^3 cells of the full radius)
-        md->grid = make_grid(md->sd.minGhostCorner, md->sd.maxGhostCorner, rlist,
-                             cfg->precision == MRMD_PREC_MIXED ? 2 : 1);
+        md->grid = cfg->precision == MRMD_PREC_MIXED
+                       ? make_grid(md->sd.minGhostCorner, md->sd.maxGhostCorner, rlist, 2)
+                       : make_list_grid(md->sd.minGhostCorner, md->sd.maxGhostCorner, rlist, n);
         if (!tile_split_params(md->sd.minGhostCorner, md->grid.extent * 1.25 + 8.0, rlist, &md->sp))
             rc = set_error(ctx, MRMD_ERR_ARG, "box too large for the mixed form's coordinate split");
     }

@@ -9,7 +9,7 @@
 // set is bit-identical to an all-FP64 build.
 //
 // Because x_j >= x_i implies cell_x(j) >= cell_x(i) (floor is monotone),
-// only the 9 + 9 cells with cell_x >= cell_x(i) can hold neighbours.
+// only the cells with cell_x >= cell_x(i) can hold neighbours.
 #include <algorithm>
 #include <cmath>
 
@@ -49,6 +49,14 @@ CellGrid make_grid(const double* gridMin, const double* gridMax, double delta, i
     g.ncell = (int64_t)n[0] * n[1] * n[2];
     g.extent = extent;
     return g;
+}
+
+CellGrid make_list_grid(const double* gridMin, const double* gridMax, double delta, int64_t n)
+{
+    const CellGrid g = make_grid(gridMin, gridMax, delta, 2);
+    // (per axis first: the product of three counts may pass 2^63)
+    const double cells = (double)g.n.x * (double)g.n.y * (double)g.n.z;
+    return cells <= 8.0 * (double)n + 1048576.0 ? g : make_grid(gridMin, gridMax, delta, 1);
 }
 
 // Bits of v spread to every third position (v < 2^10).
@@ -144,36 +152,104 @@ __global__ void k_cell_gather(const double4* __restrict__ pos, const int32_t* __
     }
 }
 
+// Rows of the list, LANES lanes of a warp per row: they take consecutive
+// candidates of each column's span, and ballots give every kept one its
+// place, so the entries come in scan order whatever LANES is.
 // SPLIT (full lists only): pairs with an FP32 distance below sqrt(nearSqF)
 // go to the first list, the others to the second (`capFar`, `countsFar`,
 // `nbrsFar`, overflow in maxCount[1]).  The split is a placement choice, not
 // a cutoff: every kept pair is in exactly one of the two lists.
-template <bool FULL, bool SPLIT = false>
+template <bool FULL, bool SPLIT, int LANES>
 __global__ void __launch_bounds__(128) k_build_list(
     const double4* __restrict__ pos, const int32_t* __restrict__ cellOf,
     const int32_t* __restrict__ cellStart, const float4* __restrict__ spos, CellGrid g,
     int64_t begin, int64_t end, double rsq, float rsqLo, float rsqHi, int64_t cap,
     int32_t* __restrict__ counts, int32_t* __restrict__ nbrs, int32_t* __restrict__ maxCount, int64_t nPos,
-    float nearSqF = 0.0f, int64_t capFar = 0, int32_t* __restrict__ countsFar = nullptr,
-    int32_t* __restrict__ nbrsFar = nullptr)
+    float nearSqF, int64_t capFar, int32_t* __restrict__ countsFar, int32_t* __restrict__ nbrsFar)
 {
-    for (int64_t i = begin + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < end;
-         i += (int64_t)gridDim.x * blockDim.x)
+    constexpr unsigned ALL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, sub = lane % LANES;
+    const unsigned mine = (LANES == 32 ? ALL : ((1u << LANES) - 1u)) << (lane & ~(LANES - 1));
+    const unsigned before = mine & ((1u << lane) - 1u);
+    const int64_t step = (int64_t)gridDim.x * blockDim.x / LANES;
+    // the same rounds in every lane of a warp
+    for (int64_t w0 = begin + (blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane) / LANES; w0 < end; w0 += step)
     {
+        const int64_t mineRow = w0 + lane / LANES;
+        const bool live = mineRow < end;
+        const int64_t i = live ? mineRow : w0;
         const int32_t ci = cellOf[i];
-        if (!MRMD_IN_BOUNDS(ci, g.ncell)) continue;
+        const bool ok = live && MRMD_IN_BOUNDS(ci, g.ncell);
+        const double4 pi = pos[i];
+        const float xi = (float)(pi.x - g.mn.x), yi = (float)(pi.y - g.mn.y), zi = (float)(pi.z - g.mn.z);
+        const int cz = ci % g.n.z, cy = (ci / g.n.z) % g.n.y, cx = ci / (g.n.z * g.n.y);
+        const int z0 = max(cz - g.reach, 0), z1 = min(cz + g.reach, g.n.z - 1);
         int32_t cnt = 0, cntFar = 0;
         const int64_t row = i - begin;
-        scan_candidates<FULL>(pos, cellStart, spos, g, i, ci, rsq, rsqLo, rsqHi, nPos, [&](int32_t j, float d2f) {
-            if (SPLIT && d2f >= nearSqF)
+        int32_t* __restrict__ out = nbrs + mrmd_dev::nbr_row(row, cap);
+        int32_t* __restrict__ outFar = SPLIT ? nbrsFar + mrmd_dev::nbr_row(row, capFar) : nullptr;
+        // the half list's neighbours lie at cell_x >= cell_x(i)
+        for (int ax = FULL ? cx - g.reach : cx, ax1 = ax + (FULL ? 2 : 1) * g.reach; ax <= ax1; ++ax)
+        {
+            for (int ay = cy - g.reach; ay <= cy + g.reach; ++ay)
             {
-                if (cntFar < capFar) nbrsFar[mrmd_dev::nbr_row(row, capFar) + 32 * (int64_t)cntFar] = j;
-                ++cntFar;
-                return;
+                int32_t s0 = 0, len = 0;
+                if (ok && ax >= 0 && ax < g.n.x && ay >= 0 && ay < g.n.y)
+                {
+                    const int32_t c0 = (ax * g.n.y + ay) * g.n.z;
+                    s0 = cellStart[c0 + z0];
+                    len = cellStart[c0 + z1 + 1] - s0;
+                    if (!MRMD_IN_BOUNDS(s0, nPos + 1) || !MRMD_IN_BOUNDS(s0 + len, nPos + 1)) len = 0;
+                }
+                const int32_t rounds = LANES == 1 ? len : __reduce_max_sync(ALL, len);
+#pragma unroll 4
+                for (int32_t t = 0; t < rounds; t += LANES)
+                {
+                    bool keep = false, far = false;
+                    int32_t j = 0;
+                    if (LANES == 1 || t + sub < len)
+                    {
+                        const float4 q = spos[s0 + t + sub];
+                        float d2f = 0.f;
+                        keep = candidate_kept<FULL>(pos, pi, i, xi, yi, zi, q, rsq, rsqLo, rsqHi, nPos, d2f);
+                        j = __float_as_int(q.w);
+                        far = SPLIT && d2f >= nearSqF;
+                    }
+                    if (LANES == 1)
+                    {
+                        if (keep && far)
+                        {
+                            if (cntFar < capFar) outFar[32 * (int64_t)cntFar] = j;
+                            ++cntFar;
+                        }
+                        else if (keep)
+                        {
+                            if (cnt < cap) out[32 * (int64_t)cnt] = j;
+                            ++cnt;
+                        }
+                        continue;
+                    }
+                    const unsigned m = __ballot_sync(ALL, keep && !far);
+                    if (keep && !far)
+                    {
+                        const int32_t k = cnt + __popc(m & before);
+                        if (k < cap) out[32 * (int64_t)k] = j;
+                    }
+                    cnt += __popc(m & mine);
+                    if (SPLIT)
+                    {
+                        const unsigned mF = __ballot_sync(ALL, keep && far);
+                        if (keep && far)
+                        {
+                            const int32_t k = cntFar + __popc(mF & before);
+                            if (k < capFar) outFar[32 * (int64_t)k] = j;
+                        }
+                        cntFar += __popc(mF & mine);
+                    }
+                }
             }
-            if (cnt < cap) nbrs[mrmd_dev::nbr_row(row, cap) + 32 * (int64_t)cnt] = j;
-            ++cnt;
-        });
+        }
+        if (!ok || sub != 0) continue;
         counts[row] = cnt < cap ? cnt : (int32_t)cap;
         if (cnt > cap) atomicMax(maxCount, cnt);
         if (SPLIT)
@@ -183,6 +259,32 @@ __global__ void __launch_bounds__(128) k_build_list(
         }
     }
 }
+
+namespace
+{
+// Launch of k_build_list<FULL, SPLIT>.
+template <bool FULL, bool SPLIT>
+int build_rows(mrmd_ctx* ctx, const CellList& cl, const double* pos4, int64_t begin, int64_t end, double rsq,
+               float rsqLo, float rsqHi, int64_t cap, int32_t* counts, int32_t* nbrs, int32_t* maxCount, int64_t nPos,
+               float nearSqF = 0.0f, int64_t capFar = 0, int32_t* countsFar = nullptr, int32_t* nbrsFar = nullptr)
+{
+    auto launch = [&](auto kernel, int lanes) {
+        kernel<<<grid_for(ctx, (end - begin) * lanes, 128, 16), 128, 0, ctx->stream>>>(
+            reinterpret_cast<const double4*>(pos4), cl.cellOf, cl.cellStart, cl.spos, cl.g, begin, end, rsq, rsqLo,
+            rsqHi, cap, counts, nbrs, maxCount, nPos, nearSqF, capFar, countsFar, nbrsFar);
+    };
+    // lanes per row: several where one lane per row leaves the SMs with few
+    // warps that wait for their loads; one for large systems, where the
+    // ballots cost more than the idle lanes.  us per launch of the half list
+    // with 1 / 2 / 4 / 8 / 16 lanes: 32,000 atoms 56 / 43 / 28 / 35 / 46,
+    // 256,000 atoms 126 / 154 / 159 / 198 / 284
+    const int64_t rows = end - begin, sms = ctx->numSMs;
+    if (rows < 64 * sms) launch(k_build_list<FULL, SPLIT, 8>, 8);
+    else if (rows < 640 * sms) launch(k_build_list<FULL, SPLIT, 4>, 4);
+    else launch(k_build_list<FULL, SPLIT, 1>, 1);
+    return after_launch(ctx, "build_list");
+}
+}  // namespace
 
 int CellList::build(mrmd_ctx* ctx, const double* pos4, int64_t n, const CellGrid& grid, bool morton,
                     int32_t* nonfinite)
@@ -307,15 +409,10 @@ int build_half_list(mrmd_ctx* ctx, mrmd_nlist* nl, const double* pos4, int64_t n
         MRMD_CUDA(ctx, cudaMemsetAsync(maxCount, 0, sizeof(int32_t), ctx->stream));
         if (rows > 0)
         {
-            if (full)
-                k_build_list<true><<<grid_for(ctx, rows, 128, 16), 128, 0, ctx->stream>>>(
-                    reinterpret_cast<const double4*>(pos4), cl->cellOf, cl->cellStart, cl->spos, cl->g, begin,
-                    end, rsq, rsqLo, rsqHi, cap, nl->counts, nl->nbrs, maxCount, nPos);
-            else
-                k_build_list<false><<<grid_for(ctx, rows, 128, 16), 128, 0, ctx->stream>>>(
-                    reinterpret_cast<const double4*>(pos4), cl->cellOf, cl->cellStart, cl->spos, cl->g, begin,
-                    end, rsq, rsqLo, rsqHi, cap, nl->counts, nl->nbrs, maxCount, nPos);
-            MRMD_TRY(after_launch(ctx, "build_list"));
+            MRMD_TRY(full ? (build_rows<true, false>(ctx, *cl, pos4, begin, end, rsq, rsqLo, rsqHi, cap, nl->counts,
+                                                     nl->nbrs, maxCount, nPos))
+                          : (build_rows<false, false>(ctx, *cl, pos4, begin, end, rsq, rsqLo, rsqHi, cap, nl->counts,
+                                                      nl->nbrs, maxCount, nPos)));
         }
         int32_t h[3] = {0, 0, 0};
         MRMD_CUDA(ctx, cudaMemcpyAsync(h, maxCount, 3 * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
@@ -372,11 +469,9 @@ int build_split_list(mrmd_ctx* ctx, mrmd_nlist* nearList, mrmd_nlist* farList, c
         MRMD_CUDA(ctx, cudaMemsetAsync(maxCount, 0, 2 * sizeof(int32_t), ctx->stream));
         MRMD_CUDA(ctx, cudaMemsetAsync(maxCount + 3, 0, 3 * sizeof(int32_t), ctx->stream));
         auto int32_rows = [&]() -> int {
-            k_build_list<true, true><<<grid_for(ctx, rows, 128, 16), 128, 0, ctx->stream>>>(
-                reinterpret_cast<const double4*>(pos4), cl->cellOf, cl->cellStart, cl->spos, cl->g, begin, end,
-                rsq, rsqLo, rsqHi, capN, nearList->counts, nearList->nbrs, maxCount, nPos, nearSqF, capF,
-                farList->counts, farList->nbrs);
-            return after_launch(ctx, "build_split_list");
+            return build_rows<true, true>(ctx, *cl, pos4, begin, end, rsq, rsqLo, rsqHi, capN, nearList->counts,
+                                          nearList->nbrs, maxCount, nPos, nearSqF, capF, farList->counts,
+                                          farList->nbrs);
         };
         if (rows > 0)
         {
@@ -533,9 +628,8 @@ int mrmd_nlist_build(mrmd_ctx* ctx, mrmd_nlist* nl, const double* pos4, int64_t 
     MRMD_CHECK_ARG(rlist > 0.0 && cellRatio > 0.0 && cellRatio <= 1.0, ctx, "bad cutoff or cell ratio");
     if (nPos > 0) MRMD_CHECK_ARG(pos4 != nullptr, ctx, "null positions");
     for (int d = 0; d < 3; ++d) MRMD_CHECK_ARG(gridMax[d] > gridMin[d], ctx, "empty grid");
-    // cells of edge >= rlist (cellRatio < 1 is accepted and rounded up to one
-    // list radius per cell, which keeps the 3-cell stencil exact)
-    CellGrid g = make_grid(gridMin, gridMax, rlist);
+    // cellRatio is accepted and has no effect: any grid gives the same list
+    CellGrid g = make_list_grid(gridMin, gridMax, rlist, nPos);
     (void)cellRatio;
     MRMD_TRY(build_half_list(ctx, nl, pos4, nPos, begin, end, rlist, g, maxNeighbors, false));
     MRMD_TRY(list_total_pairs(ctx, nl));

@@ -160,3 +160,35 @@ def test_list_order_does_not_depend_on_lanes(M):
     alone.run(20)
     for x, y in zip(b.state(), alone.state()):
         assert np.array_equal(x[sl], y)
+
+
+@pytest.mark.parametrize("cells,drop", [(13, 0), (14, 1), (29, 0), (30, 3)])
+def test_half_list_lanes_are_the_oracle_rows(M, orc, cells, drop):
+    """Eight lanes per row below 9,728 rows on 152 SMs, four below 97,280, one
+    above: each row holds exactly the oracle's neighbours."""
+    lo = [-1.0, 0.0, 7.0]
+    pos, L = fluid(cells, drop, 0.8442, 3 * cells, lo)
+    hi = [x + L for x in lo]
+    sd_o, sd_g = orc.subdomain(lo, hi, 2.8), M.Subdomain(lo, hi, 2.8)
+    ao = orc.Atoms.from_positions(pos, capacity=int(len(pos) * (1 + 6 / L) ** 3) + 256)
+    orc.create_ghosts(ao, sd_o)
+    co, no = orc.build_half_list(ao.pos, ao.n, 0, ao.numLocal, 2.8, sd_o.minGhostCorner, sd_o.maxGhostCorner, 1.0, 96)
+    ag = M.Atoms.from_arrays(pos, capacity=len(ao.pos))
+    M.GhostLayer().createGhostAtoms(ag, sd_g)
+    vl = M.HalfVerletList()
+    vl.build(ag, 0, ag.numLocalAtoms, 2.8, 1.0, sd_g.minGhostCorner, sd_g.maxGhostCorner, 20)
+    cg, ng = vl.download(96)
+    np.testing.assert_array_equal(cg, co)
+    k = np.arange(96)[None, :] < co[:, None]
+    np.testing.assert_array_equal(np.sort(np.where(k, ng, -1), 1), np.sort(np.where(k, no, -1), 1))
+
+
+def test_sparse_box_keeps_full_radius_cells(M):
+    """A box with far more half-radius cells than particles (4.4e9 of them,
+    beyond 2^31) still builds its list."""
+    L = 2300.0
+    pos = np.array([[1.0, 1.0, 1.0], [2.0, 1.0, 1.0], [L / 2] * 3, [L / 2, L / 2, L / 2 + 2.7]])
+    a = M.Atoms.from_arrays(pos, capacity=64)
+    vl = M.HalfVerletList()
+    vl.build(a, 0, 4, 2.8, 1.0, [0.0] * 3, [L] * 3, 8)
+    assert vl.total_pairs == 2
