@@ -22,6 +22,7 @@
 // fraction of its FP32 rate, and even the per-atom conversions to FP64 are
 // assembled from the float bits with integer operations.
 #include <cmath>
+#include <type_traits>
 
 #include "common.cuh"
 #include "lj_tile.cuh"
@@ -95,18 +96,11 @@ namespace
 constexpr int HT_BITS = 12;
 constexpr int HT = 1 << HT_BITS;  // hash slots per tile (load <= TILE_CAP / HT = 0.75)
 
-__global__ void k_tile_split(const double4* __restrict__ pos, int64_t n, SplitParams sp, float4* __restrict__ recA,
-                             float2* __restrict__ recB)
+__global__ void k_tile_split(const double4* __restrict__ pos, int64_t n, SplitParams sp, float4* __restrict__ rec)
 {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x)
-    {
-        float4 a;
-        float2 b;
-        tile_split(pos[i], sp, a, b);
-        recA[i] = a;
-        recB[i] = b;
-    }
+        tile_split(pos[i], sp, rec, i);
 }
 
 __device__ __forceinline__ uint32_t slot_hash(int32_t j)
@@ -256,42 +250,33 @@ struct Geom
     float r2h, r2l;
 };
 
-// dh, dl and r^2 = (r2h, r2l) of one pair; false when beyond the cutoff
-// (decided on the double-float r^2, so that pairs within 2^-24 of rc^2 land
-// on the same side as in FP64).
-__device__ __forceinline__ bool pair_geom(const float4& ai, const float2& bi, const float4& aj, const float2& bj,
-                                          RcSq rc2, Geom& g)
-{
-    g.dhx = __fsub_rn(ai.x, aj.x);  // exact
-    g.dhy = __fsub_rn(ai.y, aj.y);
-    g.dhz = __fsub_rn(ai.z, aj.z);
-    g.dlx = __fsub_rn(ai.w, aj.w);
-    g.dly = __fsub_rn(bi.x, bj.x);
-    g.dlz = __fsub_rn(bi.y, bj.y);
-    const float S = __fmaf_rn(g.dhx, g.dhx, __fmaf_rn(g.dhy, g.dhy, __fmul_rn(g.dhz, g.dhz)));  // exact
-    // C = sum dl (2 dh + dl)
-    const float C = __fmaf_rn(g.dlx, __fmaf_rn(2.0f, g.dhx, g.dlx),
-                              __fmaf_rn(g.dly, __fmaf_rn(2.0f, g.dhy, g.dly),
-                                        __fmul_rn(g.dlz, __fmaf_rn(2.0f, g.dhz, g.dlz))));
-    g.r2h = __fadd_rn(S, C);
-    g.r2l = __fsub_rn(C, __fsub_rn(g.r2h, S));
-    return !(g.r2h > rc2.h || (g.r2h == rc2.h && g.r2l > rc2.l));
-}
-
 struct Sums
 {
     float fxh = 0.f, fxl = 0.f, fyh = 0.f, fyl = 0.f, fzh = 0.f, fzl = 0.f;  // double-float pairs
     float gx = 0.f, gy = 0.f, gz = 0.f;    // FP32 pairs
-    float s3h, s3l = 0.f, s6h, s6l = 0.f;  // biased sums of u^3, u^6
+    float2 sh, sl;                         // biased sums of (u^3, u^6), heads and low parts
     int32_t cnt = 0;                       // uncapped pairs in range
     df ec{0.f, 0.f}, wc{0.f, 0.f};         // capped pairs: energy, forceFactor * r^2
 };
 
-// s += x for |x| <= bias <= |s| (Fast2Sum: exact error term into the low part)
-__device__ __forceinline__ void biased_add(float& sh, float& sl, float x)
+__device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
+
+// The hardware's approximate 1/x alone (__fdividef(1, x) for normal x, without
+// its handling of subnormal ones; every use refines or masks it).
+__device__ __forceinline__ float rcp_seed(float x)
 {
-    const float t = __fadd_rn(sh, x);
-    sl = __fadd_rn(sl, __fsub_rn(x, __fsub_rn(t, sh)));
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// s += x for |x| <= bias <= |s| (Fast2Sum: exact error term into the low
+// part), u^3 and u^6 side by side
+__device__ __forceinline__ void biased_add(float2& sh, float2& sl, float2 x)
+{
+    const float2 minus = f2(-1.f, -1.f);
+    const float2 t = __fadd2_rn(sh, x);
+    sl = __fadd2_rn(sl, __ffma2_rn(__ffma2_rn(sh, minus, t), minus, x));  // x - (t - sh)
     sh = t;
 }
 
@@ -329,7 +314,7 @@ __device__ __forceinline__ void near_pair(const Geom& g, const TileParams& tp, S
         // u = 1/r^2 = u0 + u1 (one Newton step on the exact residual), then
         // u^2, u^3, u^4 and forceFactor = u^4 (ff1 u^3 - ff2) as unnormalised
         // float pairs (head, first-order error)
-        const float u0 = __fdividef(1.0f, g.r2h);
+        const float u0 = rcp_seed(g.r2h);
         const float u1 = __fmul_rn(u0, __fmaf_rn(-g.r2l, u0, __fmaf_rn(-g.r2h, u0, 1.0f)));
         const float p2 = __fmul_rn(u0, u0);
         const float q2 = __fmaf_rn(__fadd_rn(u0, u0), u1, __fmaf_rn(u0, u0, -p2));
@@ -345,11 +330,9 @@ __device__ __forceinline__ void near_pair(const Geom& g, const TileParams& tp, S
         f1 = __fmaf_rn(p4, tl, __fmaf_rn(q4, ts.h, __fmaf_rn(p4, ts.h, -f0)));
         // u^3 = p3 + q3 and u^6 = p3^2 + 2 p3 q3 (+ the rounding of p3^2): the
         // head p3 alone carries the seed reciprocal's error, which q3 corrects
-        biased_add(s.s3h, s.s3l, p3);
-        s.s3l = __fadd_rn(s.s3l, q3);
         const float u6 = __fmul_rn(p3, p3);
-        biased_add(s.s6h, s.s6l, u6);
-        s.s6l = __fadd_rn(s.s6l, __fmaf_rn(__fadd_rn(p3, p3), q3, __fmaf_rn(p3, p3, -u6)));
+        biased_add(s.sh, s.sl, f2(p3, u6));
+        s.sl = __fadd2_rn(s.sl, f2(q3, __fmaf_rn(__fadd_rn(p3, p3), q3, __fmaf_rn(p3, p3, -u6))));
         s.cnt += 1;
     }
     acc_prod(s.fxh, s.fxl, g.dhx, g.dlx, f0, f1);
@@ -357,21 +340,74 @@ __device__ __forceinline__ void near_pair(const Geom& g, const TileParams& tp, S
     acc_prod(s.fzh, s.fzl, g.dhz, g.dlz, f0, f1);
 }
 
-__device__ __forceinline__ void far_pair(const Geom& g, const TileParams& tp, Sums& s)
+// This row's record with its signs turned, as packed operands.
+struct Own
 {
-    float u = __fdividef(1.0f, g.r2h);
-    u = __fmaf_rn(u, __fmaf_rn(-g.r2l, u, __fmaf_rn(-g.r2h, u, 1.0f)), u);
-    const float u2 = __fmul_rn(u, u);
-    const float u3 = __fmul_rn(u2, u);
-    const float u4 = __fmul_rn(u2, u2);
-    // forceFactor = u^3 (ff1 u^3 - ff2) u (action/LennardJones.hpp:60-66)
-    const float ff = __fmul_rn(u4, __fmaf_rn(tp.p.ff1h, u3, -tp.p.ff2h));
-    s.gx = __fmaf_rn(__fadd_rn(g.dhx, g.dlx), ff, s.gx);
-    s.gy = __fmaf_rn(__fadd_rn(g.dhy, g.dly), ff, s.gy);
-    s.gz = __fmaf_rn(__fadd_rn(g.dhz, g.dlz), ff, s.gz);
-    biased_add(s.s3h, s.s3l, u3);
-    biased_add(s.s6h, s.s6l, __fmul_rn(u3, u3));
-    s.cnt += 1;
+    float2 nhxy, nlxy;
+    float nhz, nlz;
+};
+
+// Two list entries of a row, in their order (has1: the second one exists),
+// with the packed FP32 instructions (two lanes per instruction, the rounding
+// of the scalar ones): the pair kernel is bound by instruction issue.  x and
+// y of a pair share an instruction where each has its own operand; past r^2
+// the two pairs share one; u^3 and u^6 of a pair do in the energy sums.  The
+// differences are formed as neighbour - own, and r^2 negated, so that no
+// packed operand needs a sign change: the products are the same bits.
+//   dh = hi_i - hi_j (exact), dl = lo_i - lo_j,
+//   S = sum dh^2 (exact), C = sum dl (2 dh + dl), r^2 = S + C as (r2h, r2l);
+// the cutoff is decided on the double-float r^2, so that pairs within 2^-24
+// of rc^2 land on the same side as in FP64.  Near pairs (NEAR rows, and
+// far-row pairs that came within r_split) go to near_pair, the others add
+//   u = 1/r^2 (one Newton step), ff = u^4 (ff1 u^3 - ff2)
+// (action/LennardJones.hpp:60-66) to the FP32 sums; a pair beyond the
+// cutoff, and a near one, takes part with u = 0, which adds exact zeros.
+template <bool NEAR, bool CAP>
+__device__ __forceinline__ void two_pairs(const Own& o, const float4& a0, const float2& b0, const float4& a1,
+                                          const float2& b1, bool has1, const TileParams& tp, Sums& s)
+{
+    const float2 two = f2(2.f, 2.f), minus = f2(-1.f, -1.f), one = f2(1.f, 1.f);
+    const float2 h0 = __fadd2_rn(f2(a0.x, a0.y), o.nhxy), h1 = __fadd2_rn(f2(a1.x, a1.y), o.nhxy);  // -dh x, y
+    const float2 l0 = __fadd2_rn(f2(a0.z, a0.w), o.nlxy), l1 = __fadd2_rn(f2(a1.z, a1.w), o.nlxy);  // -dl x, y
+    const float2 hz = f2(__fadd_rn(b0.x, o.nhz), __fadd_rn(b1.x, o.nhz));  // -dh z of both pairs
+    const float2 lz = f2(__fadd_rn(b0.y, o.nlz), __fadd_rn(b1.y, o.nlz));
+    const float2 t0 = __ffma2_rn(two, h0, l0), t1 = __ffma2_rn(two, h1, l1), tz = __ffma2_rn(two, hz, lz);
+    const float2 zz = __fmul2_rn(hz, hz), lt = __fmul2_rn(lz, tz);
+    const float2 nS = f2(__fmaf_rn(-h0.x, h0.x, __fmaf_rn(-h0.y, h0.y, -zz.x)),
+                         __fmaf_rn(-h1.x, h1.x, __fmaf_rn(-h1.y, h1.y, -zz.y)));
+    const float2 nC = f2(__fmaf_rn(-l0.x, t0.x, __fmaf_rn(-l0.y, t0.y, -lt.x)),
+                         __fmaf_rn(-l1.x, t1.x, __fmaf_rn(-l1.y, t1.y, -lt.y)));
+    const float2 nr = __fadd2_rn(nS, nC);                                  // -r2h
+    const float2 nq = __ffma2_rn(__ffma2_rn(nS, minus, nr), minus, nC);    // -r2l = -(C - (r2h - S))
+    const bool in0 = !(nr.x < -tp.rc2.h || (nr.x == -tp.rc2.h && nq.x < -tp.rc2.l));
+    const bool in1 = has1 && !(nr.y < -tp.rc2.h || (nr.y == -tp.rc2.h && nq.y < -tp.rc2.l));
+    const bool near0 = in0 && (NEAR || -nr.x < tp.rsplitSq), near1 = in1 && (NEAR || -nr.y < tp.rsplitSq);
+    if (NEAR || near0 || near1)
+    {
+        if (near0) near_pair<CAP>(Geom{-h0.x, -h0.y, -hz.x, -l0.x, -l0.y, -lz.x, -nr.x, -nq.x}, tp, s);
+        if (near1) near_pair<CAP>(Geom{-h1.x, -h1.y, -hz.y, -l1.x, -l1.y, -lz.y, -nr.y, -nq.y}, tp, s);
+    }
+    if (!NEAR)
+    {
+        float2 u = f2(rcp_seed(-nr.x), rcp_seed(-nr.y));
+        u = __ffma2_rn(u, __ffma2_rn(nq, u, __ffma2_rn(nr, u, one)), u);
+        const bool far0 = in0 && !near0, far1 = in1 && !near1;
+        u = f2(far0 ? u.x : 0.f, far1 ? u.y : 0.f);
+        const float2 u2 = __fmul2_rn(u, u), u4 = __fmul2_rn(u2, u2);
+        const float c0 = __fmul_rn(u2.x, u.x), c1 = __fmul_rn(u2.y, u.y);  // u^3
+        const float f0 = __fmul_rn(u4.x, __fmaf_rn(-tp.p.ff1h, c0, tp.p.ff2h));  // -ff
+        const float f1 = __fmul_rn(u4.y, __fmaf_rn(-tp.p.ff1h, c1, tp.p.ff2h));
+        const float2 d0 = __fadd2_rn(h0, l0), d1 = __fadd2_rn(h1, l1), dz = __fadd2_rn(hz, lz);
+        s.gx = __fmaf_rn(d0.x, f0, s.gx);
+        s.gy = __fmaf_rn(d0.y, f0, s.gy);
+        s.gz = __fmaf_rn(dz.x, f0, s.gz);
+        s.gx = __fmaf_rn(d1.x, f1, s.gx);
+        s.gy = __fmaf_rn(d1.y, f1, s.gy);
+        s.gz = __fmaf_rn(dz.y, f1, s.gz);
+        biased_add(s.sh, s.sl, f2(c0, __fmul_rn(c0, c0)));
+        biased_add(s.sh, s.sl, f2(c1, __fmul_rn(c1, c1)));
+        s.cnt += (far0 ? 1 : 0) + (far1 ? 1 : 0);
+    }
 }
 
 // The double with the value of a normal FP32 number (or zero), assembled
@@ -398,8 +434,7 @@ __device__ __forceinline__ df shfl_down_df(df v, int o)
 // Neighbour records of slot / index `idx`.
 template <bool TILE>
 __device__ __forceinline__ void load_rec(const float4* __restrict__ shA, const float2* __restrict__ shB,
-                                         const float4* __restrict__ recA, const float2* __restrict__ recB,
-                                         int32_t idx, float4& a, float2& b)
+                                         const float4* __restrict__ rec, int32_t idx, float4& a, float2& b)
 {
     if (TILE)
     {
@@ -408,18 +443,38 @@ __device__ __forceinline__ void load_rec(const float4* __restrict__ shA, const f
     }
     else
     {
-        a = __ldg(recA + idx);
-        b = __ldg(recB + idx);
+        a = __ldg(rec + 2 * (int64_t)idx);
+        b = __ldg(reinterpret_cast<const float2*>(rec + 2 * (int64_t)idx + 1));
     }
+}
+
+// Asynchronous copies of 16 and 8 bytes from global to shared memory.
+__device__ __forceinline__ void async_copy16(void* sh, const void* g)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(sh)), "l"(g));
+}
+
+__device__ __forceinline__ void async_copy8(void* sh, const void* g)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(sh)), "l"(g));
 }
 
 // TILE: one block per tile, rows as 16-bit member slots in 8-entry chunks
 // (capN, capF: chunks per row), member records in shared memory; otherwise
 // rows as int32 particle indices (capN, capF: list capacities), records
 // gathered from global memory (fallback and comparison form).
+//
+// No single unit bounds the tiled form: at 256,000 atoms it issues 65% of the
+// cycles, the FMA pipe is 46% and the shared-memory pipe 50% busy (the
+// neighbours' slots conflict in the banks).  Each row's next chunk is loaded
+// before the current one is worked on (957 -> 863 us at 4,000,000 atoms), two
+// entries share the packed FP32 instructions (two_pairs), and the records of
+// a tile's members arrive by asynchronous copies.  4,000,000 atoms 973 -> 863
+// us, 256,000 78 -> 70; of the 863 us the near rows take about 200, the
+// staging 70.  128-row tiles stage 28% more members (1068 us).
 template <bool TILE, bool CAP>
 __global__ void __launch_bounds__(TILE_ROWS, 4) k_lj_tile(
-    const float4* __restrict__ recA, const float2* __restrict__ recB, const int32_t* __restrict__ members,
+    const float4* __restrict__ rec, const int32_t* __restrict__ members,
     const int32_t* __restrict__ memberCount, int32_t smemStride, const int32_t* __restrict__ countsN,
     const void* __restrict__ colsN, int64_t capN, const int32_t* __restrict__ countsF,
     const void* __restrict__ colsF, int64_t capF, int64_t rows, int64_t nAll, double4* __restrict__ force,
@@ -434,72 +489,86 @@ __global__ void __launch_bounds__(TILE_ROWS, 4) k_lj_tile(
     int32_t nMem = 0;
     if (TILE)
     {
+        // the members' records: a thread's indices first, then all its copies
+        // in flight at once
+        constexpr int U = 6;
         nMem = memberCount[tile];
         const int32_t* mem = members + tile * TILE_CAP;
-        for (int32_t t = tid; t < nMem; t += TILE_ROWS)
+        for (int32_t t0 = tid; t0 < nMem; t0 += U * TILE_ROWS)
         {
-            const int32_t j = mem[t];
-            if (!MRMD_IN_BOUNDS(j, nAll)) continue;
-            shA[t] = __ldg(recA + j);
-            shB[t] = __ldg(recB + j);
+            int32_t j[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) j[u] = t0 + u * TILE_ROWS < nMem ? __ldg(mem + t0 + u * TILE_ROWS) : -1;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+            {
+                const int32_t t = t0 + u * TILE_ROWS;
+                if (t >= nMem || !MRMD_IN_BOUNDS(j[u], nAll)) continue;
+                async_copy16(shA + t, rec + 2 * (int64_t)j[u]);
+                async_copy8(shB + t, rec + 2 * (int64_t)j[u] + 1);
+            }
         }
+        asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
     }
     const int64_t row = tile * TILE_ROWS + tid;
     const int32_t bound = TILE ? nMem : (int32_t)nAll;
     (void)bound;  // read by MRMD_IN_BOUNDS in the bounds-checked build
     Sums s;
-    s.s3h = tp.bias3;
-    s.s6h = tp.bias6;
+    s.sh = f2(tp.bias3, tp.bias6);
+    s.sl = f2(0.f, 0.f);
     if (row < rows)
     {
-        const float4 ai = __ldg(recA + row);
-        const float2 bi = __ldg(recB + row);
+        float4 ai;
+        float2 bi;
+        load_rec<false>(nullptr, nullptr, rec, (int32_t)row, ai, bi);
         const int32_t cn = countsN[row], cf = countsF[row];
-        // one pair of slot (TILE) or particle index `idx`: near rows always in
-        // double-float, far rows in FP32 unless the pair came within r_split
-        auto pair = [&](int32_t idx, bool nearRow) {
-            if (!MRMD_IN_BOUNDS(idx, bound)) return;
-            float4 aj;
-            float2 bj;
-            load_rec<TILE>(shA, shB, recA, recB, idx, aj, bj);
-            Geom g;
-            if (!pair_geom(ai, bi, aj, bj, tp.rc2, g)) return;
-            if (nearRow || g.r2h < tp.rsplitSq)
-                near_pair<CAP>(g, tp, s);
-            else
-                far_pair(g, tp, s);
+        const Own own{f2(-ai.x, -ai.y), f2(-ai.z, -ai.w), -bi.x, -bi.y};
+        // two entries (slots or particle indices)
+        auto pairs = [&](int32_t i0, int32_t i1, bool has1, auto nearRow) {
+            if (!MRMD_IN_BOUNDS(i0, bound) || !MRMD_IN_BOUNDS(i1, bound)) return;
+            float4 a0, a1;
+            float2 b0, b1;
+            load_rec<TILE>(shA, shB, rec, i0, a0, b0);
+            load_rec<TILE>(shA, shB, rec, i1, a1, b1);
+            two_pairs<decltype(nearRow)::value, CAP>(own, a0, b0, a1, b1, has1, tp, s);
         };
         if (TILE)
         {
-            // eight slots per 16-byte chunk load
-            auto rows_of = [&](const uint4* __restrict__ chunks, int64_t nch, int32_t cnt, bool nearRow) {
-                const int64_t base = chunk_word(row, 0, nch);
-                for (int32_t g0 = 0; g0 < cnt; g0 += 8)
+            // eight slots per 16-byte chunk load, two per word
+            auto rows_of = [&](const uint4* __restrict__ chunks, int64_t nch, int32_t cnt, auto nearRow) {
+                const uint4* __restrict__ at = chunks + chunk_word(row, 0, nch);
+                uint4 next = cnt > 0 ? __ldg(at) : make_uint4(0u, 0u, 0u, 0u);
+                for (int32_t left = cnt; left > 0; left -= 8)
                 {
-                    const uint4 c = __ldg(chunks + base + ((int64_t)(g0 >> 3) << 5));
-                    uint64_t lo = ((uint64_t)c.y << 32) | c.x, hi = ((uint64_t)c.w << 32) | c.z;
-                    const int32_t m = cnt - g0 < 8 ? cnt - g0 : 8;
-                    for (int32_t q = 0; q < m; ++q)
+                    uint4 c = next;
+                    at += 32;
+                    if (left > 8) next = __ldg(at);  // in flight while this chunk is worked on
+                    for (int32_t m = left < 8 ? left : 8; m > 0; m -= 2)
                     {
-                        const int32_t idx = (int32_t)(lo & 0xffffu);
-                        lo = (lo >> 16) | (hi << 48);
-                        hi >>= 16;
-                        pair(idx, nearRow);
+                        const int32_t i0 = (int32_t)(c.x & 0xffffu), i1 = m > 1 ? (int32_t)(c.x >> 16) : i0;
+                        c.x = c.y;
+                        c.y = c.z;
+                        c.z = c.w;
+                        pairs(i0, i1, m > 1, nearRow);
                     }
                 }
             };
-            rows_of(static_cast<const uint4*>(colsN), capN, cn, true);
-            rows_of(static_cast<const uint4*>(colsF), capF, cf, false);
+            rows_of(static_cast<const uint4*>(colsN), capN, cn, std::true_type{});
+            rows_of(static_cast<const uint4*>(colsF), capF, cf, std::false_type{});
         }
         else
         {
-            const int32_t* __restrict__ nI = static_cast<const int32_t*>(colsN) + mrmd_dev::nbr_row(row, capN);
-            const int32_t* __restrict__ fI = static_cast<const int32_t*>(colsF) + mrmd_dev::nbr_row(row, capF);
-#pragma unroll 2
-            for (int32_t k = 0; k < cn; ++k) pair(__ldg(nI + 32 * (int64_t)k), true);
-#pragma unroll 2
-            for (int32_t k = 0; k < cf; ++k) pair(__ldg(fI + 32 * (int64_t)k), false);
+            auto rows_of = [&](const int32_t* __restrict__ col, int32_t cnt, auto nearRow) {
+                for (int32_t k = 0; k < cnt; k += 2)
+                {
+                    const int32_t i0 = __ldg(col + 32 * (int64_t)k);
+                    const bool has1 = k + 1 < cnt;
+                    pairs(i0, has1 ? __ldg(col + 32 * (int64_t)(k + 1)) : i0, has1, nearRow);
+                }
+            };
+            rows_of(static_cast<const int32_t*>(colsN) + mrmd_dev::nbr_row(row, capN), cn, std::true_type{});
+            rows_of(static_cast<const int32_t*>(colsF) + mrmd_dev::nbr_row(row, capF), cf, std::false_type{});
         }
         // F = near double-float sum + far FP32 sum
         auto comp = [&](float h, float l, float gsum) -> double {
@@ -510,7 +579,7 @@ __global__ void __launch_bounds__(TILE_ROWS, 4) k_lj_tile(
     }
     // per-thread sums without the offsets (exact: the heads lie in
     // [bias, 2 bias)), then a double-float block reduction on the FP32 pipe
-    df v[5] = {fast_two_sum(__fsub_rn(s.s3h, tp.bias3), s.s3l), fast_two_sum(__fsub_rn(s.s6h, tp.bias6), s.s6l),
+    df v[5] = {fast_two_sum(__fsub_rn(s.sh.x, tp.bias3), s.sl.x), fast_two_sum(__fsub_rn(s.sh.y, tp.bias6), s.sl.y),
                df{(float)s.cnt, 0.f}, s.ec, s.wc};
     const int nv = CAP ? 5 : 3;
 #pragma unroll
@@ -554,12 +623,10 @@ __global__ void __launch_bounds__(TILE_ROWS, 4) k_lj_tile(
 
 namespace mrmd_impl
 {
-int tile_split_coords(mrmd_ctx* ctx, const double* pos4, int64_t n, const SplitParams& sp, float4* recA,
-                      float2* recB)
+int tile_split_coords(mrmd_ctx* ctx, const double* pos4, int64_t n, const SplitParams& sp, float4* rec)
 {
     if (n == 0) return MRMD_OK;
-    k_tile_split<<<grid_for(ctx, n, 256), 256, 0, ctx->stream>>>(reinterpret_cast<const double4*>(pos4), n, sp,
-                                                                 recA, recB);
+    k_tile_split<<<grid_for(ctx, n, 256), 256, 0, ctx->stream>>>(reinterpret_cast<const double4*>(pos4), n, sp, rec);
     return after_launch(ctx, "tile_split");
 }
 
@@ -625,7 +692,7 @@ void tile_build_done(TileList* tl, int32_t maxMembers, bool valid, int64_t total
 }
 
 int lj_tile_forces(mrmd_ctx* ctx, const TileList* tl, const mrmd_nlist* nearList, const mrmd_nlist* farList,
-                   const float4* recA, const float2* recB, double* force4, const TileParams& tp, double* ev,
+                   const float4* rec, double* force4, const TileParams& tp, double* ev,
                    int64_t nAll, bool gather)
 {
     const int64_t rows = nearList->rows;
@@ -640,7 +707,7 @@ int lj_tile_forces(mrmd_ctx* ctx, const TileList* tl, const mrmd_nlist* nearList
         const size_t smem = (size_t)stride * (sizeof(float4) + sizeof(float2));
 #define TILE_LAUNCH(CAPV)                                                                                          \
     k_lj_tile<true, CAPV><<<grid, TILE_ROWS, smem, ctx->stream>>>(                                                \
-        recA, recB, tl->members, tl->memberCount, stride, nearList->counts, tl->nearChunks, tl->nearChunksPerRow,  \
+        rec, tl->members, tl->memberCount, stride, nearList->counts, tl->nearChunks, tl->nearChunksPerRow,  \
         farList->counts, tl->farChunks, tl->farChunksPerRow, rows, nAll, f, tp, ev)
         if (cap)
             TILE_LAUNCH(true);
@@ -651,7 +718,7 @@ int lj_tile_forces(mrmd_ctx* ctx, const TileList* tl, const mrmd_nlist* nearList
     }
 #define GATHER_LAUNCH(CAPV)                                                                                        \
     k_lj_tile<false, CAPV><<<grid, TILE_ROWS, 0, ctx->stream>>>(                                                  \
-        recA, recB, nullptr, nullptr, 0, nearList->counts, nearList->nbrs, nearList->maxNeighbors, farList->counts, \
+        rec, nullptr, nullptr, 0, nearList->counts, nearList->nbrs, nearList->maxNeighbors, farList->counts, \
         farList->nbrs, farList->maxNeighbors, rows, nAll, f, tp, ev)
     if (cap)
         GATHER_LAUNCH(true);

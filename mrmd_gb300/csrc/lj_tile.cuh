@@ -11,8 +11,10 @@
 // FP32-accurate): r^2 is known as the float pair (S + C, rounding error) to
 // about 2^-44 relative.
 //
-// Records.  Per particle A = (hi.x, hi.y, hi.z, lo.x) and B = (lo.y, lo.z):
-// 24 bytes.  The stepper writes them in its kick/drift and ghost-update
+// Records.  Per particle rec[2 i] = (hi.x, hi.y, lo.x, lo.y) and rec[2 i + 1] =
+// (hi.z, lo.z, -, -): x and y of each part adjacent for the packed FP32
+// instructions, and the particle in one 32-byte sector (as separate 16- and
+// 8-byte arrays a gather moved two).  The stepper writes them in its kick/drift and ghost-update
 // kernels; the pair kernel copies the records of a tile's neighbours into
 // shared memory once per step.
 //
@@ -40,22 +42,22 @@ constexpr int TILE_CAP = 3072;
 // otherwise.
 bool tile_split_params(const double* origin, double extent, double rlist, SplitParams* out);
 
-// (A, B) records of one position: the split of each coordinate relative to
-// the origin (a multiple of Q) on the integer pipe (split_bits: the same bits
+// The record of one position: the split of each coordinate relative to the
+// origin (a multiple of Q) on the integer pipe (split_bits: the same bits
 // as rounding x + (magic - origin) to the Q grid in FP64; no FP64 operation).
-__device__ __forceinline__ void tile_split(const double4& x, const SplitParams& sp, float4& a, float2& b)
+__device__ __forceinline__ void tile_split(const double4& x, const SplitParams& sp, float4* __restrict__ rec,
+                                           int64_t i)
 {
-    float lx, ly, lz;
-    split_bits(x.x, sp.ko.x, sp.q, sp.invScaleF, a.x, lx);
-    split_bits(x.y, sp.ko.y, sp.q, sp.invScaleF, a.y, ly);
-    split_bits(x.z, sp.ko.z, sp.q, sp.invScaleF, a.z, lz);
-    a.w = lx;
-    b = make_float2(ly, lz);
+    float4 a, b = make_float4(0.f, 0.f, 0.f, 0.f);
+    split_bits(x.x, sp.ko.x, sp.q, sp.invScaleF, a.x, a.z);
+    split_bits(x.y, sp.ko.y, sp.q, sp.invScaleF, a.y, a.w);
+    split_bits(x.z, sp.ko.z, sp.q, sp.invScaleF, b.x, b.y);
+    rec[2 * i] = a;
+    rec[2 * i + 1] = b;
 }
 
-// Records of particles [0, n) into recA / recB.
-int tile_split_coords(mrmd_ctx* ctx, const double* pos4, int64_t n, const SplitParams& sp, float4* recA,
-                      float2* recB);
+// Records of particles [0, n) into rec.
+int tile_split_coords(mrmd_ctx* ctx, const double* pos4, int64_t n, const SplitParams& sp, float4* rec);
 
 // Rows of member slots in 8-entry chunks: chunk g of row i is the 16-byte
 // word (i / 32) * chunks * 32 + 32 g + i % 32 (chunks = ceil(capacity / 8)),
@@ -114,9 +116,8 @@ TileParams make_tile_params(const LJDev& p, double rcSqr, double rsplit, int64_t
 // Forces of local atoms [0, rows) written into force4 (overwritten, ghosts
 // untouched), energy and virial added into ev[0], ev[1].  With a valid tile
 // list the neighbour records come from shared-memory tiles; otherwise (or
-// with `gather` set) they are gathered from recA / recB through the int32
-// lists.
+// with `gather` set) they are gathered from rec through the int32 lists.
 int lj_tile_forces(mrmd_ctx* ctx, const TileList* tl, const mrmd_nlist* nearList, const mrmd_nlist* farList,
-                   const float4* recA, const float2* recB, double* force4, const TileParams& tp, double* ev,
+                   const float4* rec, double* force4, const TileParams& tp, double* ev,
                    int64_t nAll, bool gather);
 }  // namespace mrmd_impl

@@ -43,17 +43,6 @@ __device__ __forceinline__ void observe_add(double (&o)[4], const double4& v, do
     o[3] += v.z;
 }
 
-// Tile-kernel records (A, B) of one position.
-__device__ __forceinline__ void split_store(const double4& x, const SplitParams& sp, float4* __restrict__ recA,
-                                            float2* __restrict__ recB, int64_t i)
-{
-    float4 a;
-    float2 b;
-    tile_split(x, sp, a, b);
-    recA[i] = a;
-    recB[i] = b;
-}
-
 // OBS: the velocities after the post-kick are the full-step velocities of
 // the previous step; their kinetic energy and momentum go to rec[2..5] of
 // that step's record (deterministic grid sum).  SPLIT: the new positions'
@@ -64,7 +53,7 @@ template <bool OBS, bool SPLIT>
 __global__ void k_fused_kick_drift(double4* __restrict__ pos, double4* __restrict__ vel, double4* __restrict__ force,
                                    const double* __restrict__ mass, const double* __restrict__ dtfmOf, int64_t n,
                                    double dt, int postKick, double* partial, unsigned* ticket, double* rec,
-                                   SplitParams sp, float4* __restrict__ recA, float2* __restrict__ recB)
+                                   SplitParams sp, float4* __restrict__ atomRec)
 {
     double o[4] = {0.0, 0.0, 0.0, 0.0};
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
@@ -102,7 +91,7 @@ __global__ void k_fused_kick_drift(double4* __restrict__ pos, double4* __restric
         // the mixed form's pair kernel overwrites every local force (no
         // accumulation, ghosts unused): only the FP64 form needs the reset
         if (SPLIT)
-            split_store(x, sp, recA, recB, i);
+            tile_split(x, sp, atomRec, i);
         else
             force[i] = make_double4(0.0, 0.0, 0.0, 0.0);
     }
@@ -120,7 +109,7 @@ __global__ void k_kick_factors(const double* __restrict__ mass, int64_t n, doubl
 // coordinates.
 __global__ void k_ghost_update_split(double4* __restrict__ pos, const int32_t* __restrict__ corr, int64_t nLocal,
                                      int64_t nGhost, double3 L, double3 delta, SplitParams sp,
-                                     float4* __restrict__ recA, float2* __restrict__ recB)
+                                     float4* __restrict__ rec)
 {
     for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < nGhost;
          g += (int64_t)gridDim.x * blockDim.x)
@@ -129,7 +118,7 @@ __global__ void k_ghost_update_split(double4* __restrict__ pos, const int32_t* _
         if (!MRMD_IN_BOUNDS(corr[idx], nLocal)) continue;
         const double4 p = ghost_position(pos[idx], pos[corr[idx]], L, delta);
         pos[idx] = p;
-        split_store(p, sp, recA, recB, idx);
+        tile_split(p, sp, rec, idx);
     }
 }
 
@@ -221,8 +210,7 @@ struct mrmd_md
     CellGrid grid{};
     int32_t* orig = nullptr;     // original index of each local atom
     int32_t* origTmp = nullptr;
-    float4* recA = nullptr;      // mixed: tile-kernel records of local + ghost atoms
-    float2* recB = nullptr;
+    float4* rec = nullptr;       // mixed: tile-kernel records of local + ghost atoms, two per atom
     int64_t splitCap = 0;
     SplitParams sp{};            // mixed: the tile kernel's coordinate split
     TileList tiles;              // mixed: the split list as shared-memory tiles
@@ -301,12 +289,10 @@ int md_rebuild(mrmd_ctx* ctx, mrmd_md* md)
     MRMD_TRY(list_total_pairs(ctx, &md->list));
     if (full && nAll > md->splitCap)
     {
-        dfree(md->recA);
-        md->recA = nullptr;
-        md->recB = nullptr;
+        dfree(md->rec);
+        md->rec = nullptr;
         const int64_t c = nAll + nAll / 8 + 64;
-        MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&md->recA), (sizeof(float4) + sizeof(float2)) * (size_t)c));
-        md->recB = reinterpret_cast<float2*>(md->recA + c);
+        MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&md->rec), 2 * sizeof(float4) * (size_t)c));
         md->splitCap = c;
     }
     md->rebuilds++;
@@ -322,8 +308,8 @@ int md_forces(mrmd_ctx* ctx, mrmd_md* md, double* ev, bool splitDone = false)
     if (md->cfg.precision == MRMD_PREC_MIXED)
     {
         const int64_t nAll = a->numLocal + a->numGhost;
-        if (!splitDone) MRMD_TRY(tile_split_coords(ctx, a->pos, nAll, md->sp, md->recA, md->recB));
-        return lj_tile_forces(ctx, &md->tiles, &md->list, &md->farList, md->recA, md->recB, a->force, md->tp, ev,
+        if (!splitDone) MRMD_TRY(tile_split_coords(ctx, a->pos, nAll, md->sp, md->rec));
+        return lj_tile_forces(ctx, &md->tiles, &md->list, &md->farList, md->rec, a->force, md->tp, ev,
                               nAll, md->cfg.gatherNeighbours != 0);
     }
     MRMD_TRY(lj_apply_fp64(ctx, md->lj, a, &md->list, nullptr, ev));
@@ -344,7 +330,7 @@ int md_kick_drift(mrmd_ctx* ctx, mrmd_md* md, bool postKick, double* prevRec, bo
     k_fused_kick_drift<O, S><<<grid, TB, 0, ctx->stream>>>(                                                     \
         reinterpret_cast<double4*>(a->pos), reinterpret_cast<double4*>(a->vel),                                 \
         reinterpret_cast<double4*>(a->force), a->mass, md->dtfm, md->n, md->cfg.dt, postKick ? 1 : 0,         \
-        md->dPartial, md->dTicket, prevRec, md->sp, md->recA, md->recB)
+        md->dPartial, md->dTicket, prevRec, md->sp, md->rec)
     if (obs && split) KD_LAUNCH(true, true);
     else if (obs) KD_LAUNCH(true, false);
     else if (split) KD_LAUNCH(false, true);
@@ -376,8 +362,7 @@ int md_plain_step(mrmd_ctx* ctx, mrmd_md* md, double* rec, double* prevRec, bool
         k_ghost_update_split<<<grid_for(ctx, a->numGhost, TB), TB, 0, ctx->stream>>>(
             reinterpret_cast<double4*>(a->pos), g->correspondingRealAtom, a->numLocal, a->numGhost,
             make_double3(sd.diameter[0], sd.diameter[1], sd.diameter[2]),
-            make_double3(0.1 * sd.diameter[0], 0.1 * sd.diameter[1], 0.1 * sd.diameter[2]), md->sp, md->recA,
-            md->recB);
+            make_double3(0.1 * sd.diameter[0], 0.1 * sd.diameter[1], 0.1 * sd.diameter[2]), md->sp, md->rec);
         MRMD_TRY(after_launch(ctx, "ghost_update_split"));
     }
     return md_forces(ctx, md, rec, true);
@@ -553,7 +538,7 @@ int mrmd_md_destroy(mrmd_ctx* ctx, mrmd_md* md)
     md->tiles.release();
     dfree(md->orig);
     dfree(md->origTmp);
-    dfree(md->recA);
+    dfree(md->rec);
     dfree(md->dEnergy);
     dfree(md->dPartial);
     dfree(md->dtfm);
@@ -751,7 +736,7 @@ int mrmd_md_eval(mrmd_ctx* ctx, mrmd_md* md, int what, double* ev2)
     {
         if (md->needRebuild || !md->forceValid) return set_error(ctx, MRMD_ERR_STATE, "no list: run or eval first");
         if (md->cfg.precision == MRMD_PREC_MIXED)
-            return lj_tile_forces(ctx, &md->tiles, &md->list, &md->farList, md->recA, md->recB, a->force, md->tp,
+            return lj_tile_forces(ctx, &md->tiles, &md->list, &md->farList, md->rec, a->force, md->tp,
                                   ev, a->numLocal + a->numGhost, md->cfg.gatherNeighbours != 0);
         return lj_apply_fp64(ctx, md->lj, a, &md->list, nullptr, ev);
     }
