@@ -86,76 +86,131 @@ struct LJIGArgs
     double* energyOut;
 };
 
-template <bool MIXED>
-__global__ void __launch_bounds__(128) k_ljig(LJIGArgs A)
+constexpr int IG_TB = 128;
+constexpr int IG_CHUNK = 40;  // list entries of a row scanned at a time
+
+// Adds v to three components unless they are all zero (most molecule forces:
+// only pairs with a hybrid member have one).
+__device__ __forceinline__ void add3(double* f, const double (&v)[3])
 {
-    // action/LJ_IdealGas.cpp:52-225, one thread per local molecule alpha
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+        if ((__double_as_longlong(v[d]) << 1) != 0) atomicAdd(f + d, v[d]);
+}
+
+// action/LJ_IdealGas.cpp:52-225, LANES lanes per local molecule alpha.  As in
+// the FP64 pair kernel the entries are scanned first: pairs of two
+// coarse-grained molecules and, between single-site molecules, those surely
+// beyond the cutoff (FP32 lower bound) drop out, the rest is dealt to the
+// row's lanes.  A single-site alpha's force stays in registers, and a beta's
+// molecule force is added only where the drift term gives one (per entry,
+// in range or not, six of nine atomics were those).  34,560 molecules 105 us
+// with one lane per row and all entries in FP64.
+template <bool MIXED, bool MULTI, int LANES>
+__global__ void __launch_bounds__(IG_TB) k_ljig(LJIGArgs A, LJDev p0)
+{
+    constexpr unsigned ALL = 0xffffffffu;
     __shared__ double red[64];
+    __shared__ uint8_t segS[IG_TB / LANES][IG_CHUNK];
+    const int lane = threadIdx.x & 31, sub = lane % LANES;
+    const unsigned mine = ((1u << LANES) - 1u) << (lane & ~(LANES - 1)), before = mine & ((1u << lane) - 1u);
+    uint8_t* seg = segS[threadIdx.x / LANES];
     double sumEnergy = 0.0, dummy = 0.0;
-    const int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (row < A.nMol)
+    const int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / LANES;
+    const bool live = row < A.nMol;
+    const int64_t alpha = A.begin + (live ? row : 0);
+    const int32_t cnt = live ? A.counts[row] : 0;
+    const double modA = A.m.modulatedLambda[alpha];
+    const bool cgA = le_zero(modA), hyA = !(ge_one(modA) || cgA);
+    const int binAlpha = hyA ? comp_bin(A.m.lambda[alpha]) : -1;
+    const double4 gA = reinterpret_cast<const double4*>(A.m.gradLambda)[alpha];
+    const int64_t sA = A.m.atomsOffset[alpha], nA = live ? A.m.numAtoms[alpha] : 0;
+    const bool oneA = nA == 1;
+    double4 pA = make_double4(0.0, 0.0, 0.0, 0.0);
+    if (oneA) pA = A.apos[sA];
+    const float3 pf = make_float3(hi_word_f32(pA.x), hi_word_f32(pA.y), hi_word_f32(pA.z));
+    const float rcUp = (float)A.rcSqr * 1.000001f;
+    const int32_t* __restrict__ col = A.nbrs + mrmd_dev::nbr_row(live ? row : 0, A.cap);
+    double fA[3] = {0.0, 0.0, 0.0};   // molecule force of alpha
+    double fAt[3] = {0.0, 0.0, 0.0};  // force on alpha's only site
+    int32_t most = cnt;
+#pragma unroll
+    for (int o = 16; o >= LANES; o >>= 1) most = max(most, __shfl_xor_sync(ALL, most, o));
+    for (int32_t k0 = 0; k0 < most; k0 += IG_CHUNK)
     {
-        const int64_t alpha = A.begin + row;
-        double fA[3] = {0.0, 0.0, 0.0};
-        const double modA = A.m.modulatedLambda[alpha];
-        int binAlpha = -1;
-        if (is_hy(modA)) binAlpha = comp_bin(A.m.lambda[alpha]);
-        const double4 gA = reinterpret_cast<const double4*>(A.m.gradLambda)[alpha];
-        const int64_t sA = A.m.atomsOffset[alpha], eA = sA + A.m.numAtoms[alpha];
-        const int32_t cnt = A.counts[row];
-        for (int32_t k = 0; k < cnt; ++k)
+        int32_t kept = 0;
+        const int32_t kEnd = min(k0 + IG_CHUNK, most);
+#pragma unroll 2
+        for (int32_t kk = k0; kk < kEnd; kk += LANES)
         {
-            const int64_t beta = A.nbrs[mrmd_dev::nbr_row(row, A.cap) + 32 * (int64_t)k];
-            double fB[3] = {0.0, 0.0, 0.0};
+            const int32_t k = kk + sub;
+            bool keep = k < cnt;
+            if (keep)
+            {
+                const int64_t beta = col[32 * (int64_t)k];
+                if (cgA) keep = !le_zero(A.m.modulatedLambda[beta]);
+                if (keep && oneA && A.m.numAtoms[beta] == 1)
+                    keep = !surely_beyond(pf, mrmd_dev::ldg4(A.apos + A.m.atomsOffset[beta]), rcUp);
+            }
+            const unsigned m = __ballot_sync(ALL, keep);
+            if (keep) seg[kept + __popc(m & before)] = (uint8_t)(k - k0);
+            kept += __popc(m & mine);
+        }
+        __syncwarp();
+        for (int32_t q = sub; q < kept; q += LANES)
+        {
+            const int64_t beta = col[32 * (int64_t)(k0 + seg[q])];
             const double modB = A.m.modulatedLambda[beta];
-            if (is_cg(modA) && is_cg(modB)) continue;
             const double4 gB = reinterpret_cast<const double4*>(A.m.gradLambda)[beta];
             const double weighting = 0.5 * (modA + modB);
-            const bool hyPair = is_hy(modA) || is_hy(modB);
+            const bool hyB = !(ge_one(modB) || le_zero(modB)), hyPair = hyA || hyB;
             const int64_t sB = A.m.atomsOffset[beta], eB = sB + A.m.numAtoms[beta];
-            int binBeta = -1;
-            if (A.sampling && is_hy(modB)) binBeta = comp_bin(A.m.lambda[beta]);
-            for (int64_t idx = sA; idx < eA; ++idx)
+            const int binBeta = A.sampling && hyB ? comp_bin(A.m.lambda[beta]) : -1;
+            double fB[3] = {0.0, 0.0, 0.0};
+            for (int64_t idx = sA; idx < sA + nA; ++idx)
             {
-                const double4 pi = A.apos[idx];
+                const double4 pi = oneA ? pA : A.apos[idx];
                 double fi[3] = {0.0, 0.0, 0.0};
-                const int32_t ti = A.atype[idx];
+                const int32_t ti = MULTI || A.sampling ? A.atype[idx] : 0;
                 for (int64_t jdx = sB; jdx < eB; ++jdx)
                 {
-                    const int32_t tj = A.atype[jdx];
-                    const LJDev& p = A.table[ti * A.numTypes + tj];
+                    const int32_t tj = MULTI || A.sampling ? A.atype[jdx] : 0;
+                    const LJDev& p = MULTI ? A.table[ti * A.numTypes + tj] : p0;
                     double ff, e, dx, dy, dz;
                     if (MIXED)
                     {
-                        PairMixed q;
-                        if (!pair_mixed(A.hi[idx], A.lo[idx], A.hi[jdx], A.lo[jdx], p, A.rc2, q)) continue;
-                        ff = (double)q.ff.h + (double)q.ff.l;
-                        e = q.e;
-                        dx = (double)q.dh.x + (double)q.dl.x;
-                        dy = (double)q.dh.y + (double)q.dl.y;
-                        dz = (double)q.dh.z + (double)q.dl.z;
+                        // the float pairs as doubles: exact conversions on
+                        // the integer pipe and one FP64 addition
+                        PairMixed q2;
+                        if (!pair_mixed(A.hi[idx], A.lo[idx], A.hi[jdx], A.lo[jdx], p, A.rc2, q2)) continue;
+                        ff = __dadd_rn(f32_to_f64(q2.ff.h), f32_to_f64(q2.ff.l));
+                        e = f32_to_f64(q2.e);
+                        dx = __dadd_rn(f32_to_f64(q2.dh.x), f32_to_f64(q2.dl.x));
+                        dy = __dadd_rn(f32_to_f64(q2.dh.y), f32_to_f64(q2.dl.y));
+                        dz = __dadd_rn(f32_to_f64(q2.dh.z), f32_to_f64(q2.dl.z));
                     }
                     else
                     {
-                        const double4 pj = A.apos[jdx];
+                        const double4 pj = mrmd_dev::ldg4(A.apos + jdx);
                         dx = pi.x - pj.x;
                         dy = pi.y - pj.y;
                         dz = pi.z - pj.z;
                         const double distSqr = dx * dx + dy * dy + dz * dz;
-                        if (distSqr > A.rcSqr) continue;
-                        lj_eval_fp64(p, distSqr, ff, e);
+                        if (gt_nonneg(distSqr, A.rcSqr)) continue;
+                        lj_eval_series(p, distSqr, ff, e);
                     }
                     const double ffactor = ff * weighting;
-                    fi[0] += dx * ffactor;
-                    fi[1] += dy * ffactor;
-                    fi[2] += dz * ffactor;
-                    atomicAdd(A.aforce + 4 * jdx + 0, -(dx * ffactor));
-                    atomicAdd(A.aforce + 4 * jdx + 1, -(dy * ffactor));
-                    atomicAdd(A.aforce + 4 * jdx + 2, -(dz * ffactor));
+                    const double gx = dx * -ffactor, gy = dy * -ffactor, gz = dz * -ffactor;
+                    fi[0] -= gx;
+                    fi[1] -= gy;
+                    fi[2] -= gz;
+                    atomicAdd(A.aforce + 4 * jdx + 0, gx);
+                    atomicAdd(A.aforce + 4 * jdx + 1, gy);
+                    atomicAdd(A.aforce + 4 * jdx + 2, gz);
                     sumEnergy += e * weighting;
-                    const double Vij = 0.5 * e;
                     if (hyPair)
                     {
+                        const double Vij = 0.5 * e;
                         fA[0] += -Vij * gA.x;
                         fA[1] += -Vij * gA.y;
                         fA[2] += -Vij * gA.z;
@@ -164,35 +219,45 @@ __global__ void __launch_bounds__(128) k_ljig(LJIGArgs A)
                         fB[2] += -Vij * gB.z;
                         if (A.sampling)
                         {
-                            if (is_hy(modA) && binAlpha != -1)
-                                atomicAdd(A.compEnergy + binAlpha * A.numTypes + ti, Vij);
-                            if (is_hy(modB) && binBeta != -1)
-                                atomicAdd(A.compEnergy + binBeta * A.numTypes + tj, Vij);
+                            if (binAlpha != -1) atomicAdd(A.compEnergy + binAlpha * A.numTypes + ti, Vij);
+                            if (binBeta != -1) atomicAdd(A.compEnergy + binBeta * A.numTypes + tj, Vij);
                         }
                     }
                 }
-                atomicAdd(A.aforce + 4 * idx + 0, fi[0]);
-                atomicAdd(A.aforce + 4 * idx + 1, fi[1]);
-                atomicAdd(A.aforce + 4 * idx + 2, fi[2]);
+                if (oneA)
+                {
+                    fAt[0] += fi[0];
+                    fAt[1] += fi[1];
+                    fAt[2] += fi[2];
+                }
+                else
+                    add3(A.aforce + 4 * idx, fi);
             }
-            double* mf = A.m.force + 4 * beta;
-            atomicAdd(mf + 0, fB[0]);
-            atomicAdd(mf + 1, fB[1]);
-            atomicAdd(mf + 2, fB[2]);
+            if (hyPair) add3(A.m.force + 4 * beta, fB);
         }
-        if (A.sampling && is_hy(modA) && binAlpha != -1)
-            for (int64_t a = sA; a < eA; ++a) atomicAdd(A.compCounter + binAlpha * A.numTypes + A.atype[a], 1.0);
-        if (is_hy(modA) && binAlpha != -1)
+        __syncwarp();
+    }
+#pragma unroll
+    for (int o = 1; o < LANES; o <<= 1)
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
         {
+            fA[d] += __shfl_xor_sync(ALL, fA[d], o);
+            fAt[d] += __shfl_xor_sync(ALL, fAt[d], o);
+        }
+    if (live && sub == 0)
+    {
+        if (hyA && binAlpha != -1)
+        {
+            if (A.sampling)
+                for (int64_t a = sA; a < sA + nA; ++a) atomicAdd(A.compCounter + binAlpha * A.numTypes + A.atype[a], 1.0);
             const double me = A.meanComp[binAlpha * A.numTypes + A.atype[sA]];
             fA[0] += me * gA.x;
             fA[1] += me * gA.y;
             fA[2] += me * gA.z;
         }
-        double* mf = A.m.force + 4 * alpha;
-        atomicAdd(mf + 0, fA[0]);
-        atomicAdd(mf + 1, fA[1]);
-        atomicAdd(mf + 2, fA[2]);
+        if (oneA) add3(A.aforce + 4 * sA, fAt);
+        add3(A.m.force + 4 * alpha, fA);
     }
     mrmd_dev::block_sum2(sumEnergy, dummy, red);
     if (threadIdx.x == 0) atomicAdd(A.energyOut, sumEnergy);
@@ -336,7 +401,6 @@ int ljig_run_async(mrmd_ctx* ctx, mrmd_ljig* s, mrmd_molecules* m, const mrmd_nl
     A.energyOut = ev;
     if (A.nMol > 0)
     {
-        const unsigned grid = (unsigned)div_up(A.nMol, 128);
         if (precision == MRMD_PREC_MIXED)
         {
             if (hiIn && loIn)
@@ -353,12 +417,31 @@ int ljig_run_async(mrmd_ctx* ctx, mrmd_ljig* s, mrmd_molecules* m, const mrmd_nl
                 A.hi = hi;
                 A.lo = hi + nAll;
             }
-            k_ljig<true><<<grid, 128, 0, ctx->stream>>>(A);
+        }
+        const LJDev p0 = to_dev(s->table[0]);
+        const bool mixed = precision == MRMD_PREC_MIXED, multi = s->numTypes > 1;
+        auto launch = [&](auto kernel, int lanes) {
+            kernel<<<(unsigned)div_up(A.nMol * lanes, IG_TB), IG_TB, 0, ctx->stream>>>(A, p0);
+        };
+#define LJIG_LANES(L)                                        \
+    if (mixed && multi) launch(k_ljig<true, true, L>, L);    \
+    else if (mixed) launch(k_ljig<true, false, L>, L);       \
+    else if (multi) launch(k_ljig<false, true, L>, L);       \
+    else launch(k_ljig<false, false, L>, L)
+        // us of the action with 1 / 2 / 4 / 8 lanes (one lane per row, every
+        // entry evaluated, before): 9,216 molecules 81 / 53 / 42 / 44 (103),
+        // 34,560 91 / 64 / 66 / 78 (102), 117,600 103 / 102 / 114 / 164
+        // (140), 460,800 533 / 485 / 545 / 795 (704), 156,800 of three sites
+        // 1088 / 644 / 594 / 610 (1260)
+        if (A.nMol < 130 * (int64_t)ctx->numSMs)
+        {
+            LJIG_LANES(4);
         }
         else
         {
-            k_ljig<false><<<grid, 128, 0, ctx->stream>>>(A);
+            LJIG_LANES(2);
         }
+#undef LJIG_LANES
         MRMD_TRY(after_launch(ctx, "ljig"));
     }
     if (s->runCounter % s->updateInterval == 0)

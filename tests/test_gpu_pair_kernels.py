@@ -192,3 +192,43 @@ def test_sparse_box_keeps_full_radius_cells(M):
     vl = M.HalfVerletList()
     vl.build(a, 0, 4, 2.8, 1.0, [0.0] * 3, [L] * 3, 8)
     assert vl.total_pairs == 2
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("n,box,apm", [(2200, (40.0, 9.0, 9.0), 3), (19759, (110.0, 19.0, 19.0), 1),
+                                       (19761, (110.0, 19.0, 19.0), 1), (20001, (110.0, 19.0, 19.0), 2)])
+def test_lj_ideal_gas_lanes(M, orc, n, box, apm, prec):
+    """LJ_IdealGas with four lanes per molecule (below 19,760 molecules on 152
+    SMs) and two, single- and multi-site, rows of more than one chunk (random
+    placement, density 0.2 to 0.5): forces before the fold-back and the energy
+    against the oracle, by the bars of the FP64 and the mixed form."""
+    from test_gpu_adress import adress_system, upload_molecules
+
+    mo, ao, corr, sd, slab, (rc, skin, _) = adress_system(orc, n, box, 17, apm)
+    co, no = orc.build_half_list(mo.pos, mo.numLocal + mo.numGhost, 0, mo.numLocal, rc + skin, sd.minGhostCorner,
+                                 sd.maxGhostCorner, 1.0, 256)
+    assert co.max() > 40
+    ig_o = orc.LJIdealGas(0.8, rc, 1.0, 1.0, True)
+    ao.force[:] = 0
+    mo.force[:] = 0
+    Eo = ig_o.run(mo, co, no, ao)
+    na, nm = ao.n, mo.numLocal + mo.numGhost
+    a = M.Atoms.from_arrays(ao.pos[:na], relative_mass=ao.relativeMass[:na], capacity=ao.capacity)
+    a.numLocalAtoms, a.numGhostAtoms = ao.numLocal, ao.numGhost
+    m = upload_molecules(M, mo, mo.numLocal, mo.numGhost)
+    m.setForce(0.0)
+    a.setForce(0.0)
+    vl = M.HalfVerletList()
+    vl.build(m, 0, mo.numLocal, rc + skin, 1.0, sd.minGhostCorner[:], sd.maxGhostCorner[:], 60)
+    ig = M.LJ_IdealGas(0.8, rc, 1.0, 1.0, True)
+    E = ig.run(m, vl, a, M.PREC_FP64 if prec == "fp64" else M.PREC_MIXED)
+    F, Fm = a.getForce(), m.download()["force"]
+    Fo, Fmo = ao.force[:na], mo.force[:nm]
+    if prec == "fp64":
+        assert_fp64_forces(F, Fo)
+        assert_fp64_forces(Fm, Fmo)
+        assert abs(E - Eo) <= 1e-10 * abs(Eo)
+    else:
+        rms = np.sqrt((Fo ** 2).sum(1).mean())
+        assert np.linalg.norm(F - Fo, axis=1).max() <= 1e-6 * rms
+        assert abs(E - Eo) <= 1e-7 * abs(Eo)
