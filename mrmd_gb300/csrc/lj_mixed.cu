@@ -81,46 +81,99 @@ struct Acc
 
 };
 
-template <bool PRED>
+constexpr int MX_CHUNK = 40;  // list entries of a row scanned at a time
+
+// One list row per LANES lanes.  As in the FP64 kernel the row's entries are
+// tested first (on the heads of the split coordinates, which bound r from
+// below: each component's low parts differ by at most one quantum), then the
+// ones that may be in range are dealt to the row's lanes; the evaluation is
+// some 200 FP32 instructions, and a third of the entries are out of range.
+// The forces become doubles by integer conversions (two FP64 conversions and
+// an addition per component before: the FP64 pipe bound the kernel).
+// Measured times: lj_mixed_half.
+template <bool PRED, int LANES>
 __global__ void __launch_bounds__(MX_TB) k_lj_mixed_half(
     const float4* __restrict__ hi, const float4* __restrict__ lo, const double4* __restrict__ pos,
-    double* __restrict__ force, const LJDev p, RcSq rc2, const int32_t* __restrict__ counts,
+    double* __restrict__ force, const LJDev p, RcSq rc2, float rcReach, const int32_t* __restrict__ counts,
     const int32_t* __restrict__ nbrs, int64_t cap, int64_t n, int64_t begin, int64_t nAll, mrmd_dev::Pred pred,
     double* __restrict__ ev)
 {
+    constexpr unsigned ALL = 0xffffffffu;
     __shared__ double red[64];
+    __shared__ uint8_t segS[MX_TB / LANES][MX_CHUNK];
+    const int lane = threadIdx.x & 31, sub = lane % LANES;
+    const unsigned mine = (LANES == 32 ? ALL : ((1u << LANES) - 1u)) << (lane & ~(LANES - 1));
+    const unsigned before = mine & ((1u << lane) - 1u);
+    uint8_t* seg = segS[threadIdx.x / LANES];
     Acc acc;
-    const int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (row < n)
+    const int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / LANES;
+    const bool live = row < n;
+    // list row `row` belongs to particle begin + row (the list's range)
+    const int64_t i = begin + (live ? row : 0);
+    const float4 hi_i = hi[i], lo_i = lo[i];
+    double4 pi;
+    if (PRED) pi = pos[i];
+    const int32_t cnt = live ? counts[row] : 0;
+    const int32_t* __restrict__ col = nbrs + mrmd_dev::nbr_row(live ? row : 0, cap);
+    int32_t most = cnt;
+#pragma unroll
+    for (int o = 16; o >= LANES; o >>= 1) most = max(most, __shfl_xor_sync(ALL, most, o));
+    for (int32_t k0 = 0; k0 < most; k0 += MX_CHUNK)
     {
-        // list row `row` belongs to particle begin + row (the list's range)
-        const int64_t i = begin + row;
-        const float4 hi_i = hi[i], lo_i = lo[i];
-        double4 pi;
-        if (PRED) pi = pos[i];
-        const int32_t cnt = counts[row];
-        const int32_t* __restrict__ col = nbrs + mrmd_dev::nbr_row(row, cap);
-        for (int32_t k = 0; k < cnt; ++k)
+        int32_t kept = 0;
+        const int32_t kEnd = min(k0 + MX_CHUNK, most);
+#pragma unroll 4
+        for (int32_t kk = k0; kk < kEnd; kk += LANES)
         {
-            const int32_t j = __ldg(col + 32 * (int64_t)k);
-            if (!MRMD_IN_BOUNDS(j, nAll)) continue;
-            if (PRED)
+            const int32_t k = kk + sub;
+            bool keep = k < cnt;
+            if (keep)
             {
-                const double4 pj = mrmd_dev::ldg4(pos + j);
-                if (!mrmd_dev::pred2(pred, pi.x, pi.y, pi.z, pj.x, pj.y, pj.z)) continue;
+                const int32_t j = __ldg(col + 32 * (int64_t)k);
+                keep = MRMD_IN_BOUNDS(j, nAll);
+                if (keep)
+                {
+                    const float4 hj = __ldg(hi + j);
+                    const float dx = hi_i.x - hj.x, dy = hi_i.y - hj.y, dz = hi_i.z - hj.z;
+                    keep = !(__fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz)) > rcReach);
+                    if (PRED && keep)
+                    {
+                        const double4 pj = mrmd_dev::ldg4(pos + j);
+                        keep = mrmd_dev::pred2(pred, pi.x, pi.y, pi.z, pj.x, pj.y, pj.z);
+                    }
+                }
             }
-            PairMixed q;
-            if (!pair_mixed(hi_i, lo_i, __ldg(hi + j), __ldg(lo + j), p, rc2, q)) continue;
-            acc.add(q);
-            atomicAdd(force + 4 * (int64_t)j + 0, -prod_d(q.dh.x, q.dl.x, q.ff));
-            atomicAdd(force + 4 * (int64_t)j + 1, -prod_d(q.dh.y, q.dl.y, q.ff));
-            atomicAdd(force + 4 * (int64_t)j + 2, -prod_d(q.dh.z, q.dl.z, q.ff));
+            const unsigned m = __ballot_sync(ALL, keep);
+            if (keep) seg[kept + __popc(m & before)] = (uint8_t)(k - k0);
+            kept += __popc(m & mine);
         }
-        atomicAdd(force + 4 * i + 0, (double)acc.fx.h + (double)acc.fx.l);
-        atomicAdd(force + 4 * i + 1, (double)acc.fy.h + (double)acc.fy.l);
-        atomicAdd(force + 4 * i + 2, (double)acc.fz.h + (double)acc.fz.l);
+        __syncwarp();
+        for (int32_t q = sub; q < kept; q += LANES)
+        {
+            const int32_t j = __ldg(col + 32 * (int64_t)(k0 + seg[q]));
+            PairMixed f;
+            if (!pair_mixed(hi_i, lo_i, __ldg(hi + j), __ldg(lo + j), p, rc2, f)) continue;
+            acc.add(f);
+            // -(dh + dl) ff: the product of the turned force factor
+            const df nff = {-f.ff.h, -f.ff.l};
+            atomicAdd(force + 4 * (int64_t)j + 0, prod_d(f.dh.x, f.dl.x, nff));
+            atomicAdd(force + 4 * (int64_t)j + 1, prod_d(f.dh.y, f.dl.y, nff));
+            atomicAdd(force + 4 * (int64_t)j + 2, prod_d(f.dh.z, f.dl.z, nff));
+        }
+        __syncwarp();
     }
-    double e = (double)acc.e.h + (double)acc.e.l, w = (double)acc.w.h + (double)acc.w.l;
+    double g[3] = {__dadd_rn(f32_to_f64(acc.fx.h), f32_to_f64(acc.fx.l)),
+                   __dadd_rn(f32_to_f64(acc.fy.h), f32_to_f64(acc.fy.l)),
+                   __dadd_rn(f32_to_f64(acc.fz.h), f32_to_f64(acc.fz.l))};
+#pragma unroll
+    for (int o = 1; o < LANES; o <<= 1)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) g[d] += __shfl_xor_sync(ALL, g[d], o);
+    if (live && sub == 0)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) atomicAdd(force + 4 * i + d, g[d]);
+    double e = __dadd_rn(f32_to_f64(acc.e.h), f32_to_f64(acc.e.l));
+    double w = __dadd_rn(f32_to_f64(acc.w.h), f32_to_f64(acc.w.l));
     mrmd_dev::block_sum2(e, w, red);
     if (threadIdx.x == 0)
     {
@@ -137,16 +190,42 @@ int lj_mixed_half(mrmd_ctx* ctx, const float4* hi, const float4* lo, const mrmd_
     const int64_t n = nl->rows;
     if (n == 0) return MRMD_OK;
     const bool usePred = pred != nullptr && pred->kind != MRMD_PRED_ALWAYS;
-    const unsigned grid = (unsigned)div_up(n, MX_TB);
     const mrmd_dev::Pred dp = to_dev_pred(pred);
     const RcSq rc2 = make_rcsq(lj->rcSqr);
     const double4* pos = reinterpret_cast<const double4*>(a->pos);
-    if (usePred)
-        k_lj_mixed_half<true><<<grid, MX_TB, 0, ctx->stream>>>(hi, lo, pos, a->force, lj->p0, rc2, nl->counts,
-                                                               nl->nbrs, nl->maxNeighbors, n, nl->begin, a->numLocal + a->numGhost, dp, ev);
+    // |dl| is at most one quantum per component: a pair within rc has heads
+    // within rc + sqrt(3) quanta
+    const double reach = std::sqrt(lj->rcSqr) + 1.7320509 * split_params_for(nl).invScale;
+    const float rcReach = (float)(reach * reach * (1.0 + 1e-6));
+    auto launch = [&](auto kernel, int lanes) {
+        kernel<<<(unsigned)div_up(n * lanes, MX_TB), MX_TB, 0, ctx->stream>>>(
+            hi, lo, pos, a->force, lj->p0, rc2, rcReach, nl->counts, nl->nbrs, nl->maxNeighbors, n, nl->begin,
+            a->numLocal + a->numGhost, dp, ev);
+    };
+#define MX_LANES(L)                                       \
+    if (usePred) launch(k_lj_mixed_half<true, L>, L);     \
+    else launch(k_lj_mixed_half<false, L>, L)
+    // lanes per row: us with 1 / 2 / 4 / 8 lanes (one lane per row, every entry
+    // evaluated, FP64 conversions, before)
+    //       4,000 atoms   50 /  31 /  23 /  19   (60)
+    //      32,000         53 /  40 /  37 /  44   (69)
+    //      87,808         80 /  73 /  71 /  83   (125)
+    //     256,000        185 / 158 / 161 / 204   (327)
+    //   4,000,000       2112 / 2030 / 2235 / 2958   (4536)
+    const int64_t sms = ctx->numSMs;
+    if (n < 40 * sms)
+    {
+        MX_LANES(8);
+    }
+    else if (n < 640 * sms)
+    {
+        MX_LANES(4);
+    }
     else
-        k_lj_mixed_half<false><<<grid, MX_TB, 0, ctx->stream>>>(hi, lo, pos, a->force, lj->p0, rc2, nl->counts,
-                                                                nl->nbrs, nl->maxNeighbors, n, nl->begin, a->numLocal + a->numGhost, dp, ev);
+    {
+        MX_LANES(2);
+    }
+#undef MX_LANES
     return after_launch(ctx, "lj_mixed_half");
 }
 

@@ -154,13 +154,14 @@ __device__ __forceinline__ void df_acc_prod(df& s, float dh, float dl, const df&
     s.l += t.l + e;
 }
 
-// The same product as a double (for FP64 atomics of the j-force).
+// The same product as a double (for FP64 atomics of the j-force): two exact
+// conversions on the integer pipe and one FP64 addition.
 __device__ __forceinline__ double prod_d(float dh, float dl, const df& ff)
 {
     const float p = dh * ff.h;
     float e = __fmaf_rn(dh, ff.h, -p);
     e = __fmaf_rn(dh, ff.l, e);
     e = __fmaf_rn(dl, ff.h, e);
-    return (double)p + (double)e;
+    return __dadd_rn(f32_to_f64(p), f32_to_f64(e));
 }
 }  // namespace mrmd_impl

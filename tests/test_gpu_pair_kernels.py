@@ -232,3 +232,24 @@ def test_lj_ideal_gas_lanes(M, orc, n, box, apm, prec):
         rms = np.sqrt((Fo ** 2).sum(1).mean())
         assert np.linalg.norm(F - Fo, axis=1).max() <= 1e-6 * rms
         assert abs(E - Eo) <= 1e-7 * abs(Eo)
+
+
+# Eight lanes per row below 6,080 atoms on 152 SMs, four below 97,280, two
+# above; rows of more than 40 entries (several chunks) with rc 4.
+@pytest.mark.parametrize("cells,drop,rc,cap,pred,lo", [
+    (4, 255, 2.5, 0.0, None, [0.0, 0.0, 0.0]),
+    (5, 3, 2.5, 0.95, None, [-3.0, 2.5, 0.0]),
+    (12, 833, 2.5, 0.0, "either", [0.0, 0.0, 0.0]),      # 6,079
+    (12, 831, 4.0, 0.95, None, [0.0, 0.0, 0.0]),         # 6,081
+    (29, 277, 2.5, 0.95, "both", [0.0, 0.0, 0.0]),       # 97,279
+    (29, 275, 3.2, 0.0, None, [100.0, -100.0, 0.1]),     # 97,281
+])
+def test_mixed_half_lanes(M, orc, cells, drop, rc, cap, pred, lo):
+    """Forces within the mixed form's bar of the oracle's (1e-6 of the rms
+    force), the energy within 1e-7."""
+    pos, L = fluid(cells, drop, 0.8 if cells > 4 else 0.4, cells + drop, lo)
+    (Fo, Eo, Wo), gpu = both(M, orc, pos, lo, L, rc, orc.lj_table(cap, rc, 1.0, 1.0, 1, True), pred)
+    F, E, W = gpu(M.LennardJones(rc, 1.0, 1.0, cap, is_shifted=True), M.PREC_MIXED)
+    rms = np.sqrt((Fo ** 2).sum(1).mean())
+    assert np.linalg.norm(F - Fo, axis=1).max() <= 1e-6 * rms
+    assert abs(E - Eo) <= 1e-7 * abs(Eo)
