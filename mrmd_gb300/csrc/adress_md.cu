@@ -70,7 +70,6 @@ int ad_rebuild(mrmd_ctx* ctx, mrmd_adress* s)
     const double rlist = s->cfg.rc + s->cfg.skin;
     MRMD_TRY(build_half_list(ctx, &s->list, m->pos, nM, 0, m->numLocal, rlist, s->grid,
                              s->list.maxNeighbors > 0 ? s->list.maxNeighbors : s->cfg.maxNeighbors, false));
-    MRMD_TRY(list_total_pairs(ctx, &s->list));
     const int64_t nA = a->numLocal + a->numGhost;
     if (s->cfg.precision == MRMD_PREC_MIXED && nA > s->splitCap)
     {

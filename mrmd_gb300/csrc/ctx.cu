@@ -155,12 +155,15 @@ void* scratch(mrmd_ctx* ctx, size_t bytes)
 }
 
 // ------------------------------------------------------------------ scan --
-// Three-phase exclusive scan: per-tile scan with tile totals, scan of the
-// tile totals (recursively), add offsets.  Tiles are 1024 items handled by
-// 256 threads x 4 items.
+// Exclusive scan in two launches (one for a single tile): per-tile scans with
+// tile totals, then every tile sums the totals before it and adds them.  Above
+// SCAN_DIRECT tiles, where those sums would cost more than another level, the
+// totals are scanned themselves first.  Tiles are 1024 items handled by 256
+// threads x 4 items.
 constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 4;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
+constexpr int64_t SCAN_DIRECT = 2048;
 
 template <typename T>
 __device__ __forceinline__ T warp_incl_scan(T v)
@@ -177,7 +180,7 @@ __device__ __forceinline__ T warp_incl_scan(T v)
 
 template <typename T>
 __global__ void k_scan_tiles(const T* __restrict__ in, T* __restrict__ out, int64_t n,
-                             T* __restrict__ tileSums)
+                             T* __restrict__ tileSums, T* __restrict__ total)
 {
     __shared__ T warpSums[SCAN_THREADS / 32];
     const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
@@ -207,24 +210,38 @@ __global__ void k_scan_tiles(const T* __restrict__ in, T* __restrict__ out, int6
         if (base + k < n) out[base + k] = prefix;
         prefix += v[k];
     }
-    if (threadIdx.x == SCAN_THREADS - 1) tileSums[blockIdx.x] = prefix;
+    if (threadIdx.x == SCAN_THREADS - 1)
+    {
+        tileSums[blockIdx.x] = prefix;
+        if (total && gridDim.x == 1) *total = prefix;
+    }
 }
 
+// tileOffsets: the scanned totals, or null (the block sums tileSums itself)
 template <typename T>
-__global__ void k_scan_add(T* __restrict__ out, int64_t n, const T* __restrict__ tileOffsets)
+__global__ void k_scan_add(T* __restrict__ out, int64_t n, const T* __restrict__ tileSums,
+                           const T* __restrict__ tileOffsets, T* __restrict__ total)
 {
+    __shared__ T warpSums[SCAN_THREADS / 32];
+    T off = 0;
+    if (tileOffsets)
+        off = tileOffsets[blockIdx.x];
+    else
+    {
+        T sum = 0;
+        for (int64_t t = threadIdx.x; t < blockIdx.x; t += SCAN_THREADS) sum += tileSums[t];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if ((threadIdx.x & 31) == 0) warpSums[threadIdx.x >> 5] = sum;
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < SCAN_THREADS / 32; ++w) off += warpSums[w];
+    }
     const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
-    const T off = tileOffsets[blockIdx.x];
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; ++k)
         if (base + k < n) out[base + k] += off;
-}
-
-template <typename T>
-__global__ void k_scan_total(const T* __restrict__ tileSums, const T* __restrict__ tileOffsets,
-                             int64_t tiles, T* __restrict__ total)
-{
-    *total = tileOffsets[tiles - 1] + tileSums[tiles - 1];
+    if (total && threadIdx.x == 0 && blockIdx.x == gridDim.x - 1) *total = off + tileSums[blockIdx.x];
 }
 
 template <typename T>
@@ -240,24 +257,14 @@ static int scan_rec(mrmd_ctx* ctx, const T* in, T* out, int64_t n, T* total, cha
     T* tileOffsets = tileSums + tiles;
     char* next = reinterpret_cast<char*>(tileOffsets + tiles);
     next = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(next) + 255) & ~uintptr_t(255));
-    k_scan_tiles<T><<<(unsigned)tiles, SCAN_THREADS, 0, ctx->stream>>>(in, out, n, tileSums);
+    k_scan_tiles<T><<<(unsigned)tiles, SCAN_THREADS, 0, ctx->stream>>>(in, out, n, tileSums, total);
     MRMD_TRY(after_launch(ctx, "scan_tiles"));
-    if (tiles > 1)
-    {
-        MRMD_TRY(scan_rec<T>(ctx, tileSums, tileOffsets, tiles, nullptr, next));
-        k_scan_add<T><<<(unsigned)tiles, SCAN_THREADS, 0, ctx->stream>>>(out, n, tileOffsets);
-        MRMD_TRY(after_launch(ctx, "scan_add"));
-    }
-    else
-    {
-        MRMD_CUDA(ctx, cudaMemsetAsync(tileOffsets, 0, sizeof(T), ctx->stream));
-    }
-    if (total)
-    {
-        k_scan_total<T><<<1, 1, 0, ctx->stream>>>(tileSums, tileOffsets, tiles, total);
-        MRMD_TRY(after_launch(ctx, "scan_total"));
-    }
-    return MRMD_OK;
+    if (tiles == 1) return MRMD_OK;
+    const bool direct = tiles <= SCAN_DIRECT;
+    if (!direct) MRMD_TRY(scan_rec<T>(ctx, tileSums, tileOffsets, tiles, nullptr, next));
+    k_scan_add<T><<<(unsigned)tiles, SCAN_THREADS, 0, ctx->stream>>>(out, n, tileSums, direct ? nullptr : tileOffsets,
+                                                                     total);
+    return after_launch(ctx, "scan_add");
 }
 
 template <typename T>

@@ -4,8 +4,7 @@
 // X, Y, Z, every atom (real or earlier ghost) with x < minInner gets an
 // image at +L and every atom with x >= maxInner one at -L; images of one
 // pass are appended "+L images in source order, then -L images in source
-// order".  A stable exclusive scan gives the same order as the reference's
-// parallel_scan, so ghost indices are identical to the reference's.
+// order", so ghost indices are identical to the reference's.
 #include "common.cuh"
 #include "ghost_impl.cuh"
 
@@ -60,21 +59,6 @@ __device__ __forceinline__ void add_comp(double4& p, int axis, double v)
         p.z = __dadd_rn(p.z, v);
 }
 
-// packed (lo, hi) selection flags of one axis pass
-__global__ void k_ghost_flags(const double4* __restrict__ pos, int64_t n, int axis, double minInner,
-                              double maxInner, int64_t* __restrict__ flags)
-{
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x)
-    {
-        const double x = comp(pos[i], axis);
-        int64_t f = 0;
-        if (x < minInner) f |= 1;
-        if (x >= maxInner) f |= (int64_t)1 << 32;
-        flags[i] = f;
-    }
-}
-
 __device__ __forceinline__ void copy_atom(mrmd_atoms a, int64_t dst, int64_t src)
 {
     // data/Atoms.hpp:97-110
@@ -87,36 +71,230 @@ __device__ __forceinline__ void copy_atom(mrmd_atoms a, int64_t dst, int64_t src
     a.relativeMass[dst] = a.relativeMass[src];
 }
 
-__global__ void k_ghost_copy(mrmd_atoms a, int32_t* __restrict__ corr, int64_t n, int axis,
-                             double minInner, double maxInner, double L,
-                             const int64_t* __restrict__ offsets, const int64_t* __restrict__ total)
+// The ghosts of all three passes from one look at the local atoms.  An
+// image of a later axis is taken of locals and of earlier images alike, and an
+// image keeps its source's coordinates on the other axes, so the atom's six
+// selection flags (x < minInner, x >= maxInner, ...) say which of the 26
+// images it has.  The passes append them kind after kind, each kind in source
+// order: kind k's images start where those of the kinds before it end, and an
+// atom's place among them is the number of atoms before it that have the kind.
+// So: counts per block of atoms and kind (k_image_count), their scan (one
+// block, k_image_scan), and the images with the real atom -> ghosts table
+// (k_image_write); an atom's ghosts ascend with the kind.  (Three passes of
+// flags, scan, host read-back and copy, then counting, scanning, filling and
+// sorting the table, took 26 launches and four round trips.)
+constexpr int KINDS = 26;
+constexpr int IMG_TB = 256;
+constexpr int IMG_ROUNDS = 4;  // atoms per thread
+constexpr int IMG_ATOMS = IMG_TB * IMG_ROUNDS;
+
+// flags of kind k: bit 2 d: +L on axis d, bit 2 d + 1: -L
+__host__ __device__ constexpr uint32_t kind_flags(int k)
 {
-    const int64_t numLo = (*total) & 0xffffffffLL;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x)
+    if (k < 2) return 1u << k;                                           // x
+    const uint32_t xy[3] = {0u, 1u, 2u};
+    if (k < 8) return (4u << ((k - 2) / 3)) | xy[(k - 2) % 3];           // y of locals and x images
+    const int g = (k - 8) % 9;                                           // z of the nine groups before
+    return (16u << ((k - 8) / 9)) | (g < 3 ? xy[g] : ((4u << ((g - 3) / 3)) | xy[(g - 3) % 3]));
+}
+
+struct ImageBox
+{
+    double lo[3], hi[3], L[3];  // inner corners, lengths
+};
+
+__device__ __forceinline__ uint32_t image_flags(const double4& p, const ImageBox& b)
+{
+    uint32_t f = 0u;
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
     {
-        const double x = comp(reinterpret_cast<const double4*>(a.pos)[i], axis);
-        const int64_t off = offsets[i];
-        const int32_t real = corr[i] == -1 ? (int32_t)i : corr[i];
-        if (x < minInner && MRMD_IN_BOUNDS(n + (off & 0xffffffffLL), a.capacity))
+        const double x = comp(p, d);
+        f |= (x < b.lo[d] ? 1u : 0u) << (2 * d);
+        f |= (x >= b.hi[d] ? 2u : 0u) << (2 * d);
+    }
+    return f;
+}
+
+// blockCount[k * blocks + block]: atoms of the block with kind k
+__global__ void __launch_bounds__(IMG_TB) k_image_count(const double4* __restrict__ pos, int64_t n, ImageBox box,
+                                                        int32_t* __restrict__ blockCount)
+{
+    __shared__ int32_t cnt[KINDS];
+    if (threadIdx.x < KINDS) cnt[threadIdx.x] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < IMG_ROUNDS; ++q)
+    {
+        const int64_t i = blockIdx.x * (int64_t)IMG_ATOMS + q * IMG_TB + threadIdx.x;
+        const uint32_t f = i < n ? image_flags(pos[i], box) : 0u;
+        if (__ballot_sync(0xffffffffu, f != 0u) == 0u) continue;
+#pragma unroll
+        for (int k = 0; k < KINDS; ++k)
         {
-            const int64_t dst = n + (off & 0xffffffffLL);
-            copy_atom(a, dst, i);
-            double4 p = reinterpret_cast<double4*>(a.pos)[dst];
-            add_comp(p, axis, L);
-            reinterpret_cast<double4*>(a.pos)[dst] = p;
-            corr[dst] = real;
-        }
-        if (x >= maxInner && MRMD_IN_BOUNDS(n + numLo + (off >> 32), a.capacity))
-        {
-            const int64_t dst = n + numLo + (off >> 32);
-            copy_atom(a, dst, i);
-            double4 p = reinterpret_cast<double4*>(a.pos)[dst];
-            add_comp(p, axis, -L);
-            reinterpret_cast<double4*>(a.pos)[dst] = p;
-            corr[dst] = real;
+            const unsigned m = __ballot_sync(0xffffffffu, (f & kind_flags(k)) == kind_flags(k));
+            if (m && (threadIdx.x & 31) == 0) atomicAdd(&cnt[k], __popc(m));
         }
     }
+    __syncthreads();
+    if (threadIdx.x < KINDS) blockCount[threadIdx.x * (int64_t)gridDim.x + blockIdx.x] = cnt[threadIdx.x];
+}
+
+// One warp per kind: exclusive scan over the blocks; then start[k]: images of
+// the kinds before k, start[KINDS]: all images.
+__global__ void __launch_bounds__(KINDS * 32) k_image_scan(int32_t* __restrict__ blockCount, int64_t blocks,
+                                                           int64_t* __restrict__ start)
+{
+    __shared__ int64_t total[KINDS];
+    const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
+    int32_t* c = blockCount + k * blocks;
+    int64_t carry = 0;  // (a kind has at most one image per atom: offsets fit 32 bits)
+    for (int64_t b0 = 0; b0 < blocks; b0 += 256)
+    {
+        int32_t v[8], sum = 0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+        {
+            const int64_t b = b0 + lane * 8 + q;
+            v[q] = b < blocks ? c[b] : 0;
+            sum += v[q];
+        }
+        int32_t incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+        {
+            const int32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        int32_t off = (int32_t)carry + incl - sum;
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+        {
+            const int64_t b = b0 + lane * 8 + q;
+            if (b < blocks) c[b] = off;
+            off += v[q];
+        }
+        carry += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) total[k] = carry;
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        int64_t s = 0;
+        for (int q = 0; q < KINDS; ++q)
+        {
+            start[q] = s;
+            s += total[q];
+        }
+        start[KINDS] = s;
+    }
+}
+
+// The images (data/Atoms.hpp:97-110 with the shifted position), their real
+// atoms in corr, and the table ghostStart / ghostList.
+__global__ void __launch_bounds__(IMG_TB) k_image_write(mrmd_atoms a, int64_t n, ImageBox box,
+                                                        const int32_t* __restrict__ blockOffset,
+                                                        const int64_t* __restrict__ start, int32_t* __restrict__ corr,
+                                                        int32_t* __restrict__ ghostStart,
+                                                        int32_t* __restrict__ ghostList)
+{
+    constexpr int WARPS = IMG_TB / 32;
+    __shared__ int32_t place[KINDS];         // atoms before this round with kind k
+    __shared__ int32_t warpCnt[WARPS][KINDS];  // per warp, then exclusive over the warps
+    __shared__ int32_t warpImg[WARPS];       // images of the warp's atoms
+    __shared__ int32_t imgBefore;            // images of all atoms before this round
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    const double4* pos = reinterpret_cast<const double4*>(a.pos);
+    if (threadIdx.x < KINDS) place[threadIdx.x] = blockOffset[threadIdx.x * (int64_t)gridDim.x + blockIdx.x];
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        int32_t s = 0;
+        for (int k = 0; k < KINDS; ++k) s += place[k];
+        imgBefore = s;
+    }
+    for (int q = 0; q < IMG_ROUNDS; ++q)
+    {
+        const int64_t i = blockIdx.x * (int64_t)IMG_ATOMS + q * IMG_TB + threadIdx.x;
+        double4 p = make_double4(0.0, 0.0, 0.0, 0.0);
+        if (i < n) p = pos[i];
+        const uint32_t f = i < n ? image_flags(p, box) : 0u;
+        int32_t mine = 1;  // images of the atom
+#pragma unroll
+        for (int d = 0; d < 3; ++d) mine *= 1 + (int)((f >> (2 * d)) & 1u) + (int)((f >> (2 * d + 1)) & 1u);
+        mine -= 1;
+        int32_t incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+        {
+            const int32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        if (lane == 31) warpImg[warp] = incl;
+        const bool any = __ballot_sync(0xffffffffu, f != 0u) != 0u;
+        if (lane < KINDS) warpCnt[warp][lane] = 0;
+        __syncwarp();
+        if (any)
+        {
+#pragma unroll
+            for (int k = 0; k < KINDS; ++k)
+            {
+                const unsigned m = __ballot_sync(0xffffffffu, (f & kind_flags(k)) == kind_flags(k));
+                if (lane == 0) warpCnt[warp][k] = __popc(m);
+            }
+        }
+        __syncthreads();
+        // exclusive over the warps; `place` moves on after the round
+        int32_t roundTotal = 0;
+        if (threadIdx.x < KINDS)
+        {
+            for (int w = 0; w < WARPS; ++w)
+            {
+                const int32_t c = warpCnt[w][threadIdx.x];
+                warpCnt[w][threadIdx.x] = place[threadIdx.x] + roundTotal;
+                roundTotal += c;
+            }
+        }
+        __syncthreads();
+        int32_t list = imgBefore + incl - mine;
+        for (int w = 0; w < warp; ++w) list += warpImg[w];
+        if (i < n)
+        {
+            ghostStart[i] = list;
+            corr[i] = -1;
+        }
+        if (any)
+        {
+#pragma unroll 1
+            for (int k = 0; k < KINDS; ++k)
+            {
+                const uint32_t kf = kind_flags(k);
+                const bool has = (f & kf) == kf;
+                const unsigned m = __ballot_sync(0xffffffffu, has);
+                if (!has) continue;
+                const int64_t dst = n + start[k] + warpCnt[warp][k] + __popc(m & below);
+                if (!MRMD_IN_BOUNDS(dst, a.capacity)) continue;
+                copy_atom(a, dst, i);
+                double4 s = p;
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+                {
+                    if ((kf >> (2 * d)) & 1u) add_comp(s, d, box.L[d]);
+                    if ((kf >> (2 * d + 1)) & 1u) add_comp(s, d, -box.L[d]);
+                }
+                reinterpret_cast<double4*>(a.pos)[dst] = s;
+                corr[dst] = (int32_t)i;
+                ghostList[list++] = (int32_t)dst;
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x < KINDS) place[threadIdx.x] += roundTotal;
+        if (threadIdx.x == 0)
+            for (int w = 0; w < WARPS; ++w) imgBefore += warpImg[w];
+        __syncthreads();
+    }
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) ghostStart[n] = (int32_t)start[KINDS];
 }
 
 __global__ void k_fill_i32(int32_t* p, int64_t n, int32_t v)
@@ -421,45 +599,40 @@ int mrmd_ghost_create(mrmd_ctx* ctx, mrmd_ghost_layer* g, mrmd_atoms* a, const m
     // GhostExchange::createGhostAtomsXYZ, communication/GhostExchange.cpp:171-181
     if (!ctx || !g || !a || !sd) return MRMD_ERR_ARG;
     const int64_t nLocal = a->numLocal;
-    MRMD_TRY(ensure_layer(ctx, g, a->capacity > nLocal + 1 ? a->capacity : nLocal + 1, nLocal + 1));
-    k_fill_i32<<<grid_for(ctx, g->capacity, TB), TB, 0, ctx->stream>>>(g->correspondingRealAtom,
-                                                                        g->capacity, -1);
-    MRMD_TRY(after_launch(ctx, "fill_corr"));
     a->numGhost = 0;
-    int64_t* total = reinterpret_cast<int64_t*>(ctx->devScalars);
-    for (int axis = 0; axis < 3; ++axis)
+    const int64_t blocks = div_up(nLocal > 0 ? nLocal : 1, IMG_ATOMS);
+    int64_t* start = static_cast<int64_t*>(
+        scratch(ctx, sizeof(int64_t) * (KINDS + 1) + sizeof(int32_t) * KINDS * (size_t)blocks));
+    if (!start) return MRMD_ERR_OOM;
+    int32_t* counts = reinterpret_cast<int32_t*>(start + KINDS + 1);
+    ImageBox box{};
+    for (int d = 0; d < 3; ++d)
     {
-        const int64_t n = a->numLocal + a->numGhost;
-        int64_t* offs = static_cast<int64_t*>(scratch(ctx, sizeof(int64_t) * (size_t)(n + 1)));
-        if (!offs) return MRMD_ERR_OOM;
-        k_ghost_flags<<<grid_for(ctx, n, TB), TB, 0, ctx->stream>>>(
-            reinterpret_cast<const double4*>(a->pos), n, axis, sd->minInnerCorner[axis],
-            sd->maxInnerCorner[axis], offs);
-        MRMD_TRY(after_launch(ctx, "ghost_flags"));
-        MRMD_TRY(scan_exclusive_i64(ctx, offs, offs, n, total));
-        int64_t hTotal = 0;
-        MRMD_CUDA(ctx, cudaMemcpyAsync(&hTotal, total, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
-        MRMD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        const int64_t numLo = hTotal & 0xffffffffLL, numHi = hTotal >> 32;
-        const int64_t need = n + numLo + numHi;
-        if (need > INT32_MAX) return set_error(ctx, MRMD_ERR_CAPACITY, "more than 2^31 atoms");
-        if (need > a->capacity)
-        {
-            MRMD_TRY(mrmd_atoms_reserve(ctx, a, need + need / 8 + 64));
-        }
-        MRMD_TRY(ensure_layer(ctx, g, a->capacity, nLocal + 1));
-        if (numLo + numHi > 0)
-        {
-            k_ghost_copy<<<grid_for(ctx, n, TB), TB, 0, ctx->stream>>>(
-                *a, g->correspondingRealAtom, n, axis, sd->minInnerCorner[axis], sd->maxInnerCorner[axis],
-                sd->diameter[axis], offs, total);
-            MRMD_TRY(after_launch(ctx, "ghost_copy"));
-        }
-        a->numGhost += numLo + numHi;
+        box.lo[d] = sd->minInnerCorner[d];
+        box.hi[d] = sd->maxInnerCorner[d];
+        box.L[d] = sd->diameter[d];
     }
+    k_image_count<<<(unsigned)blocks, IMG_TB, 0, ctx->stream>>>(reinterpret_cast<const double4*>(a->pos), nLocal, box,
+                                                                counts);
+    MRMD_TRY(after_launch(ctx, "image_count"));
+    k_image_scan<<<1, KINDS * 32, 0, ctx->stream>>>(counts, blocks, start);
+    MRMD_TRY(after_launch(ctx, "image_scan"));
+    int64_t* hTotal = reinterpret_cast<int64_t*>(ctx->hostScalars);
+    MRMD_CUDA(ctx, cudaMemcpyAsync(hTotal, start + KINDS, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
+    MRMD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    const int64_t need = nLocal + *hTotal;
+    if (need > INT32_MAX) return set_error(ctx, MRMD_ERR_CAPACITY, "more than 2^31 atoms");
+    if (need > a->capacity) MRMD_TRY(mrmd_atoms_reserve(ctx, a, need + need / 8 + 64));
+    MRMD_TRY(ensure_layer(ctx, g, a->capacity > nLocal + 1 ? a->capacity : nLocal + 1, nLocal + 1));
+    // -1 (locals and unused entries)
+    MRMD_CUDA(ctx, cudaMemsetAsync(g->correspondingRealAtom + need, 0xff, sizeof(int32_t) * (size_t)(g->capacity - need),
+                                   ctx->stream));
+    k_image_write<<<(unsigned)blocks, IMG_TB, 0, ctx->stream>>>(*a, nLocal, box, counts, start,
+                                                                g->correspondingRealAtom, g->ghostStart, g->ghostList);
+    MRMD_TRY(after_launch(ctx, "image_write"));
+    a->numGhost = need - nLocal;
     g->numLocal = a->numLocal;
     g->numGhost = a->numGhost;
-    MRMD_TRY(build_csr(ctx, g, g->numLocal, g->numGhost));
     return finish(ctx, "ghost_create");
 }
 

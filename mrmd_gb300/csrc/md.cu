@@ -278,7 +278,6 @@ int md_rebuild(mrmd_ctx* ctx, mrmd_md* md)
         MRMD_TRY(build_split_list(ctx, &md->list, &md->farList, a->pos, nAll, 0, a->numLocal, rlist,
                                   md->rsplit + 0.5 * md->cfg.skin, md->grid,
                                   md->cfg.gatherNeighbours ? nullptr : &md->tiles, md->cfg.tileBuild == 0));
-        MRMD_TRY(list_total_pairs(ctx, &md->farList));
         md->tp = make_tile_params(md->lj->p0, md->lj->rcSqr, md->rsplit, md->farList.maxNeighbors);
     }
     else
@@ -286,7 +285,6 @@ int md_rebuild(mrmd_ctx* ctx, mrmd_md* md)
         MRMD_TRY(build_half_list(ctx, &md->list, a->pos, nAll, 0, a->numLocal, rlist, md->grid,
                                  md->list.maxNeighbors > 0 ? md->list.maxNeighbors : md->cfg.maxNeighbors, false));
     }
-    MRMD_TRY(list_total_pairs(ctx, &md->list));
     if (full && nAll > md->splitCap)
     {
         dfree(md->rec);

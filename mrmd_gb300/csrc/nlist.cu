@@ -118,10 +118,11 @@ __global__ void k_cell_scatter(const int32_t* __restrict__ cellOf, int64_t n,
 }
 
 // Stable order inside each cell: every slot of the (unordered) scatter
-// output counts the smaller ids of its cell and moves its id to that rank.
-__global__ void k_cell_rank(const int32_t* __restrict__ cellOf, const int32_t* __restrict__ cellStart,
-                            const int32_t* __restrict__ unordered, int64_t n, int32_t* __restrict__ sorted,
-                            int64_t nkeys)
+// output counts the smaller ids of its cell and moves its id to that rank,
+// with its FP32 coordinates relative to the grid origin.
+__global__ void k_cell_rank(const double4* __restrict__ pos, const int32_t* __restrict__ cellOf,
+                            const int32_t* __restrict__ cellStart, const int32_t* __restrict__ unordered, int64_t n,
+                            double3 origin, int32_t* __restrict__ sorted, float4* __restrict__ spos, int64_t nkeys)
 {
     for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < n;
          s += (int64_t)gridDim.x * blockDim.x)
@@ -129,26 +130,16 @@ __global__ void k_cell_rank(const int32_t* __restrict__ cellOf, const int32_t* _
         const int32_t v = unordered[s];
         if (!MRMD_IN_BOUNDS(v, n)) continue;
         const int32_t c = cellOf[v];
+        const double4 p = pos[v];
         if (!MRMD_IN_BOUNDS(c, nkeys)) continue;
         const int32_t b = cellStart[c], e = cellStart[c + 1];
         if (!MRMD_IN_BOUNDS(b, n + 1) || !MRMD_IN_BOUNDS(e, n + 1)) continue;
         int32_t rank = 0;
         for (int32_t t = b; t < e; ++t) rank += unordered[t] < v;
-        if (MRMD_IN_BOUNDS(b + rank, n)) sorted[b + rank] = v;
-    }
-}
-
-__global__ void k_cell_gather(const double4* __restrict__ pos, const int32_t* __restrict__ sorted,
-                              int64_t n, double3 origin, float4* __restrict__ spos)
-{
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < n;
-         s += (int64_t)gridDim.x * blockDim.x)
-    {
-        const int32_t j = sorted[s];
-        if (!MRMD_IN_BOUNDS(j, n)) continue;
-        const double4 p = pos[j];
-        spos[s] = make_float4((float)(p.x - origin.x), (float)(p.y - origin.y), (float)(p.z - origin.z),
-                              __int_as_float(j));
+        if (!MRMD_IN_BOUNDS(b + rank, n)) continue;
+        sorted[b + rank] = v;
+        spos[b + rank] = make_float4((float)(p.x - origin.x), (float)(p.y - origin.y), (float)(p.z - origin.z),
+                                     __int_as_float(v));
     }
 }
 
@@ -165,8 +156,10 @@ __global__ void __launch_bounds__(128) k_build_list(
     const int32_t* __restrict__ cellStart, const float4* __restrict__ spos, CellGrid g,
     int64_t begin, int64_t end, double rsq, float rsqLo, float rsqHi, int64_t cap,
     int32_t* __restrict__ counts, int32_t* __restrict__ nbrs, int32_t* __restrict__ maxCount, int64_t nPos,
-    float nearSqF, int64_t capFar, int32_t* __restrict__ countsFar, int32_t* __restrict__ nbrsFar)
+    float nearSqF, int64_t capFar, int32_t* __restrict__ countsFar, int32_t* __restrict__ nbrsFar,
+    unsigned long long* __restrict__ totals)
 {
+    uint32_t sumNear = 0u, sumFar = 0u;  // entries of this lane's rows
     constexpr unsigned ALL = 0xffffffffu;
     const int lane = threadIdx.x & 31, sub = lane % LANES;
     const unsigned mine = (LANES == 32 ? ALL : ((1u << LANES) - 1u)) << (lane & ~(LANES - 1));
@@ -251,17 +244,36 @@ __global__ void __launch_bounds__(128) k_build_list(
         }
         if (!ok || sub != 0) continue;
         counts[row] = cnt < cap ? cnt : (int32_t)cap;
+        sumNear += (uint32_t)cnt;
         if (cnt > cap) atomicMax(maxCount, cnt);
         if (SPLIT)
         {
             countsFar[row] = cntFar < capFar ? cntFar : (int32_t)capFar;
+            sumFar += (uint32_t)cntFar;
             if (cntFar > capFar) atomicMax(maxCount + 1, cntFar);
         }
     }
+    add_totals(sumNear, sumFar, totals);
 }
 
 namespace
 {
+// The flags cleared but for the non-finite one (set by the binning, once).
+int clear_counts(mrmd_ctx* ctx, int32_t* flags)
+{
+    MRMD_CUDA(ctx, cudaMemsetAsync(flags, 0, 2 * sizeof(int32_t), ctx->stream));
+    MRMD_CUDA(ctx, cudaMemsetAsync(flags + 3, 0, sizeof(ListFlags) - 3 * sizeof(int32_t), ctx->stream));
+    return MRMD_OK;
+}
+
+int read_flags(mrmd_ctx* ctx, const int32_t* flags, ListFlags* out)
+{
+    MRMD_CUDA(ctx, cudaMemcpyAsync(ctx->hostScalars, flags, sizeof(ListFlags), cudaMemcpyDeviceToHost, ctx->stream));
+    MRMD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    std::memcpy(out, ctx->hostScalars, sizeof(ListFlags));
+    return bounds_check(ctx);
+}
+
 // Launch of k_build_list<FULL, SPLIT>.
 template <bool FULL, bool SPLIT>
 int build_rows(mrmd_ctx* ctx, const CellList& cl, const double* pos4, int64_t begin, int64_t end, double rsq,
@@ -271,7 +283,7 @@ int build_rows(mrmd_ctx* ctx, const CellList& cl, const double* pos4, int64_t be
     auto launch = [&](auto kernel, int lanes) {
         kernel<<<grid_for(ctx, (end - begin) * lanes, 128, 16), 128, 0, ctx->stream>>>(
             reinterpret_cast<const double4*>(pos4), cl.cellOf, cl.cellStart, cl.spos, cl.g, begin, end, rsq, rsqLo,
-            rsqHi, cap, counts, nbrs, maxCount, nPos, nearSqF, capFar, countsFar, nbrsFar);
+            rsqHi, cap, counts, nbrs, maxCount, nPos, nearSqF, capFar, countsFar, nbrsFar, list_totals(maxCount));
     };
     // lanes per row: several where one lane per row leaves the SMs with few
     // warps that wait for their loads; one for large systems, where the
@@ -302,9 +314,11 @@ int CellList::build(mrmd_ctx* ctx, const double* pos4, int64_t n, const CellGrid
         dfree(cellOf);
         dfree(sorted);
         dfree(spos);
-        cellOf = sorted = nullptr;
+        dfree(unordered);
+        cellOf = sorted = unordered = nullptr;
         spos = nullptr;
         const int64_t c = n + n / 4 + 64;
+        MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&unordered), sizeof(int32_t) * (size_t)c));
         MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&cellOf), sizeof(int32_t) * (size_t)c));
         MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&sorted), sizeof(int32_t) * (size_t)c));
         MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&spos), sizeof(float4) * (size_t)c));
@@ -312,18 +326,17 @@ int CellList::build(mrmd_ctx* ctx, const double* pos4, int64_t n, const CellGrid
     }
     if (nkeys + 1 > capCells)
     {
+        // one allocation: cell starts, then the scatter's cursors
         dfree(cellStart);
-        dfree(cursor);
-        cellStart = cursor = nullptr;
+        cellStart = nullptr;
         const int64_t c = nkeys + 1;
-        MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&cellStart), sizeof(int32_t) * (size_t)c));
-        MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&cursor), sizeof(int32_t) * (size_t)c));
+        MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&cellStart), 2 * sizeof(int32_t) * (size_t)c));
         capCells = c;
     }
+    int32_t* cursor = cellStart + (nkeys + 1);
     numParticles = n;
     constexpr int TB = 256;
-    MRMD_CUDA(ctx, cudaMemsetAsync(cellStart, 0, sizeof(int32_t) * (size_t)(nkeys + 1), ctx->stream));
-    MRMD_CUDA(ctx, cudaMemsetAsync(cursor, 0, sizeof(int32_t) * (size_t)(nkeys + 1), ctx->stream));
+    MRMD_CUDA(ctx, cudaMemsetAsync(cellStart, 0, 2 * sizeof(int32_t) * (size_t)(nkeys + 1), ctx->stream));
     if (n > 0)
     {
         k_cell_count<<<grid_for(ctx, n, TB), TB, 0, ctx->stream>>>(reinterpret_cast<const double4*>(pos4), n,
@@ -334,16 +347,11 @@ int CellList::build(mrmd_ctx* ctx, const double* pos4, int64_t n, const CellGrid
     MRMD_TRY(scan_exclusive_i32(ctx, cellStart, cellStart, nkeys + 1, nullptr));
     if (n > 0)
     {
-        // unordered scatter into `spos` storage (reused as int32 scratch), then
-        // stable ranks into `sorted`
-        int32_t* unordered = reinterpret_cast<int32_t*>(spos);
         k_cell_scatter<<<grid_for(ctx, n, TB), TB, 0, ctx->stream>>>(cellOf, n, cellStart, cursor, unordered, nkeys);
         MRMD_TRY(after_launch(ctx, "cell_scatter"));
-        k_cell_rank<<<grid_for(ctx, n, TB), TB, 0, ctx->stream>>>(cellOf, cellStart, unordered, n, sorted, nkeys);
+        k_cell_rank<<<grid_for(ctx, n, TB), TB, 0, ctx->stream>>>(reinterpret_cast<const double4*>(pos4), cellOf,
+                                                                  cellStart, unordered, n, g.mn, sorted, spos, nkeys);
         MRMD_TRY(after_launch(ctx, "cell_rank"));
-        k_cell_gather<<<grid_for(ctx, n, TB), TB, 0, ctx->stream>>>(reinterpret_cast<const double4*>(pos4),
-                                                                    sorted, n, g.mn, spos);
-        MRMD_TRY(after_launch(ctx, "cell_gather"));
     }
     return MRMD_OK;
 }
@@ -353,9 +361,9 @@ void CellList::release()
     dfree(cellOf);
     dfree(sorted);
     dfree(spos);
+    dfree(unordered);
     dfree(cellStart);
-    dfree(cursor);
-    cellOf = sorted = cellStart = cursor = nullptr;
+    cellOf = sorted = unordered = cellStart = nullptr;
     spos = nullptr;
     capN = capCells = 0;
 }
@@ -388,9 +396,9 @@ int build_half_list(mrmd_ctx* ctx, mrmd_nlist* nl, const double* pos4, int64_t n
                     int64_t end, double rlist, const CellGrid& grid, int64_t maxNeighbors, bool full)
 {
     CellList* cl = static_cast<CellList*>(nl->cells);
-    // [0] longest row, [2] non-finite position flag
+    // ListFlags: longest row, non-finite position flag, entries of all rows
     int32_t* maxCount = reinterpret_cast<int32_t*>(ctx->devScalars);
-    MRMD_CUDA(ctx, cudaMemsetAsync(maxCount, 0, 3 * sizeof(int32_t), ctx->stream));
+    MRMD_CUDA(ctx, cudaMemsetAsync(maxCount, 0, sizeof(ListFlags), ctx->stream));
     MRMD_TRY(cl->build(ctx, pos4, nPos, grid, false, maxCount + 2));
     const int64_t rows = end - begin;
     // FP32 error band: coordinates are stored relative to the grid origin
@@ -406,7 +414,7 @@ int build_half_list(mrmd_ctx* ctx, mrmd_nlist* nl, const double* pos4, int64_t n
     for (int attempt = 0; attempt < 4; ++attempt)
     {
         MRMD_TRY(ensure_list_storage(ctx, nl, rows, cap));
-        MRMD_CUDA(ctx, cudaMemsetAsync(maxCount, 0, sizeof(int32_t), ctx->stream));
+        if (attempt > 0) MRMD_TRY(clear_counts(ctx, maxCount));
         if (rows > 0)
         {
             MRMD_TRY(full ? (build_rows<true, false>(ctx, *cl, pos4, begin, end, rsq, rsqLo, rsqHi, cap, nl->counts,
@@ -414,31 +422,20 @@ int build_half_list(mrmd_ctx* ctx, mrmd_nlist* nl, const double* pos4, int64_t n
                           : (build_rows<false, false>(ctx, *cl, pos4, begin, end, rsq, rsqLo, rsqHi, cap, nl->counts,
                                                       nl->nbrs, maxCount, nPos)));
         }
-        int32_t h[3] = {0, 0, 0};
-        MRMD_CUDA(ctx, cudaMemcpyAsync(h, maxCount, 3 * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
-        MRMD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        MRMD_TRY(bounds_check(ctx));
-        if (h[2]) return set_error(ctx, MRMD_ERR_NONFINITE, "non-finite particle position at the list build");
-        const int32_t hMax = h[0];
+        ListFlags h{};
+        MRMD_TRY(read_flags(ctx, maxCount, &h));
+        if (h.i[2]) return set_error(ctx, MRMD_ERR_NONFINITE, "non-finite particle position at the list build");
+        const int32_t hMax = h.i[0];
         if (hMax <= cap)
         {
             nl->rows = rows;
             nl->begin = begin;
+            nl->totalPairs = (int64_t)h.totals[0];
             return MRMD_OK;
         }
         cap = hMax + hMax / 8 + 4;  // Cabana grows and rebuilds the same way
     }
     return set_error(ctx, MRMD_ERR_NLIST_OVERFLOW, "neighbour list kept overflowing");
-}
-
-__global__ void k_count_sum(const int32_t* __restrict__ counts, int64_t n, unsigned long long* out)
-{
-    unsigned long long s = 0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x)
-        s += (unsigned long long)counts[i];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(out, s);
 }
 
 int build_split_list(mrmd_ctx* ctx, mrmd_nlist* nearList, mrmd_nlist* farList, const double* pos4, int64_t nPos,
@@ -447,9 +444,10 @@ int build_split_list(mrmd_ctx* ctx, mrmd_nlist* nearList, mrmd_nlist* farList, c
 {
     if (tiles && begin != 0) return set_error(ctx, MRMD_ERR_ARG, "tile lists need rows from particle 0");
     CellList* cl = static_cast<CellList*>(nearList->cells);
-    // [0], [1] longest near and far rows, [2] non-finite position flag
+    // ListFlags: longest near and far rows, non-finite position flag, the tile
+    // build's largest tile, overflow flag and member total, list entries
     int32_t* maxCount = reinterpret_cast<int32_t*>(ctx->devScalars);
-    MRMD_CUDA(ctx, cudaMemsetAsync(maxCount, 0, 3 * sizeof(int32_t), ctx->stream));
+    MRMD_CUDA(ctx, cudaMemsetAsync(maxCount, 0, sizeof(ListFlags), ctx->stream));
     MRMD_TRY(cl->build(ctx, pos4, nPos, grid, false, maxCount + 2));
     const int64_t rows = end - begin;
     // the same FP32 error band as build_half_list
@@ -465,9 +463,7 @@ int build_split_list(mrmd_ctx* ctx, mrmd_nlist* nearList, mrmd_nlist* farList, c
     {
         MRMD_TRY(ensure_list_storage(ctx, nearList, rows, capN));
         MRMD_TRY(ensure_list_storage(ctx, farList, rows, capF));
-        // [3..5]: the tile build's largest tile, overflow flag, member total
-        MRMD_CUDA(ctx, cudaMemsetAsync(maxCount, 0, 2 * sizeof(int32_t), ctx->stream));
-        MRMD_CUDA(ctx, cudaMemsetAsync(maxCount + 3, 0, 3 * sizeof(int32_t), ctx->stream));
+        if (attempt > 0) MRMD_TRY(clear_counts(ctx, maxCount));
         auto int32_rows = [&]() -> int {
             return build_rows<true, true>(ctx, *cl, pos4, begin, end, rsq, rsqLo, rsqHi, capN, nearList->counts,
                                           nearList->nbrs, maxCount, nPos, nearSqF, capF, farList->counts,
@@ -486,10 +482,9 @@ int build_split_list(mrmd_ctx* ctx, mrmd_nlist* nearList, mrmd_nlist* farList, c
             else
                 MRMD_TRY(int32_rows());
         }
-        int32_t hMax[6] = {0, 0, 0, 0, 0, 0};
-        MRMD_CUDA(ctx, cudaMemcpyAsync(hMax, maxCount, 6 * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
-        MRMD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        MRMD_TRY(bounds_check(ctx));
+        ListFlags h{};
+        const int32_t* hMax = h.i;
+        MRMD_TRY(read_flags(ctx, maxCount, &h));
         if (hMax[2]) return set_error(ctx, MRMD_ERR_NONFINITE, "non-finite particle position at the list build");
         if (tiles) tiles->unfitTiles = 0;
         if (tiles && rows > 0 && hMax[4] != 0 && hMax[0] <= capN && hMax[1] <= capF)
@@ -498,17 +493,17 @@ int build_split_list(mrmd_ctx* ctx, mrmd_nlist* nearList, mrmd_nlist* farList, c
             // their tile form
             tiles->unfitTiles = hMax[4];
             tiles->twoPassBuilds++;
-            MRMD_CUDA(ctx, cudaMemsetAsync(maxCount + 3, 0, 3 * sizeof(int32_t), ctx->stream));
+            MRMD_TRY(clear_counts(ctx, maxCount));
             MRMD_TRY(int32_rows());
             MRMD_TRY(tile_build_launch(ctx, tiles, rows, nPos, nearList, farList, maxCount));
-            MRMD_CUDA(ctx, cudaMemcpyAsync(hMax, maxCount, 6 * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
-            MRMD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-            MRMD_TRY(bounds_check(ctx));
+            MRMD_TRY(read_flags(ctx, maxCount, &h));
         }
         if (hMax[0] <= capN && hMax[1] <= capF)
         {
             nearList->rows = farList->rows = rows;
             nearList->begin = farList->begin = begin;
+            nearList->totalPairs = (int64_t)h.totals[0];
+            farList->totalPairs = (int64_t)h.totals[1];
             if (tiles) tile_build_done(tiles, hMax[3], hMax[4] == 0, hMax[5]);
             return MRMD_OK;
         }
@@ -516,22 +511,6 @@ int build_split_list(mrmd_ctx* ctx, mrmd_nlist* nearList, mrmd_nlist* farList, c
         if (hMax[1] > capF) capF = hMax[1] + hMax[1] / 8 + 4;
     }
     return set_error(ctx, MRMD_ERR_NLIST_OVERFLOW, "neighbour list kept overflowing");
-}
-
-int list_total_pairs(mrmd_ctx* ctx, mrmd_nlist* nl)
-{
-    unsigned long long* d = reinterpret_cast<unsigned long long*>(ctx->devScalars + 8);
-    MRMD_CUDA(ctx, cudaMemsetAsync(d, 0, sizeof(unsigned long long), ctx->stream));
-    if (nl->rows > 0)
-    {
-        k_count_sum<<<grid_for(ctx, nl->rows, 256, 4), 256, 0, ctx->stream>>>(nl->counts, nl->rows, d);
-        MRMD_TRY(after_launch(ctx, "count_sum"));
-    }
-    unsigned long long h = 0;
-    MRMD_CUDA(ctx, cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
-    MRMD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    nl->totalPairs = (int64_t)h;
-    return MRMD_OK;
 }
 
 int check_list_fits(mrmd_ctx* ctx, const mrmd_nlist* nl, int64_t numLocal, int64_t nAll)
@@ -632,7 +611,6 @@ int mrmd_nlist_build(mrmd_ctx* ctx, mrmd_nlist* nl, const double* pos4, int64_t 
     CellGrid g = make_list_grid(gridMin, gridMax, rlist, nPos);
     (void)cellRatio;
     MRMD_TRY(build_half_list(ctx, nl, pos4, nPos, begin, end, rlist, g, maxNeighbors, false));
-    MRMD_TRY(list_total_pairs(ctx, nl));
     return finish(ctx, "nlist_build");
 }
 

@@ -120,6 +120,30 @@ __device__ __forceinline__ bool candidate_kept(const double4* __restrict__ pos, 
     return (d2 <= rsq) && (FULL || lex_above(pi, pj));
 }
 
+// What a list build counts on the device, cleared before it and read back
+// with one copy.
+struct ListFlags
+{
+    int32_t i[6];  // longest near and far rows, non-finite position, largest tile, tiles that did not fit, members
+    unsigned long long totals[2];  // entries of all near and all far rows
+};
+
+__host__ __device__ inline unsigned long long* list_totals(int32_t* flags)
+{
+    return reinterpret_cast<unsigned long long*>(flags + 6);
+}
+
+// The warps' entry counts into totals[0] (near or only rows) and [1] (far).
+__device__ __forceinline__ void add_totals(uint32_t nearRows, uint32_t farRows,
+                                           unsigned long long* __restrict__ totals)
+{
+    nearRows = __reduce_add_sync(0xffffffffu, nearRows);
+    farRows = __reduce_add_sync(0xffffffffu, farRows);
+    if ((threadIdx.x & 31) != 0) return;
+    if (nearRows) atomicAdd(totals, (unsigned long long)nearRows);
+    if (farRows) atomicAdd(totals + 1, (unsigned long long)farRows);
+}
+
 // Particles binned by cell: sorted[] holds particle ids in cell order
 // (ascending id inside a cell), spos[] their FP32 coordinates relative to
 // the grid origin with the id bit-cast into w.
@@ -127,8 +151,8 @@ struct CellList
 {
     CellGrid g{};
     int32_t* cellOf = nullptr;
-    int32_t* cellStart = nullptr;  // [ncell + 1]
-    int32_t* cursor = nullptr;
+    int32_t* cellStart = nullptr;  // [ncell + 1], then the scatter's cursors
+    int32_t* unordered = nullptr;
     int32_t* sorted = nullptr;
     float4* spos = nullptr;
     int64_t capN = 0, capCells = 0, numParticles = 0;
@@ -157,7 +181,6 @@ struct TileList;
 int build_split_list(mrmd_ctx* ctx, mrmd_nlist* nearList, mrmd_nlist* farList, const double* pos4, int64_t nPos,
                      int64_t begin, int64_t end, double rlist, double rnear, const CellGrid& grid,
                      TileList* tiles = nullptr, bool onePass = true);
-int list_total_pairs(mrmd_ctx* ctx, mrmd_nlist* nl);
 // The tile form of the split full list over rows [0, rows) built in one
 // pass from the cell list `cl` (tile_list.cu), without the int32 rows: the
 // near/far counts and tl's members and chunks.  flags as build_split_list's;

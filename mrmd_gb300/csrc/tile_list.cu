@@ -304,6 +304,7 @@ __global__ void __launch_bounds__(TILE_ROWS, 4) k_tile_list(
         if (an.cnt > capN) atomicMax(&flags[0], an.cnt);
         if (af.cnt > capF) atomicMax(&flags[1], af.cnt);
     }
+    add_totals((uint32_t)an.cnt, (uint32_t)af.cnt, list_totals(flags));
     __syncthreads();
 
     // ---- members: the used positions in order

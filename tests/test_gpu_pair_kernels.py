@@ -253,3 +253,60 @@ def test_mixed_half_lanes(M, orc, cells, drop, rc, cap, pred, lo):
     rms = np.sqrt((Fo ** 2).sum(1).mean())
     assert np.linalg.norm(F - Fo, axis=1).max() <= 1e-6 * rms
     assert abs(E - Eo) <= 1e-7 * abs(Eo)
+
+
+# Blocks of 1,024 atoms, the scan of 256 blocks at a time; boxes thinner than
+# two ghost layers (an atom with images on both sides of an axis).
+@pytest.mark.parametrize("n,box,thickness", [
+    (1, (6.0, 6.0, 6.0), 2.8), (1023, (14.0, 11.0, 9.0), 2.8), (1024, (5.0, 9.0, 4.0), 2.8),
+    (1025, (4.0, 4.0, 4.0), 3.5), (5000, (40.0, 3.0, 12.0), 2.8), (263200, (90.0, 60.0, 50.0), 2.8),
+    (700, (20.0, 20.0, 20.0), 0.0),
+])
+def test_ghost_images_bit_exact(M, orc, n, box, thickness):
+    """Ghost positions, order, real atoms and the folded-back forces are the
+    oracle's, bit for bit."""
+    rng = np.random.default_rng(n)
+    pos = rng.uniform(0, 1, (n, 3)) * np.asarray(box)
+    pos[:3] = np.array([[0.0, 0.0, 0.0], [thickness] * 3, np.asarray(box) - thickness])[: min(n, 3)] % np.asarray(box)
+    sd_o, sd_g = orc.subdomain([0, 0, 0], list(box), thickness), M.Subdomain([0, 0, 0], list(box), thickness)
+    ao = orc.Atoms.from_positions(pos, capacity=28 * n + 64 if n < 10000 else 2 * n)
+    corr = orc.create_ghosts(ao, sd_o)
+    ag = M.Atoms.from_arrays(pos, vel=pos * 2, type=np.arange(n) % 7, mass=1.0 + np.arange(n) % 3)  # room for n ghosts
+    gl = M.GhostLayer()
+    gl.createGhostAtoms(ag, sd_g)
+    assert ag.numGhostAtoms == ao.n - n
+    d = ag.download()
+    np.testing.assert_array_equal(d["pos"], ao.pos[: ao.n])
+    real = gl.correspondingRealAtom(ao.n)
+    np.testing.assert_array_equal(real[n:], corr[n: ao.n])
+    assert np.all(real[:n] == -1)
+    np.testing.assert_array_equal(d["vel"][n:], d["vel"][real[n:]])
+    np.testing.assert_array_equal(d["type"][n:], d["type"][real[n:]])
+    np.testing.assert_array_equal(d["mass"][n:], d["mass"][real[n:]])
+    f = rng.normal(0, 1, (ao.n, 3))
+    ao.force[: ao.n] = f
+    orc.ghost_to_real(ao, corr)
+    ag.upload(n, ao.n - n, force=f)
+    gl.contributeBackGhostToReal(ag)
+    np.testing.assert_array_equal(ag.getForce(), ao.force[: ao.n])
+
+
+# Half-radius cells of the list grid: one scan tile (1,024 cells) and one more
+# cell than that, many tiles, and more than 2,048 tiles (2,097,152 cells),
+# where the tile totals are scanned in a launch of their own.
+@pytest.mark.parametrize("n,box", [(900, (8.0, 8.0, 8.0)), (900, (20.5, 5.0, 2.5)), (5000, (30.0, 30.0, 30.0)),
+                                   (200000, (66.0, 66.0, 66.0))])
+def test_list_counts_over_scan_sizes(M, n, box):
+    """The half list's pairs are those within the radius, and its totals are
+    the sums of its counts."""
+    spatial = pytest.importorskip("scipy.spatial")
+    pos = np.random.default_rng(n).uniform(0, 1, (n, 3)) * np.asarray(box)
+    a = M.Atoms.from_arrays(pos)
+    vl = M.HalfVerletList()
+    vl.build(a, 0, n, 1.0, 1.0, [0.0] * 3, list(box), 30)
+    counts, nbrs = vl.download()
+    tree = spatial.cKDTree(pos)
+    assert vl.total_pairs == counts.sum() == (tree.count_neighbors(tree, 1.0) - n) // 2
+    got = np.concatenate([np.stack([np.full(c, i), nbrs[i, :c]], 1) for i, c in enumerate(counts) if c])
+    got = np.unique(np.sort(got, 1), axis=0)
+    np.testing.assert_array_equal(got, np.unique(np.sort(tree.query_pairs(1.0, output_type="ndarray"), 1), axis=0))
