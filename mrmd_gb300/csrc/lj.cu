@@ -95,12 +95,17 @@ constexpr int LJ_BLOCKS = 5;  // resident blocks per SM: with 6 or 7 the segment
 // length, 47 rounds for 38 entries.  At 256,000 atoms 4.91e6 FP64 warp
 // instructions (22 per pair in range are 4.85e6), FP64 pipe 76% active.
 // Measured times: lj_rows_per_warp.
+//
+// realOf (may be null): the real atom of every ghost; a ghost's force then goes
+// straight to it, and no fold-back follows (its pass over all atoms, bound by
+// its dependent loads, took 9 us of a 4,000-atom step and 20 at 256,000).
 template <bool PRED, bool MULTI, int R>
 __global__ void __launch_bounds__(LJ_TB, LJ_BLOCKS) k_lj_fp64(
     const double4* __restrict__ pos, double* __restrict__ force, const int32_t* __restrict__ type,
     const LJDev p0, const LJDev* __restrict__ table, int32_t numTypesIndex, double rcSqr, float rcSqrUp,
     const int32_t* __restrict__ counts, const int32_t* __restrict__ nbrs, int64_t cap, int64_t n,
-    int64_t begin, int64_t nAll, mrmd_dev::Pred pred, double* __restrict__ ev)
+    int64_t begin, int64_t nAll, mrmd_dev::Pred pred, const int32_t* __restrict__ realOf, int64_t nLocal,
+    double* __restrict__ ev)
 {
     constexpr int G = 32 / R;  // lanes scanning one row
     constexpr unsigned ALL = 0xffffffffu;
@@ -247,9 +252,10 @@ __global__ void __launch_bounds__(LJ_TB, LJ_BLOCKS) k_lj_fp64(
                     fx -= gx;
                     fy -= gy;
                     fz -= gz;
-                    atomicAdd(force + 4 * j + 0, gx);
-                    atomicAdd(force + 4 * j + 1, gy);
-                    atomicAdd(force + 4 * j + 2, gz);
+                    double* fj = force + 4 * (realOf && j >= nLocal ? (int64_t)realOf[j] : j);
+                    atomicAdd(fj + 0, gx);
+                    atomicAdd(fj + 1, gy);
+                    atomicAdd(fj + 2, gz);
                 }
                 atomicAdd(force + 4 * i + 0, fx);
                 atomicAdd(force + 4 * i + 1, fy);
@@ -297,7 +303,7 @@ int lj_rows_per_warp(const mrmd_ctx* ctx, int64_t n)
 }  // namespace
 
 int lj_apply_fp64(mrmd_ctx* ctx, const mrmd_lj* lj, mrmd_atoms* a, const mrmd_nlist* nl,
-                  const mrmd_pred* pred, double* ev)
+                  const mrmd_pred* pred, double* ev, const int32_t* realOf)
 {
     const int64_t n = nl->rows;
     if (n == 0) return MRMD_OK;
@@ -311,7 +317,7 @@ int lj_apply_fp64(mrmd_ctx* ctx, const mrmd_lj* lj, mrmd_atoms* a, const mrmd_nl
         const unsigned grid = (unsigned)(groups < most ? groups : most);
         kernel<<<grid, LJ_TB, 0, ctx->stream>>>(pos, a->force, a->type, lj->p0, lj->dTable, (int32_t)lj->numTypesIndex,
                                                 lj->rcSqr, rcSqrUp, nl->counts, nl->nbrs, nl->maxNeighbors, n,
-                                                nl->begin, a->numLocal + a->numGhost, dp, ev);
+                                                nl->begin, a->numLocal + a->numGhost, dp, realOf, a->numLocal, ev);
     };
 #define LJ_ROWS(R)                                              \
     if (usePred && multi) launch(k_lj_fp64<true, true, R>, R);  \

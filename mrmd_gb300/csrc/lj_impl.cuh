@@ -251,7 +251,7 @@ struct mrmd_lj
 namespace mrmd_impl
 {
 int lj_apply_fp64(mrmd_ctx* ctx, const mrmd_lj* lj, mrmd_atoms* a, const mrmd_nlist* nl,
-                  const mrmd_pred* pred, double* ev);
+                  const mrmd_pred* pred, double* ev, const int32_t* realOf = nullptr);
 int lj_apply_mixed(mrmd_ctx* ctx, const mrmd_lj* lj, mrmd_atoms* a, const mrmd_nlist* nl,
                    const mrmd_pred* pred, double* ev);
 }  // namespace mrmd_impl

@@ -7,7 +7,6 @@
 //   or ghost position update
 //   (mixed) FP32 split coordinates of local + ghost atoms
 //   pair force (FP64: half list + atomics; mixed: full list, no atomics)
-//   (FP64) ghost force fold-back
 // and the final post-kick when a run ends.  The kick arithmetic is the
 // reference's (two kicks with the same force, then the drift), so fusing
 // post(s-1) with pre(s) changes no bit.  The K-1 steps between rebuilds
@@ -310,8 +309,8 @@ int md_forces(mrmd_ctx* ctx, mrmd_md* md, double* ev, bool splitDone = false)
         return lj_tile_forces(ctx, &md->tiles, &md->list, &md->farList, md->rec, a->force, md->tp, ev,
                               nAll, md->cfg.gatherNeighbours != 0);
     }
-    MRMD_TRY(lj_apply_fp64(ctx, md->lj, a, &md->list, nullptr, ev));
-    return mrmd_ghost_reduce_force(ctx, &md->ghosts, a);
+    // the ghosts' forces go to their real atoms: no fold-back
+    return lj_apply_fp64(ctx, md->lj, a, &md->list, nullptr, ev, md->ghosts.correspondingRealAtom);
 }
 
 // Kick / drift / force reset of one step; prevRec (may be null) receives the
@@ -736,7 +735,7 @@ int mrmd_md_eval(mrmd_ctx* ctx, mrmd_md* md, int what, double* ev2)
         if (md->cfg.precision == MRMD_PREC_MIXED)
             return lj_tile_forces(ctx, &md->tiles, &md->list, &md->farList, md->rec, a->force, md->tp,
                                   ev, a->numLocal + a->numGhost, md->cfg.gatherNeighbours != 0);
-        return lj_apply_fp64(ctx, md->lj, a, &md->list, nullptr, ev);
+        return lj_apply_fp64(ctx, md->lj, a, &md->list, nullptr, ev, md->ghosts.correspondingRealAtom);
     }
     const int oldSync = ctx->sync;
     ctx->sync = 0;
