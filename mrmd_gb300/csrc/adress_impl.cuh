@@ -6,6 +6,7 @@
 #include <cmath>
 
 #include "common.cuh"
+#include "lj_impl.cuh"
 
 namespace mrmd_impl
 {
@@ -73,15 +74,15 @@ __device__ __forceinline__ void slab_eval(const SlabDev& s, double x, double& la
 }
 
 // CheckRegion.hpp:25-38 with REGION_CHECK_EPSILON = 0
-__device__ __forceinline__ bool is_at(double l) { return l >= 1.0; }
-__device__ __forceinline__ bool is_cg(double l) { return l <= 0.0; }
+__device__ __forceinline__ bool is_at(double l) { return ge_one(l); }
+__device__ __forceinline__ bool is_cg(double l) { return le_zero(l); }
 __device__ __forceinline__ bool is_hy(double l) { return !is_at(l) && !is_cg(l); }
 
 __device__ __forceinline__ int comp_bin(double lambda)
 {
     // MultiHistogram(0, 1, 200).getBin (data/MultiHistogram.hpp:60-66)
     const double inv = 1.0 / ((1.0 - 0.0) / (double)COMP_BINS);
-    int64_t b = (int64_t)floor((lambda - 0.0) * inv);
+    int64_t b = __double2ll_rd(lambda * inv);
     if (b < 0 || b >= COMP_BINS) return -1;
     return (int)b;
 }

@@ -641,7 +641,8 @@ __device__ __forceinline__ df df_shfl_xor(df v, int o)
     return {__shfl_xor_sync(0xffffffffu, v.h, o), __shfl_xor_sync(0xffffffffu, v.l, o)};
 }
 
-__device__ __forceinline__ double to_d(df v) { return (double)v.h + (double)v.l; }
+// (conversions on the integer pipe: of the FP64 pipe only the sum)
+__device__ __forceinline__ double to_d(df v) { return __dadd_rn(f32_to_f64(v.h), f32_to_f64(v.l)); }
 
 // CheckRegion's hybrid test on a double-float weight in [0, 1]
 __device__ __forceinline__ bool is_hy_df(float2 v)
@@ -718,6 +719,14 @@ constexpr int SCAN_CHUNK = 40;
 // 22 FP64 instructions (distance 3, r^2 3, force factor and energy 10,
 // weight 2, forces 3, energy 1; the comparisons are integer ones) against
 // ~40 for every entry before.
+//
+// Mixed rows are bound by the latency of their loads (24 warps on an SM wait
+// for entry, then weight, then coordinates, in turn), so the next entry is
+// loaded a round ahead and the partner's coordinates together with its
+// weight: 264 -> 211 us at 64 replicas (730,000 molecules), 425 -> 391 at
+// 1.04M, 29.9 -> 28.1 at 34,560.  (Weights a round ahead too: the same;
+// coordinates a round ahead: registers spill, 256 us; 72 or 64 registers a
+// thread for more warps: 232 and 219.)
 template <bool MIXED, int TPR, bool CL = false>
 __device__ __forceinline__ RowOut row_force(const BDev& B, int32_t i, bool valid, int sub, bool sampling, int32_t c,
                                             int lane, uint8_t* seg)
@@ -749,7 +758,7 @@ __device__ __forceinline__ RowOut row_force(const BDev& B, int32_t i, bool valid
     double dfx = 0.0, dfy = 0.0, dfz = 0.0, dvs = 0.0, dcs = 0.0;
     double imgFx = 0.0, energy = 0.0;
     float fenergy = 0.0f;
-    const int binAlpha = is_hy(la.y) ? comp_bin(la.x) : -1;
+    const int binAlpha = sampling && is_hy(la.y) ? comp_bin(la.x) : -1;
     float ffx = 0.0f, ffy = 0.0f, ffz = 0.0f, vsF = 0.0f, csF = 0.0f;  // FP32 sums of the far pairs
     // one list entry; returns the mixed form's (e, w) of the pair's energy e w
     const float2 none = make_float2(0.f, 0.f);
@@ -765,6 +774,14 @@ __device__ __forceinline__ RowOut row_force(const BDev& B, int32_t i, bool valid
             partModF = B.lamtf[j];
         else
             partMod = B.lamt[j];
+        // an own weight above zero: the partner's coordinates are needed
+        // whatever its weight is, and load beside it
+        float4 hj, lj;
+        if (MIXED && ltA.x > 0.0f)
+        {
+            hj = B.hi[j];
+            lj = B.lo[j];
+        }
         float2 ownImgF = ltA;
         int imgSide = 0;  // mixed form: 1 / 2 when the own slot is i's -L / +L image in x
         if (rev && !R.consistent)
@@ -816,7 +833,11 @@ __device__ __forceinline__ RowOut row_force(const BDev& B, int32_t i, bool valid
         {
             const float2 ownF = ownImgF;
             if (ownF.x <= 0.0f && partModF.x <= 0.0f) return none;  // both coarse grained: ideal gas
-            const float4 hj = B.hi[j], lj = B.lo[j];
+            if (!(ltA.x > 0.0f))
+            {
+                hj = B.hi[j];
+                lj = B.lo[j];
+            }
             if (B.farF32 && ownIsSelf)
             {
                 // beyond r_split: plain FP32 (the LJ pair force is at most
@@ -951,9 +972,12 @@ __device__ __forceinline__ RowOut row_force(const BDev& B, int32_t i, bool valid
             const int32_t* col = nbrs + mrmd_dev::nbr_row(i, cap);
             if (TPR == 1 || !B.rowOrderEnergy)
             {
+                int32_t ahead = sub < cnt ? col[32 * (int64_t)sub] : 0;
                 for (int k = sub; k < cnt; k += TPR)
                 {
-                    const float2 ew = pair_entry(col[32 * (int64_t)k]);
+                    const int32_t entry = ahead;
+                    if (k + TPR < cnt) ahead = col[32 * (int64_t)(k + TPR)];
+                    const float2 ew = pair_entry(entry);
                     fenergy = __fmaf_rn(ew.x, ew.y, fenergy);
                 }
                 return;
@@ -963,10 +987,13 @@ __device__ __forceinline__ RowOut row_force(const BDev& B, int32_t i, bool valid
             int most = cnt;
 #pragma unroll
             for (int off = 16; off >= TPR; off >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, off));
+            int32_t ahead = sub < cnt ? col[32 * (int64_t)sub] : 0;
             for (int k0 = 0; k0 < most; k0 += TPR)
             {
+                const int32_t entry = ahead;
+                if (k0 + TPR + sub < cnt) ahead = col[32 * (int64_t)(k0 + TPR + sub)];
                 float2 ew = none;
-                if (k0 + sub < cnt) ew = pair_entry(col[32 * (int64_t)(k0 + sub)]);
+                if (k0 + sub < cnt) ew = pair_entry(entry);
 #pragma unroll
                 for (int q = 0; q < TPR; ++q)
                     fenergy = __fmaf_rn(__shfl_sync(0xffffffffu, ew.x, q, TPR), __shfl_sync(0xffffffffu, ew.y, q, TPR),
@@ -1034,6 +1061,8 @@ __device__ __forceinline__ RowOut row_force(const BDev& B, int32_t i, bool valid
     RowOut o;
     if (MIXED)
     {
+        // the sums that a run or a box without them leaves at zero
+        const bool anyImg = __any_sync(0xffffffffu, !R.consistent), anyComp = __any_sync(0xffffffffu, sampling);
 #pragma unroll
         for (int off = 1; off < TPR; off <<= 1)
         {
@@ -1041,12 +1070,15 @@ __device__ __forceinline__ RowOut row_force(const BDev& B, int32_t i, bool valid
             fy = df_add(fy, df_shfl_xor(fy, off));
             fz = df_add(fz, df_shfl_xor(fz, off));
             vs = df_add(vs, df_shfl_xor(vs, off));
-            cs = df_add(cs, df_shfl_xor(cs, off));
-            vImgM = df_add(vImgM, df_shfl_xor(vImgM, off));
-            vImgP = df_add(vImgP, df_shfl_xor(vImgP, off));
+            if (anyComp) cs = df_add(cs, df_shfl_xor(cs, off));
+            if (anyImg)
+            {
+                vImgM = df_add(vImgM, df_shfl_xor(vImgM, off));
+                vImgP = df_add(vImgP, df_shfl_xor(vImgP, off));
+            }
         }
-        o.vImgM = to_d(vImgM);
-        o.vImgP = to_d(vImgP);
+        o.vImgM = anyImg ? to_d(vImgM) : 0.0;
+        o.vImgP = anyImg ? to_d(vImgP) : 0.0;
         o.fx = to_d(fx);
         o.fy = to_d(fy);
         o.fz = to_d(fz);
@@ -1072,16 +1104,17 @@ __device__ __forceinline__ RowOut row_force(const BDev& B, int32_t i, bool valid
         o.vImgM = 0.0;
         o.vImgP = 0.0;
     }
+    // (rowOrderEnergy: every lane has the row's energy already)
 #pragma unroll
     for (int off = 1; off < TPR; off <<= 1)
     {
-        imgFx += __shfl_xor_sync(0xffffffffu, imgFx, off);
-        if (MIXED && !CL && B.rowOrderEnergy)
-            continue;  // every lane has the row's sum
-        if (MIXED)
-            fenergy += __shfl_xor_sync(0xffffffffu, fenergy, off);
-        else
+        if (!MIXED)
+        {
+            imgFx += __shfl_xor_sync(0xffffffffu, imgFx, off);
             energy += __shfl_xor_sync(0xffffffffu, energy, off);
+        }
+        else if (CL || !B.rowOrderEnergy)
+            fenergy += __shfl_xor_sync(0xffffffffu, fenergy, off);
     }
     o.imgFx = imgFx;
     o.energy = energy;
@@ -1163,7 +1196,7 @@ __device__ __forceinline__ void force_body(const BDev& B, int64_t gtid, uint8_t*
         const double4 x = B.pos[i];
         if (B.tfEnabled)
         {
-            const int64_t b = (int64_t)floor((x.x - R.tfMin) * R.tfInvBin);
+            const int64_t b = __double2ll_rd((x.x - R.tfMin) * R.tfInvBin);
             if (b >= 0 && b < R.tfBins)
             {
                 f.x = __dadd_rn(f.x, B.tfForce[R.tfBase + b]);
