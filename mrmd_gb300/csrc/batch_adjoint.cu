@@ -83,10 +83,12 @@ LJDiff make_ljdiff(double eps, double sig, double rc, double rcap, int shifted)
     return L;
 }
 
-// f (force factor), e (energy), their s-derivatives and parameter partials
+// f (force factor), its s-derivative, e (energy; its s-derivative is -f/2, in
+// the cap too) and the sigma partials; the epsilon partials are f / epsilon
+// and e / epsilon
 struct LJVals
 {
-    double f, fp, e, ep, fe, fs, ee, es;
+    double f, fp, e, fs, es;
 };
 
 __device__ __forceinline__ LJVals lj_diff(const LJDiff& L, double s)
@@ -94,13 +96,12 @@ __device__ __forceinline__ LJVals lj_diff(const LJDiff& L, double s)
     LJVals o;
     if (s >= L.capSqr)
     {
-        const double u = 1.0 / s, u3 = u * u * u, u6 = u3 * u3;
-        o.f = u3 * u * (L.ff1 * u3 - L.ff2);
-        o.fp = u * u * (-7.0 * L.ff1 * u6 + 4.0 * L.ff2 * u3);
-        o.e = u3 * (L.ef1 * u3 - L.ef2) - L.shift;
-        o.ep = u * (-6.0 * L.ef1 * u6 + 3.0 * L.ef2 * u3);
-        o.fs = u3 * u * (L.ff1s * u3 - L.ff2s);
-        o.es = u3 * (L.ef1s * u3 - L.ef2s) - L.shifts;
+        const double u = rcp_series(s), u2 = u * u, u3 = u2 * u, u4 = u2 * u2;
+        o.f = u4 * fma(L.ff1, u3, -L.ff2);
+        o.fp = u2 * u3 * fma(-7.0 * L.ff1, u3, 4.0 * L.ff2);
+        o.e = fma(u3, fma(L.ef1, u3, -L.ef2), -L.shift);
+        o.fs = u4 * fma(L.ff1s, u3, -L.ff2s);
+        o.es = fma(u3, fma(L.ef1s, u3, -L.ef2s), -L.shifts);
     }
     else
     {
@@ -109,13 +110,9 @@ __device__ __forceinline__ LJVals lj_diff(const LJDiff& L, double s)
         o.f = L.C / r;
         o.fp = -0.5 * L.C / (s * r);
         o.e = L.Ec - (r - L.rcap) * L.C - L.shift;
-        o.ep = -0.5 * L.C / r;
         o.fs = L.Cs / r;
         o.es = L.Ecs - (r - L.rcap) * L.Cs - L.shifts;
     }
-    // every factor is proportional to epsilon
-    o.fe = o.f / L.eps;
-    o.ee = o.e / L.eps;
     return o;
 }
 
@@ -148,7 +145,9 @@ LJDiffF to_float(const LJDiff& L)
                    (float)L.rcSqr};
 }
 
-constexpr int ADJ_TPR = 4;  // lanes per row of the adjoint pair kernel
+constexpr int ADJ_TPR = 4;    // lanes per row of the adjoint pair kernel
+constexpr int ADJ_TB = 64;
+constexpr int ADJ_CHUNK = 128;  // entries scanned at a time (their places fit a byte)
 
 struct AdjArgs
 {
@@ -168,10 +167,22 @@ struct AdjArgs
 // TPR lanes share a row (entries k = sub, sub + TPR, ...) and reduce with a
 // fixed butterfly, so that the few long rows of the atomistic and hybrid
 // regions are spread over more warps.
+//
+// The kernel is bound by the FP64 pipe (two lanes a clock and SM), which a
+// warp holds for an entry as long with one lane at work as with 32.  So the
+// entries are walked once without FP64 work (the FP32 pairs are evaluated
+// there, MIXED; pairs surely beyond rc or of two coarse-grained molecules
+// dropped), and the rest is dealt evenly to the row's lanes: 3 FP64 rounds a
+// row instead of 17 in the mixed form.  A pair takes ~55 FP64 instructions
+// (one reciprocal, the parameter factors taken out of the sums) against ~110
+// before.  65,536 molecules, mixed: 164 -> 63 us.  Rows differ (coarse-grained
+// ones end at once), so blocks are small: 64 threads 63 us, 256 66; with 80 or
+// 64 registers a thread for more warps 77 and 103.
 template <bool MIXED, int TPR>
-__global__ void __launch_bounds__(TB) k_adj_force(BDev B, AdjArgs A)
+__global__ void __launch_bounds__(ADJ_TB, 8) k_adj_force(BDev B, AdjArgs A)
 {
     __shared__ double red[64];
+    __shared__ uint8_t places[ADJ_TB / TPR][ADJ_CHUNK];
     double ge = 0.0, gs = 0.0;
     const int64_t gtid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const bool valid = gtid < (int64_t)B.N * TPR;
@@ -195,71 +206,103 @@ __global__ void __launch_bounds__(TB) k_adj_force(BDev B, AdjArgs A)
             mi = B.lamtf[i].x;
             gi = (float)la.z;
         }
+        const float3 pf = make_float3(hi_word_f32(pi.x), hi_word_f32(pi.y), hi_word_f32(pi.z));
+        const float rcUp = (float)A.L.rcSqr * 1.000001f;
+        const bool ownCG = le_zero(la.y);
         const int cnt = valid ? B.counts[i] : 0;
-        const int64_t rowBase = mrmd_dev::nbr_row(i, B.listCap);
-        for (int k = sub; k < cnt; k += TPR)
-        {
-            const int32_t j = B.nbrs[rowBase + 32 * (int64_t)k] & 0x7fffffff;
-            if (MIXED)
+        const int32_t* col = B.nbrs + mrmd_dev::nbr_row(i, B.listCap);
+        // true: the entry needs the FP64 form
+        auto scan_entry = [&](const int32_t j) -> bool {
+            if (!MIXED)
             {
-                // no FP64 operation on the FP32 path: weights and adjoint in FP32
-                const float mj = B.lamtf[j].x;
-                if (mi <= 0.0f && mj <= 0.0f) continue;  // both coarse grained
-                const float4 hj = B.hi[j], loj = B.lo[j];
-                const float rx = (hi_i.x - hj.x) + (lo_i.x - loj.x);
-                const float ry = (hi_i.y - hj.y) + (lo_i.y - loj.y);
-                const float rz = (hi_i.z - hj.z) + (lo_i.z - loj.z);
-                const float s = __fmaf_rn(rx, rx, __fmaf_rn(ry, ry, rz * rz));
-                const LJDiffF& L = A.Lf;
-                if (s > L.rcSq * 1.0000005f) continue;
-                if (s >= B.rsplitSq && s < L.rcSq * 0.9999995f)
-                {
-                    // a ghost takes its source's adjoint and (the replica is
-                    // consistent) its source's weight derivative
-                    const int32_t src = j < B.N ? j : B.gSrc[j - B.N];
-                    const float4 afj = A.af[src];
-                    const float u = __fdividef(1.0f, s), u3 = u * u * u, u6 = u3 * u3;
-                    const float f = u3 * u * __fmaf_rn(L.ff1, u3, -L.ff2);
-                    const float fp = u * u * __fmaf_rn(-7.0f * L.ff1, u6, 4.0f * L.ff2 * u3);
-                    const float e = __fmaf_rn(u3, __fmaf_rn(L.ef1, u3, -L.ef2), -L.shift);
-                    const float ep = u * __fmaf_rn(-6.0f * L.ef1, u6, 3.0f * L.ef2 * u3);
-                    const float fs = u3 * u * __fmaf_rn(L.ff1s, u3, -L.ff2s);
-                    const float es = __fmaf_rn(u3, __fmaf_rn(L.ef1s, u3, -L.ef2s), -L.shifts);
-                    const float w = 0.5f * (mi + mj);
-                    const float dax = afi.x - afj.x, day = afi.y - afj.y, daz = afi.z - afj.z;
-                    const float q = __fmaf_rn(dax, rx, __fmaf_rn(day, ry, daz * rz));
-                    const float agsum = afi.w + afj.w;
-                    const float c1 = 2.0f * w * fp * q - ep * agsum;
-                    fbx += c1 * rx + w * f * dax + 0.5f * gi * f * q;
-                    fby += c1 * ry + w * f * day;
-                    fbz += c1 * rz + w * f * daz;
-                    fesum += e;
-                    fge += 0.5f * (w * q * f - 0.5f * e * agsum) * L.invEps;
-                    fgs += 0.5f * (w * q * fs - 0.5f * es * agsum);
-                    continue;
-                }
+                if (ownCG && le_zero(B.lamt[j])) return false;  // both coarse grained
+                return !surely_beyond(pf, mrmd_dev::ldg4(B.pos + j), rcUp);
             }
-            const double4 lj = B.lam[j];
-            if (!MIXED && la.y <= 0.0 && lj.y <= 0.0) continue;  // both coarse grained
+            // no FP64 operation on the FP32 path: weights and adjoint in FP32
+            const float mj = B.lamtf[j].x;
+            if (mi <= 0.0f && mj <= 0.0f) return false;  // both coarse grained
+            const float4 hj = B.hi[j], loj = B.lo[j];
+            const float rx = (hi_i.x - hj.x) + (lo_i.x - loj.x);
+            const float ry = (hi_i.y - hj.y) + (lo_i.y - loj.y);
+            const float rz = (hi_i.z - hj.z) + (lo_i.z - loj.z);
+            const float s = __fmaf_rn(rx, rx, __fmaf_rn(ry, ry, rz * rz));
+            const LJDiffF& L = A.Lf;
+            if (s > L.rcSq * 1.0000005f) return false;
+            if (!(s >= B.rsplitSq && s < L.rcSq * 0.9999995f)) return true;
+            // a ghost takes its source's adjoint and (the replica is
+            // consistent) its source's weight derivative
+            const int32_t src = j < B.N ? j : B.gSrc[j - B.N];
+            const float4 afj = A.af[src];
+            const float u = __fdividef(1.0f, s), u3 = u * u * u, u6 = u3 * u3;
+            const float f = u3 * u * __fmaf_rn(L.ff1, u3, -L.ff2);
+            const float fp = u * u * __fmaf_rn(-7.0f * L.ff1, u6, 4.0f * L.ff2 * u3);
+            const float e = __fmaf_rn(u3, __fmaf_rn(L.ef1, u3, -L.ef2), -L.shift);
+            const float ep = u * __fmaf_rn(-6.0f * L.ef1, u6, 3.0f * L.ef2 * u3);
+            const float fs = u3 * u * __fmaf_rn(L.ff1s, u3, -L.ff2s);
+            const float es = __fmaf_rn(u3, __fmaf_rn(L.ef1s, u3, -L.ef2s), -L.shifts);
+            const float w = 0.5f * (mi + mj);
+            const float dax = afi.x - afj.x, day = afi.y - afj.y, daz = afi.z - afj.z;
+            const float q = __fmaf_rn(dax, rx, __fmaf_rn(day, ry, daz * rz));
+            const float agsum = afi.w + afj.w;
+            const float c1 = 2.0f * w * fp * q - ep * agsum;
+            fbx += c1 * rx + w * f * dax + 0.5f * gi * f * q;
+            fby += c1 * ry + w * f * day;
+            fbz += c1 * rz + w * f * daz;
+            fesum += e;
+            fge += 0.5f * (w * q * f - 0.5f * e * agsum) * L.invEps;
+            fgs += 0.5f * (w * q * fs - 0.5f * es * agsum);
+            return false;
+        };
+        double gq = 0.0;  // sum of f q / 2 (times g_i: the pair term of the own weight)
+        auto pair_entry = [&](const int32_t j) {
             const double4 pj = B.pos[j];
             const double rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
             const double s = rx * rx + ry * ry + rz * rz;
-            if (s > A.L.rcSqr) continue;
+            if (gt_nonneg(s, A.L.rcSqr)) return;
+            const double4 lj = B.lam[j];
             const int32_t src = j < B.N ? j : B.gSrc[j - B.N];
             const double4 aj = A.a[src];
             const LJVals V = lj_diff(A.L, s);
-            const double w = 0.5 * (la.y + lj.y);
+            const double w2 = la.y + lj.y;  // 2 w_ij
             const double dax = ai.x - aj.x, day = ai.y - aj.y, daz = ai.z - aj.z;
             const double q = dax * rx + day * ry + daz * rz;
-            const double agj = aj.x * lj.z;
-            const double c1 = 2.0 * w * V.fp * q - V.ep * (agi + agj);
-            bx += c1 * rx + w * V.f * dax + 0.5 * la.z * V.f * q;
-            by += c1 * ry + w * V.f * day;
-            bz += c1 * rz + w * V.f * daz;
+            const double ag = fma(aj.x, lj.z, agi);
+            const double wq = w2 * q, hf = 0.5 * V.f, wf = w2 * hf;
+            const double c1 = fma(wq, V.fp, hf * ag);  // 2 w f' q - e' ag
+            bx = fma(c1, rx, fma(wf, dax, bx));
+            by = fma(c1, ry, fma(wf, day, by));
+            bz = fma(c1, rz, fma(wf, daz, bz));
+            gq = fma(hf, q, gq);
             esum += V.e;
-            ge += 0.5 * (w * q * V.fe - 0.5 * V.ee * (agi + agj));
-            gs += 0.5 * (w * q * V.fs - 0.5 * V.es * (agi + agj));
+            // 4 epsilon and 4 times the parameter terms of half the pair
+            ge += fma(wq, V.f, -(V.e * ag));
+            gs += fma(wq, V.fs, -(V.es * ag));
+        };
+        const unsigned mine = ((1u << TPR) - 1u) << (threadIdx.x & 31 & ~(TPR - 1));
+        const unsigned before = mine & ((1u << (threadIdx.x & 31)) - 1u);
+        uint8_t* place = places[threadIdx.x / TPR];
+        int most = cnt;
+#pragma unroll
+        for (int off = 16; off >= TPR; off >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, off));
+        for (int k0 = 0; k0 < most; k0 += ADJ_CHUNK)
+        {
+            int kept = 0;
+            const int kEnd = min(k0 + ADJ_CHUNK, most);
+            for (int kk = k0; kk < kEnd; kk += TPR)
+            {
+                const int k = kk + sub;
+                const bool keep = k < cnt && scan_entry(col[32 * (int64_t)k] & 0x7fffffff);
+                const unsigned m = __ballot_sync(0xffffffffu, keep);
+                if (keep) place[kept + __popc(m & before)] = (uint8_t)(k - k0);
+                kept += __popc(m & mine);
+            }
+            __syncwarp();
+            for (int q = sub; q < kept; q += TPR) pair_entry(col[32 * (int64_t)(k0 + place[q])] & 0x7fffffff);
+            __syncwarp();
         }
+        bx = fma(la.z, gq, bx);
+        ge *= 0.25 / A.L.eps;
+        gs *= 0.25;
         if (MIXED)
         {
             bx += (double)fbx;
@@ -352,47 +395,75 @@ struct LossDev
 {
     double xmin, Lx, binW, invSig2, norm, cutoff;
     int32_t bins;
-    double* rho;        // [bins] sum of kernel values
+    int32_t copies;     // 1 or 32
+    double* rho;        // [bins][copies] sums of kernel values
+    double* fold;       // [bins] sums over the copies
     const double* coef; // [bins] dL/d(rho_b) / (window * area)
 };
 
-__global__ void k_loss_density(BDev B, LossDev D)
+// Calls f(bin, d) for the bins whose centre lies within the cutoff of x, d the
+// distance to the nearest image of the centre.
+template <typename F>
+__device__ __forceinline__ void for_bins(const LossDev& D, double x, F f)
 {
     const int span = (int)ceil(D.cutoff / D.binW) + 1;
-    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < B.N; i += gridDim.x * blockDim.x)
+    const int b0 = (int)floor((x - D.xmin) / D.binW);
+    // bins visited once each: the centre counted from b0 is the nearest image
+    // already, and the period (a division per bin) drops out
+    const bool once = 2 * (span + 1) <= D.bins;
+    const double d0 = x - (D.xmin + ((double)b0 + 0.5) * D.binW);
+    double o = -(double)span;
+    int b = (b0 - span) % D.bins;
+    if (b < 0) b += D.bins;
+    for (int k = -span; k <= span; ++k, o += 1.0)
     {
-        const double x = B.pos[i].x;
-        const int b0 = (int)floor((x - D.xmin) / D.binW);
-        for (int o = -span; o <= span; ++o)
+        double d;
+        if (once)
+            d = fma(-o, D.binW, d0);
+        else
         {
-            int b = (b0 + o) % D.bins;
-            if (b < 0) b += D.bins;
-            double d = x - (D.xmin + ((double)b + 0.5) * D.binW);
+            d = x - (D.xmin + ((double)b + 0.5) * D.binW);
             d -= D.Lx * rint(d / D.Lx);
-            if (fabs(d) > D.cutoff) continue;
-            atomicAdd(D.rho + b, D.norm * exp(-0.5 * d * d * D.invSig2));
         }
+        if (!(fabs(d) > D.cutoff)) f(b, d);
+        b = b + 1 == D.bins ? 0 : b + 1;
     }
+}
+
+// Bound by the atomics while neighbouring molecules, which fall into the same
+// bins, meet at one address (the L2 slice that holds it takes one a clock):
+// with `copies` each lane adds to its own column, and a warp's adds go to
+// consecutive addresses.  65,536 molecules: 136 -> 30 us (and k_loss_grad 47
+// -> 31, which is bound by its exponentials on the FP64 pipe).
+__global__ void k_loss_density(BDev B, LossDev D)
+{
+    const int copy = threadIdx.x & (D.copies - 1);
+    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < B.N; i += gridDim.x * blockDim.x)
+        for_bins(D, B.pos[i].x, [&](int b, double d) {
+            atomicAdd(D.rho + (int64_t)b * D.copies + copy, D.norm * exp(-0.5 * d * d * D.invSig2));
+        });
+}
+
+// the sums of the bins' copies, one warp a bin
+__global__ void k_loss_fold(LossDev D)
+{
+    const int b = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (b >= D.bins) return;
+    double v = lane < D.copies ? D.rho[(int64_t)b * D.copies + lane] : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) D.fold[b] = v;
 }
 
 __global__ void k_loss_grad(BDev B, LossDev D, double4* __restrict__ xbar)
 {
-    const int span = (int)ceil(D.cutoff / D.binW) + 1;
+    const double c = D.norm * D.invSig2;
     for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < B.N; i += gridDim.x * blockDim.x)
     {
-        const double x = B.pos[i].x;
-        const int b0 = (int)floor((x - D.xmin) / D.binW);
         double g = 0.0;
-        for (int o = -span; o <= span; ++o)
-        {
-            int b = (b0 + o) % D.bins;
-            if (b < 0) b += D.bins;
-            double d = x - (D.xmin + ((double)b + 0.5) * D.binW);
-            d -= D.Lx * rint(d / D.Lx);
-            if (fabs(d) > D.cutoff) continue;
-            g += D.coef[b] * (-d * D.invSig2) * D.norm * exp(-0.5 * d * d * D.invSig2);
-        }
-        xbar[i].x += g;
+        for_bins(D, B.pos[i].x,
+                 [&](int b, double d) { g = fma(D.coef[b] * -d, exp(-0.5 * d * d * D.invSig2), g); });
+        xbar[i].x += c * g;
     }
 }
 }  // namespace
@@ -412,7 +483,8 @@ struct mrmd_diff
     float4* adjf = nullptr;  // mixed form: FP32 copy of adj
     double* grad = nullptr;    // [2]
     double* tfGrad = nullptr;  // [nBins]
-    double* rho = nullptr;     // [lossBins]
+    double* rho = nullptr;     // [lossBins][copies]
+    double* fold = nullptr;    // [lossBins]
     double* coef = nullptr;    // [lossBins]
     std::vector<double> hRho;
     bool haveForward = false;
@@ -420,6 +492,10 @@ struct mrmd_diff
 
 namespace
 {
+// columns of the density: with more bins than that the molecules spread over
+// the bins themselves
+int32_t loss_copies(const mrmd_diff* d) { return d->dc.lossBins <= 4096 ? 32 : 1; }
+
 LossDev loss_dev(const mrmd_diff* d)
 {
     LossDev D{};
@@ -430,7 +506,9 @@ LossDev loss_dev(const mrmd_diff* d)
     D.invSig2 = 1.0 / (d->dc.lossSigma * d->dc.lossSigma);
     D.norm = 1.0 / (std::sqrt(2.0 * 3.141592653589793238462643383279502884) * d->dc.lossSigma);
     D.cutoff = 6.0 * d->dc.lossSigma;
+    D.copies = loss_copies(d);
     D.rho = d->rho;
+    D.fold = d->fold;
     D.coef = d->coef;
     return D;
 }
@@ -515,7 +593,8 @@ int mrmd_diff_create(mrmd_ctx* ctx, mrmd_diff** out, const mrmd_batch_config* cf
     if (rc == MRMD_OK) rc = grow(ctx, d->adjf, 0, N);
     if (rc == MRMD_OK) rc = grow(ctx, d->grad, 0, (int64_t)2);
     if (rc == MRMD_OK) rc = grow(ctx, d->tfGrad, 0, (int64_t)std::max(d->nBins, 1));
-    if (rc == MRMD_OK) rc = grow(ctx, d->rho, 0, dc->lossBins);
+    if (rc == MRMD_OK) rc = grow(ctx, d->rho, 0, dc->lossBins * loss_copies(d));
+    if (rc == MRMD_OK) rc = grow(ctx, d->fold, 0, dc->lossBins);
     if (rc == MRMD_OK) rc = grow(ctx, d->coef, 0, dc->lossBins);
     if (rc == MRMD_OK) rc = snapshot(ctx, d->b, d->init, true);
     if (rc == MRMD_OK) rc = check_cuda(ctx, cudaStreamSynchronize(ctx->stream), "diff create");
@@ -535,7 +614,7 @@ int mrmd_diff_destroy(mrmd_ctx* ctx, mrmd_diff* d)
     if (ctx) cudaStreamSynchronize(ctx->stream);
     snap_free(d->init);
     for (auto& s : d->ckpt) snap_free(s);
-    void* ptrs[] = {d->x2, d->xbar, d->vbar, d->Fbar, d->adj, d->adjf, d->grad, d->tfGrad, d->rho, d->coef};
+    void* ptrs[] = {d->x2, d->xbar, d->vbar, d->Fbar, d->adj, d->adjf, d->grad, d->tfGrad, d->rho, d->fold, d->coef};
     for (void* p : ptrs) dfree(p);
     if (d->b) mrmd_batch_destroy(ctx, d->b);
     delete d;
@@ -576,7 +655,9 @@ int mrmd_diff_forward(mrmd_ctx* ctx, mrmd_diff* d, const double* tfTable, double
     // the initial state first: its snapshot holds a TF table too
     int rc = restore_initial(ctx, d);
     if (rc == MRMD_OK) rc = set_params(ctx, d, tfTable, epsilon, sigma);
-    if (rc == MRMD_OK) rc = check_cuda(ctx, cudaMemsetAsync(d->rho, 0, sizeof(double) * d->dc.lossBins, ctx->stream), "rho");
+    if (rc == MRMD_OK)
+        rc = check_cuda(ctx, cudaMemsetAsync(d->rho, 0, sizeof(double) * d->dc.lossBins * loss_copies(d), ctx->stream),
+                        "rho");
     const int64_t S = d->dc.steps, C = d->dc.checkpointInterval, W = d->dc.window;
     for (int64_t st = 0; st < S && rc == MRMD_OK; ++st)
     {
@@ -585,7 +666,12 @@ int mrmd_diff_forward(mrmd_ctx* ctx, mrmd_diff* d, const double* tfTable, double
         if (rc == MRMD_OK && st >= S - W) rc = accumulate_density(ctx, d);
     }
     b->steps = S;
-    if (rc == MRMD_OK) rc = d2h(ctx, d->hRho.data(), d->rho, sizeof(double) * d->dc.lossBins);
+    if (rc == MRMD_OK)
+    {
+        k_loss_fold<<<(unsigned)div_up(d->dc.lossBins * 32, TB), TB, 0, ctx->stream>>>(loss_dev(d));
+        rc = after_launch(ctx, "loss fold");
+    }
+    if (rc == MRMD_OK) rc = d2h(ctx, d->hRho.data(), d->fold, sizeof(double) * d->dc.lossBins);
     ctx->sync = oldSync;
     MRMD_TRY(rc);
     // L = sum_b (rho_b - rho_uniform)^2, rho_b = kernel sum / (window * area)
@@ -684,11 +770,11 @@ int mrmd_diff_backward(mrmd_ctx* ctx, mrmd_diff* d, double* gradTable, double* g
             }
             if (rc == MRMD_OK)
             {
-                const unsigned ga = (unsigned)div_up((int64_t)N * ADJ_TPR, TB);
+                const unsigned ga = (unsigned)div_up((int64_t)N * ADJ_TPR, ADJ_TB);
                 if (mixed)
-                    k_adj_force<true, ADJ_TPR><<<ga, TB, 0, ctx->stream>>>(b->B, A);
+                    k_adj_force<true, ADJ_TPR><<<ga, ADJ_TB, 0, ctx->stream>>>(b->B, A);
                 else
-                    k_adj_force<false, ADJ_TPR><<<ga, TB, 0, ctx->stream>>>(b->B, A);
+                    k_adj_force<false, ADJ_TPR><<<ga, ADJ_TB, 0, ctx->stream>>>(b->B, A);
                 rc = after_launch(ctx, "adj force");
             }
             if (rc == MRMD_OK && st >= S - W)
@@ -754,10 +840,10 @@ int mrmd_diff_force_vjp(mrmd_ctx* ctx, mrmd_diff* d, const double* tfTable, doub
         if (b->cfg.precision == MRMD_PREC_MIXED)
         {
             k_adj_float<<<grid_for(ctx, (int64_t)N, TB), TB, 0, ctx->stream>>>(d->adj, b->B.lam, (int32_t)N, d->adjf);
-            k_adj_force<true, ADJ_TPR><<<(unsigned)div_up((int64_t)N * ADJ_TPR, TB), TB, 0, ctx->stream>>>(b->B, A);
+            k_adj_force<true, ADJ_TPR><<<(unsigned)div_up((int64_t)N * ADJ_TPR, ADJ_TB), ADJ_TB, 0, ctx->stream>>>(b->B, A);
         }
         else
-            k_adj_force<false, ADJ_TPR><<<(unsigned)div_up((int64_t)N * ADJ_TPR, TB), TB, 0, ctx->stream>>>(b->B, A);
+            k_adj_force<false, ADJ_TPR><<<(unsigned)div_up((int64_t)N * ADJ_TPR, ADJ_TB), ADJ_TB, 0, ctx->stream>>>(b->B, A);
         rc = after_launch(ctx, "adj force");
     }
     if (rc == MRMD_OK && xbar3) rc = d2h(ctx, h.data(), d->xbar, sizeof(double4) * N);

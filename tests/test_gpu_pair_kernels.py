@@ -310,3 +310,62 @@ def test_list_counts_over_scan_sizes(M, n, box):
     got = np.concatenate([np.stack([np.full(c, i), nbrs[i, :c]], 1) for i, c in enumerate(counts) if c])
     got = np.unique(np.sort(got, 1), axis=0)
     np.testing.assert_array_equal(got, np.unique(np.sort(tree.query_pairs(1.0, output_type="ndarray"), 1), axis=0))
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("n", [2, 9, 128, 129, 130, 300])
+def test_adjoint_rows_over_chunk_edges(M, n, prec):
+    """The adjoint of one force evaluation with rows of n - 1 entries (chunks
+    of 128; n = 130, 300: more than one), all pairs in range and atomistic,
+    against the sum over pairs in FP64.  FP64: 1e-12 of the summed magnitudes
+    (under 100 roundings a pair and 300 adds, each 2^-53, is 5e-14).  Mixed:
+    pairs beyond r_split in FP32, about 20 roundings a term and 75 adds a lane,
+    each 2^-24: 6e-6 of the magnitudes."""
+    rng = np.random.default_rng(n)
+    box, rc, cap = [40.0, 10.0, 10.0], 2.5, 0.7842
+    pos = np.array([19.3, 4.3, 4.3]) + rng.uniform(0, 1.4, (n, 3))
+    rep = M.Replica(n, [0, 0, 0], box, [20.0, 5.0, 5.0], 10.0, 31)
+    d = M.DiffSystem(rep, pos, np.zeros((n, 3)), hybrid_diameter=5.0, steps=5, window=5, checkpoint_interval=5,
+                     loss_bins=32, loss_sigma=1.0, capping_distance=cap, rebuild_interval=5,
+                     precision=M.PREC_FP64 if prec == "fp64" else M.PREC_MIXED)
+    a = rng.normal(size=(n, 3))
+    _, xbar, _, ge, gs = d.force_vjp(np.zeros(d.num_bins), 1.0, 1.0, a)
+    r = pos[:, None] - pos[None]
+    da = a[:, None] - a[None]
+    s = (r * r).sum(2) + np.eye(n)
+    q = (da * r).sum(2)
+    far = s >= cap * cap
+    C = 48 * cap ** -13 - 24 * cap ** -7  # force at the cap, d/dsigma below
+    Cs = 12 * 48 * cap ** -13 - 6 * 24 * cap ** -7
+    f = np.where(far, 48 * s ** -7 - 24 * s ** -4, C / np.sqrt(s))
+    fp = np.where(far, -7 * 48 * s ** -8 + 4 * 24 * s ** -5, -0.5 * C * s ** -1.5)
+    fs = np.where(far, 12 * 48 * s ** -7 - 6 * 24 * s ** -4, Cs / np.sqrt(s))
+    off = 1.0 - np.eye(n)
+    t1, t2 = 2 * (fp * q * off)[:, :, None] * r, (f * off)[:, :, None] * da
+    tol = 1e-12 if prec == "fp64" else 6e-6
+    assert np.all(np.abs(xbar - (t1 + t2).sum(1)) <= tol * (np.abs(t1) + np.abs(t2)).sum(1))
+    assert abs(ge - 0.5 * (q * f * off).sum()) <= tol * np.abs(q * f * off).sum()
+    assert abs(gs - 0.5 * (q * fs * off).sum()) <= tol * np.abs(q * fs * off).sum()
+
+
+# Bins wider than the kernel's reach allows for one visit each (4, 5), the
+# first count that takes the direct form (6), 32 columns a bin and one (4,097)
+@pytest.mark.parametrize("bins", [4, 5, 6, 33, 4096, 4097])
+def test_density_loss_over_bin_counts(M, bins):
+    """The loss of one step's smoothed density against NumPy in FP64 (a sum of
+    n terms rounds to under 1e-13 of itself)."""
+    n, L, area = 500, 40.0, 100.0
+    rng = np.random.default_rng(5)
+    pos = rng.uniform(0, 1, (n, 3)) * [L, 10.0, 10.0]
+    rep = M.Replica(n, [0, 0, 0], [L, 10.0, 10.0], [20.0, 5.0, 5.0], 10.0, 31)
+    d = M.DiffSystem(rep, pos, rng.normal(size=(n, 3)), hybrid_diameter=5.0, steps=1, window=1, checkpoint_interval=5,
+                     loss_bins=bins, loss_sigma=1.0, capping_distance=0.7842, rebuild_interval=5,
+                     precision=M.PREC_FP64)
+    tab = rng.normal(0, 0.3, d.num_bins)
+    L0 = d.forward(tab, 1.0, 1.0)
+    x = d.state()[0][:, 0]
+    dd = x[:, None] - (np.arange(bins) + 0.5) * (L / bins)
+    dd -= L * np.rint(dd / L)
+    k = np.where(np.abs(dd) > 6.0, 0.0, np.exp(-0.5 * dd * dd) / np.sqrt(2 * np.pi))
+    rho = k.sum(0) / area
+    assert abs(L0 - ((rho - n / (L * area)) ** 2).sum()) <= 1e-11 * (rho ** 2).sum()
