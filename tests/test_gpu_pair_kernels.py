@@ -369,3 +369,42 @@ def test_density_loss_over_bin_counts(M, bins):
     k = np.where(np.abs(dd) > 6.0, 0.0, np.exp(-0.5 * dd * dd) / np.sqrt(2 * np.pi))
     rho = k.sum(0) / area
     assert abs(L0 - ((rho - n / (L * area)) ** 2).sum()) <= 1e-11 * (rho ** 2).sum()
+
+
+# Blocks of 256 and of 1,024 molecules (above 152 * 1,024), one to three atoms
+# in a molecule, boxes thinner than two ghost layers
+@pytest.mark.parametrize("n,box,thickness", [
+    (1, (6.0, 6.0, 6.0), 2.8), (255, (4.0, 9.0, 5.0), 2.8), (257, (14.0, 3.5, 9.0), 2.8), (5000, (40.0, 12.0, 12.0), 2.8),
+    (160000, (90.0, 60.0, 50.0), 2.8), (300, (20.0, 20.0, 20.0), 0.0),
+])
+def test_molecule_images_bit_exact(M, orc, n, box, thickness):
+    """Ghost molecules and their atoms, in the oracle's order, bit for bit."""
+    rng = np.random.default_rng(n)
+    size = rng.integers(1, 4, n)
+    first = np.concatenate([[0], np.cumsum(size)[:-1]])
+    na = int(size.sum())
+    mpos = rng.uniform(0, 1, (n, 3)) * np.asarray(box)
+    apos = np.repeat(mpos, size, axis=0) + rng.normal(0, 0.15, (na, 3))
+    room = 27 if n < 10000 else 3
+    mo = orc.Molecules(n * room + 64)
+    mo.pos[:n], mo.atomsOffset[:n], mo.numAtoms[:n], mo.numLocal = mpos, first, size, n
+    mo.lambda_[:n] = rng.uniform(0, 1, n)
+    ao = orc.Atoms.from_positions(apos, capacity=na * room + 64)
+    corr = orc.multires_create_ghosts(mo, ao, orc.subdomain([0, 0, 0], list(box), thickness))
+    m = M.Molecules(n)  # room for no ghost
+    m.upload(n, 0, pos=mpos, force=np.zeros((n, 3)), lambda_=mo.lambda_[:n], modulated_lambda=np.zeros(n),
+             grad_lambda=np.zeros((n, 3)), atoms_offset=first, num_atoms=size)
+    a = M.Atoms.from_arrays(apos, type=np.arange(na) % 7)
+    gl = M.MultiResGhostLayer()
+    gl.createGhostAtoms(m, a, M.Subdomain([0, 0, 0], list(box), thickness))
+    nm, nt = mo.numLocal + mo.numGhost, ao.numLocal + ao.numGhost
+    assert (m.numGhostMolecules, a.numGhostAtoms) == (mo.numGhost, ao.numGhost)
+    d, da = m.download(), a.download()
+    np.testing.assert_array_equal(d["pos"], mo.pos[:nm])
+    np.testing.assert_array_equal(d["atomsOffset"], mo.atomsOffset[:nm])
+    np.testing.assert_array_equal(d["numAtoms"], mo.numAtoms[:nm])
+    np.testing.assert_array_equal(d["lambda_"], mo.lambda_[:nm])
+    np.testing.assert_array_equal(da["pos"], ao.pos[:nt])
+    real = gl.correspondingRealAtom(nt)
+    np.testing.assert_array_equal(real[na:], corr[na:nt])
+    np.testing.assert_array_equal(da["type"][na:], da["type"][real[na:]])
