@@ -45,6 +45,8 @@ CellGrid make_grid(const double* gridMin, const double* gridMax, double delta, i
     g.rdx = make_double3(rdx[0], rdx[1], rdx[2]);
     g.mnf = make_float3((float)mn[0], (float)mn[1], (float)mn[2]);
     g.rdxf = make_float3((float)rdx[0], (float)rdx[1], (float)rdx[2]);
+    g.h = make_float3((float)(1.0 / rdx[0]), (float)(1.0 / rdx[1]), (float)(1.0 / rdx[2]));
+    g.margin = (float)std::ldexp(extent, -20);
     g.n = make_int3(n[0], n[1], n[2]);
     g.ncell = (int64_t)n[0] * n[1] * n[2];
     g.extent = extent;
@@ -176,7 +178,7 @@ __global__ void __launch_bounds__(128) k_build_list(
         const double4 pi = pos[i];
         const float xi = (float)(pi.x - g.mn.x), yi = (float)(pi.y - g.mn.y), zi = (float)(pi.z - g.mn.z);
         const int cz = ci % g.n.z, cy = (ci / g.n.z) % g.n.y, cx = ci / (g.n.z * g.n.y);
-        const int z0 = max(cz - g.reach, 0), z1 = min(cz + g.reach, g.n.z - 1);
+        const int za = max(cz - g.reach, 0), zb = min(cz + g.reach, g.n.z - 1);
         int32_t cnt = 0, cntFar = 0;
         const int64_t row = i - begin;
         int32_t* __restrict__ out = nbrs + mrmd_dev::nbr_row(row, cap);
@@ -187,7 +189,9 @@ __global__ void __launch_bounds__(128) k_build_list(
             for (int ay = cy - g.reach; ay <= cy + g.reach; ++ay)
             {
                 int32_t s0 = 0, len = 0;
-                if (ok && ax >= 0 && ax < g.n.x && ay >= 0 && ay < g.n.y)
+                int z0 = za, z1 = zb;
+                if (ok && ax >= 0 && ax < g.n.x && ay >= 0 && ay < g.n.y &&
+                    trim_column(g, xi, yi, zi, rsqHi, cx, cy, ax, ay, z0, z1))
                 {
                     const int32_t c0 = (ax * g.n.y + ay) * g.n.z;
                     s0 = cellStart[c0 + z0];
@@ -289,7 +293,8 @@ int build_rows(mrmd_ctx* ctx, const CellList& cl, const double* pos4, int64_t be
     // warps that wait for their loads; one for large systems, where the
     // ballots cost more than the idle lanes.  us per launch of the half list
     // with 1 / 2 / 4 / 8 / 16 lanes: 32,000 atoms 56 / 43 / 28 / 35 / 46,
-    // 256,000 atoms 126 / 154 / 159 / 198 / 284
+    // 256,000 atoms 126 / 154 / 159 / 198 / 284 (before the cells out of reach
+    // were skipped)
     const int64_t rows = end - begin, sms = ctx->numSMs;
     if (rows < 64 * sms) launch(k_build_list<FULL, SPLIT, 8>, 8);
     else if (rows < 640 * sms) launch(k_build_list<FULL, SPLIT, 4>, 4);

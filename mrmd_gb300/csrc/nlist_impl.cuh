@@ -18,6 +18,8 @@ struct CellGrid
     double extent;  // max |coordinate| relative bound used for FP32 error bands
     int reach;      // list builds search cells within +-reach per axis
     float3 mnf, rdxf;  // mn, rdx rounded to FP32 (the binning's FP32 estimate)
+    float3 h;          // cell edges
+    float margin;      // bounds the FP32 rounding of coordinates and cell edges relative to mn
 };
 
 // n = max(1, floor(L * reach / delta)) cells per axis, edge L/n >= delta / reach,
@@ -65,26 +67,51 @@ __device__ __forceinline__ bool lex_above(const double4& pi, const double4& pj)
     return (pj.x > pi.x) || ((pj.x == pi.x) && ((pj.y > pi.y) || ((pj.y == pi.y) && (pj.z > pi.z))));
 }
 
+// The cells of column (ax, ay) that can hold a particle within the list radius
+// of the one at (xi, yi, zi) (relative to mn) in cell (cx, cy, .): [z0, z1] cut
+// to them; false when there is none.  The distance to a column is that to its
+// nearer edge; the outermost cells reach outwards without end, which only adds
+// to the far side.  Of the 125 cells within two cells per axis of a sphere of
+// two cells' radius 84 remain (half list of 256,000 atoms 133 -> 124 us, tile
+// list of 32,000 122 -> 118).
+__device__ __forceinline__ bool trim_column(const CellGrid& g, float xi, float yi, float zi, float reachSq, int cx,
+                                            int cy, int ax, int ay, int& z0, int& z1)
+{
+    const float ex = ax > cx ? (float)ax * g.h.x - xi : xi - (float)(ax + 1) * g.h.x;
+    const float ey = ay > cy ? (float)ay * g.h.y - yi : yi - (float)(ay + 1) * g.h.y;
+    const float dx = ax == cx ? 0.f : fmaxf(ex - g.margin, 0.f), dy = ay == cy ? 0.f : fmaxf(ey - g.margin, 0.f);
+    const float rest = __fmaf_rn(-dx, dx, __fmaf_rn(-dy, dy, reachSq));
+    if (rest < 0.f) return false;
+    float rz;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(rz) : "f"(rest));
+    rz = __fmaf_rn(rz, 1.000001f, g.margin);
+    z0 = max(z0, min(__float2int_rd((zi - rz) * g.rdxf.z - 1e-3f), g.n.z - 1));
+    z1 = min(z1, max(__float2int_rd((zi + rz) * g.rdxf.z + 1e-3f), 0));
+    return true;
+}
+
 // The candidate spans of particle i in cell ci: the columns within g.reach
 // cells per axis (only cell_x >= cell_x(i) for the half list), each column's
-// z range [z0, z1] as one contiguous span [s0, s1) of the cell-sorted
-// particles.  span(ax, ay, c0, z0, z1, s0, s1) is called in scan order
-// (c0: the cell index of (ax, ay, 0)).
+// z range [z0, z1] (trim_column) as one contiguous span [s0, s1) of the
+// cell-sorted particles.  span(ax, ay, c0, z0, z1, s0, s1) is called in scan
+// order (c0: the cell index of (ax, ay, 0)).
 template <bool FULL, class Span>
 __device__ __forceinline__ void for_each_span(const int32_t* __restrict__ cellStart, const CellGrid& g, int32_t ci,
-                                              int64_t nPos, Span&& span)
+                                              float xi, float yi, float zi, float reachSq, int64_t nPos, Span&& span)
 {
     const int cz = ci % g.n.z;
     const int cy = (ci / g.n.z) % g.n.y;
     const int cx = ci / (g.n.z * g.n.y);
     const int R = g.reach;
     const int axEnd = min(cx + R, g.n.x - 1);
-    const int z0 = max(cz - R, 0), z1 = min(cz + R, g.n.z - 1);
+    const int za = max(cz - R, 0), zb = min(cz + R, g.n.z - 1);
     const int ay0 = max(cy - R, 0), ay1 = min(cy + R, g.n.y - 1);
     for (int ax = FULL ? max(cx - R, 0) : cx; ax <= axEnd; ++ax)
     {
         for (int ay = ay0; ay <= ay1; ++ay)
         {
+            int z0 = za, z1 = zb;
+            if (!trim_column(g, xi, yi, zi, reachSq, cx, cy, ax, ay, z0, z1)) continue;
             // cells (ax, ay, z0..z1) are adjacent in the cell order, so their
             // particles form one contiguous span of the sorted arrays
             const int32_t c0 = (ax * g.n.y + ay) * g.n.z;

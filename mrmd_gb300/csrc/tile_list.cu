@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(TILE_ROWS, 4) k_tile_list(
                 chunk_push(an, (uint32_t)slot, nearChunks, row, chN);
         };
         const int zbRow = (ci % g.n.z) >> ZB_BITS;
-        for_each_span<true>(cellStart, g, ci, nPos, [&](int ax, int ay, int32_t, int, int, int32_t s0, int32_t s1) {
+        for_each_span<true>(cellStart, g, ci, xi, yi, zi, rsqHi, nPos, [&](int ax, int ay, int32_t, int, int, int32_t s0, int32_t s1) {
             const int h = col_find(colKey, (ax * g.n.y + ay) * nzb + zbRow);
             if (h < 0) return;  // unreachable: the table holds every entry of the row's stencil
             const int32_t delta = colDelta[h];

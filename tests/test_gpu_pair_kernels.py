@@ -408,3 +408,25 @@ def test_molecule_images_bit_exact(M, orc, n, box, thickness):
     real = gl.correspondingRealAtom(nt)
     np.testing.assert_array_equal(real[na:], corr[na:nt])
     np.testing.assert_array_equal(da["type"][na:], da["type"][real[na:]])
+
+
+# Rows of one lane and of several (97,280 and 9,728 rows on 152 SMs); particles
+# up to 3 beyond the grid (they sit in its outermost cells), a grid far from
+# the origin (FP32 coordinates good to 1e-4 there), one cell on an axis.
+@pytest.mark.parametrize("n,box,origin,out", [(3000, (9.0, 7.0, 6.0), 0.0, 3.0), (3000, (9.0, 7.0, 1.0), 1000.0, 0.0),
+                                              (12000, (22.0, 14.0, 17.0), -37.3, 0.4), (100000, (50.0, 50.0, 50.0), 0.0, 2.0)])
+def test_list_keeps_every_pair_when_cells_are_cut(M, n, box, origin, out):
+    """Cells out of reach of a row are skipped; the list is still every pair
+    within the radius."""
+    spatial = pytest.importorskip("scipy.spatial")
+    box = np.asarray(box)
+    pos = origin + np.random.default_rng(n).uniform(0, 1, (n, 3)) * (box + 2 * out) - out
+    a = M.Atoms.from_arrays(pos)
+    vl = M.HalfVerletList()
+    vl.build(a, 0, n, 1.3, 1.0, [origin] * 3, list(origin + box), 60)
+    counts, nbrs = vl.download()
+    got = np.concatenate([np.stack([np.full(c, i), nbrs[i, :c]], 1) for i, c in enumerate(counts) if c])
+    got = np.unique(np.sort(got, 1), axis=0)
+    assert len(got) == counts.sum()
+    tree = spatial.cKDTree(pos)
+    np.testing.assert_array_equal(got, np.unique(np.sort(tree.query_pairs(1.3, output_type="ndarray"), 1), axis=0))
