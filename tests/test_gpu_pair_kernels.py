@@ -259,7 +259,7 @@ def test_mixed_half_lanes(M, orc, cells, drop, rc, cap, pred, lo):
 # two ghost layers (an atom with images on both sides of an axis).
 @pytest.mark.parametrize("n,box,thickness", [
     (1, (6.0, 6.0, 6.0), 2.8), (1023, (14.0, 11.0, 9.0), 2.8), (1024, (5.0, 9.0, 4.0), 2.8),
-    (1025, (4.0, 4.0, 4.0), 3.5), (5000, (40.0, 3.0, 12.0), 2.8), (263200, (90.0, 60.0, 50.0), 2.8),
+    (1025, (4.0, 4.0, 4.0), 3.5), (5000, (40.0, 3.0, 12.0), 2.8), (263200, (90.0, 60.0, 50.0), 2.8), (320001, (90.0, 60.0, 50.0), 2.8),
     (700, (20.0, 20.0, 20.0), 0.0),
 ])
 def test_ghost_images_bit_exact(M, orc, n, box, thickness):
@@ -371,11 +371,11 @@ def test_density_loss_over_bin_counts(M, bins):
     assert abs(L0 - ((rho - n / (L * area)) ** 2).sum()) <= 1e-11 * (rho ** 2).sum()
 
 
-# Blocks of 256 and of 1,024 molecules (above 152 * 1,024), one to three atoms
+# Blocks of 256 and of 1,024 molecules (above 152 * 2,048), one to three atoms
 # in a molecule, boxes thinner than two ghost layers
 @pytest.mark.parametrize("n,box,thickness", [
     (1, (6.0, 6.0, 6.0), 2.8), (255, (4.0, 9.0, 5.0), 2.8), (257, (14.0, 3.5, 9.0), 2.8), (5000, (40.0, 12.0, 12.0), 2.8),
-    (160000, (90.0, 60.0, 50.0), 2.8), (300, (20.0, 20.0, 20.0), 0.0),
+    (320000, (90.0, 60.0, 50.0), 2.8), (300, (20.0, 20.0, 20.0), 0.0),
 ])
 def test_molecule_images_bit_exact(M, orc, n, box, thickness):
     """Ghost molecules and their atoms, in the oracle's order, bit for bit."""
