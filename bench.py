@@ -515,7 +515,7 @@ def adress_main(args, rank, world, local_rank):
         res[form] = dict(ms=ms, value=n * args.steps / (ms * 1e-3), launches=launches, clocks=clk.summary(),
                          stats=s.stats())
         s.close()
-        # the same system on the batched engine (one replica): four launches per step, 50-step graphs
+        # the same system on the batched engine (one replica): three launches per step, 50-step graphs
         rep = M.Replica(n, [0, 0, 0], list(c["box"]), list(c["center"]), c["at"], 1234)
         b = M.BatchSystem([rep], pos, vel, hybrid_diameter=c["hy"], nu=c["nu"], rc=c["rc"], skin=c["skin"],
                           capping_distance=c["cap"], precision=prec, dt=c["dt"], gamma=c["gamma"],

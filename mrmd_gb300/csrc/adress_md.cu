@@ -16,7 +16,7 @@
 // With unit masses (single-site molecules of the AdResS workload) the same
 // step runs on the batched engine with one replica instead (batch.cu: full
 // list without the pairs of molecules that stay coarse grained, FP32 far
-// pairs in the mixed form, four launches per step in CUDA graphs); the
+// pairs in the mixed form, three launches per step in CUDA graphs); the
 // composed actions above serve other masses.
 #include <cmath>
 #include <vector>
