@@ -351,18 +351,6 @@ __global__ void __launch_bounds__(ADJ_TB, 8) k_adj_force(BDev B, AdjArgs A)
     }
 }
 
-// a = Fbar + h vbar: the adjoint of the step's force (it feeds the post kick
-// v3 = v2 + h F and, through Fbar, the next step's pre kick)
-__global__ void k_adj_prepare(const double4* __restrict__ Fbar, const double4* __restrict__ vbar,
-                              double4* __restrict__ a, int32_t n, double h)
-{
-    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    {
-        const double4 f = Fbar[i], v = vbar[i];
-        a[i] = make_double4(f.x + h * v.x, f.y + h * v.y, f.z + h * v.z, 0.0);
-    }
-}
-
 // FP32 copy of the adjoint for the mixed form's FP32 pair path: (a, a.x m')
 __global__ void k_adj_float(const double4* __restrict__ a, const double4* __restrict__ lam, int32_t n,
                             float4* __restrict__ af)
@@ -755,19 +743,7 @@ int mrmd_diff_backward(mrmd_ctx* ctx, mrmd_diff* d, double* gradTable, double* g
                 builtFor = rb;
             }
             if (rc == MRMD_OK)
-                rc = check_cuda(ctx, cudaMemcpyAsync(b->B.pos, d->x2 + (st - st0) * N, sizeof(double4) * (size_t)N,
-                                                     cudaMemcpyDeviceToDevice, ctx->stream),
-                                "x2");
-            if (rc == MRMD_OK) rc = derive_locals(ctx, b);
-            if (rc == MRMD_OK) rc = update_ghosts(ctx, b);
-            if (rc != MRMD_OK) break;
-            k_adj_prepare<<<g, TB, 0, ctx->stream>>>(d->Fbar, d->vbar, d->adj, N, h);
-            rc = after_launch(ctx, "adj prepare");
-            if (rc == MRMD_OK && mixed)
-            {
-                k_adj_float<<<g, TB, 0, ctx->stream>>>(d->adj, b->B.lam, N, d->adjf);
-                rc = after_launch(ctx, "adj float");
-            }
+                rc = adj_state(ctx, b, AdjState{d->x2 + (st - st0) * N, d->Fbar, d->vbar, d->adj, d->adjf, h});
             if (rc == MRMD_OK)
             {
                 const unsigned ga = (unsigned)div_up((int64_t)N * ADJ_TPR, ADJ_TB);

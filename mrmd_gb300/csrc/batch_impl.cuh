@@ -336,8 +336,18 @@ int rebuild_checked(mrmd_ctx* ctx, mrmd_batch* b, bool sort);
 int step(mrmd_ctx* ctx, mrmd_batch* b, int64_t st, bool checkRebuild);
 // weights (and split coordinates) of the locals at their current positions
 int derive_locals(mrmd_ctx* ctx, mrmd_batch* b);
-// ghost positions and weights from their sources (the ghosts of the last rebuild)
-int update_ghosts(mrmd_ctx* ctx, mrmd_batch* b);
+// One adjoint step's state: positions x, and a = Fbar + h vbar, the adjoint of
+// the step's force (it feeds the post kick v3 = v2 + h F and, through Fbar, the
+// next step's pre kick); af: (a, a.x m') in FP32 (mixed form).
+struct AdjState
+{
+    const double4 *x, *Fbar, *vbar;
+    double4* a;
+    float4* af;
+    double h;
+};
+// the locals at A.x, the ghosts of the last rebuild after them, and the adjoint
+int adj_state(mrmd_ctx* ctx, mrmd_batch* b, const AdjState& A);
 // ghosts, list and the force kernel at the current positions (the kernel's
 // epilogue also applies the post-force kick to the velocities)
 int eval_forces(mrmd_ctx* ctx, mrmd_batch* b);
