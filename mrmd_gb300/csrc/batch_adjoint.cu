@@ -383,23 +383,56 @@ struct LossDev
 {
     double xmin, Lx, binW, invSig2, norm, cutoff;
     int32_t bins;
+    int32_t span;       // bins on each side of a molecule's own within reach
     int32_t copies;     // 1 or 32
     double* rho;        // [bins][copies] sums of kernel values
     double* fold;       // [bins] sums over the copies
+    const double* gauss;  // [span + 1], null: exponentials per bin
     const double* coef; // [bins] dL/d(rho_b) / (window * area)
 };
 
-// Calls f(bin, d) for the bins whose centre lies within the cutoff of x, d the
-// distance to the nearest image of the centre.
+// Calls f(bin, d, e) for the bins whose centre lies within the cutoff of x: d the
+// distance to the nearest image of the centre, e = exp(-d^2 / 2 sigma^2).
+// With bins that each come once, d = d0 - o w for the bin o places from x's own
+// (the nearest image already, so the period, a division per bin, drops out).
+// Few bins, none much wider than sigma (D.gauss != null): then
+//   e = exp(-d0^2 / 2 sigma^2) exp(d0 w / sigma^2)^o gauss[o],
+//   gauss[o] = exp(-(o w)^2 / 2 sigma^2),
+// two exponentials and a reciprocal a molecule instead of one exponential a
+// bin (they bound the kernels on the FP64 pipe), with at most 16 factors
+// multiplied up; the direct form's own argument, up to 18, costs as many bits.
 template <typename F>
 __device__ __forceinline__ void for_bins(const LossDev& D, double x, F f)
 {
-    const int span = (int)ceil(D.cutoff / D.binW) + 1;
+    const int span = D.span;
     const int b0 = (int)floor((x - D.xmin) / D.binW);
-    // bins visited once each: the centre counted from b0 is the nearest image
-    // already, and the period (a division per bin) drops out
     const bool once = 2 * (span + 1) <= D.bins;
     const double d0 = x - (D.xmin + ((double)b0 + 0.5) * D.binW);
+    if (D.gauss)
+    {
+        const double g0 = exp(-0.5 * d0 * d0 * D.invSig2), r = exp(d0 * D.binW * D.invSig2);
+        int mid = b0 % D.bins;
+        if (mid < 0) mid += D.bins;
+        auto side = [&](int from, int dir, double factor) {
+            double p = from ? g0 * factor : g0, o = (double)(dir * from);
+            int b = mid + dir * from;
+            if (b < 0) b += D.bins;
+            if (b >= D.bins) b -= D.bins;
+            for (int k = from; k <= span; ++k)
+            {
+                const double d = fma(-o, D.binW, d0);
+                if (!(fabs(d) > D.cutoff)) f(b, d, p * D.gauss[k]);
+                p *= factor;
+                o += (double)dir;
+                b += dir;
+                if (b < 0) b += D.bins;
+                if (b >= D.bins) b -= D.bins;
+            }
+        };
+        side(0, 1, r);
+        side(1, -1, 1.0 / r);
+        return;
+    }
     double o = -(double)span;
     int b = (b0 - span) % D.bins;
     if (b < 0) b += D.bins;
@@ -413,7 +446,7 @@ __device__ __forceinline__ void for_bins(const LossDev& D, double x, F f)
             d = x - (D.xmin + ((double)b + 0.5) * D.binW);
             d -= D.Lx * rint(d / D.Lx);
         }
-        if (!(fabs(d) > D.cutoff)) f(b, d);
+        if (!(fabs(d) > D.cutoff)) f(b, d, exp(-0.5 * d * d * D.invSig2));
         b = b + 1 == D.bins ? 0 : b + 1;
     }
 }
@@ -421,15 +454,14 @@ __device__ __forceinline__ void for_bins(const LossDev& D, double x, F f)
 // Bound by the atomics while neighbouring molecules, which fall into the same
 // bins, meet at one address (the L2 slice that holds it takes one a clock):
 // with `copies` each lane adds to its own column, and a warp's adds go to
-// consecutive addresses.  65,536 molecules: 136 -> 30 us (and k_loss_grad 47
-// -> 31, which is bound by its exponentials on the FP64 pipe).
+// consecutive addresses.  65,536 molecules: 136 -> 30 us, and 18 with
+// the Gaussians by factors (k_loss_grad 47 -> 31 -> 20).
 __global__ void k_loss_density(BDev B, LossDev D)
 {
     const int copy = threadIdx.x & (D.copies - 1);
     for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < B.N; i += gridDim.x * blockDim.x)
-        for_bins(D, B.pos[i].x, [&](int b, double d) {
-            atomicAdd(D.rho + (int64_t)b * D.copies + copy, D.norm * exp(-0.5 * d * d * D.invSig2));
-        });
+        for_bins(D, B.pos[i].x,
+                 [&](int b, double, double e) { atomicAdd(D.rho + (int64_t)b * D.copies + copy, D.norm * e); });
 }
 
 // the sums of the bins' copies, one warp a bin
@@ -450,7 +482,7 @@ __global__ void k_loss_grad(BDev B, LossDev D, double4* __restrict__ xbar)
     {
         double g = 0.0;
         for_bins(D, B.pos[i].x,
-                 [&](int b, double d) { g = fma(D.coef[b] * -d, exp(-0.5 * d * d * D.invSig2), g); });
+                 [&](int b, double d, double e) { g = fma(D.coef[b] * -d, e, g); });
         xbar[i].x += c * g;
     }
 }
@@ -473,6 +505,7 @@ struct mrmd_diff
     double* tfGrad = nullptr;  // [nBins]
     double* rho = nullptr;     // [lossBins][copies]
     double* fold = nullptr;    // [lossBins]
+    double* gauss = nullptr;   // [span + 1], null: not used
     double* coef = nullptr;    // [lossBins]
     std::vector<double> hRho;
     bool haveForward = false;
@@ -483,6 +516,8 @@ namespace
 // columns of the density: with more bins than that the molecules spread over
 // the bins themselves
 int32_t loss_copies(const mrmd_diff* d) { return d->dc.lossBins <= 4096 ? 32 : 1; }
+
+int32_t loss_span(const LossDev& D) { return (int32_t)std::ceil(D.cutoff / D.binW) + 1; }
 
 LossDev loss_dev(const mrmd_diff* d)
 {
@@ -496,6 +531,8 @@ LossDev loss_dev(const mrmd_diff* d)
     D.cutoff = 6.0 * d->dc.lossSigma;
     D.copies = loss_copies(d);
     D.rho = d->rho;
+    D.span = loss_span(D);
+    D.gauss = d->gauss;
     D.fold = d->fold;
     D.coef = d->coef;
     return D;
@@ -584,6 +621,15 @@ int mrmd_diff_create(mrmd_ctx* ctx, mrmd_diff** out, const mrmd_batch_config* cf
     if (rc == MRMD_OK) rc = grow(ctx, d->rho, 0, dc->lossBins * loss_copies(d));
     if (rc == MRMD_OK) rc = grow(ctx, d->fold, 0, dc->lossBins);
     if (rc == MRMD_OK) rc = grow(ctx, d->coef, 0, dc->lossBins);
+    const LossDev ld = loss_dev(d);
+    const double step2 = ld.binW * ld.binW * ld.invSig2;  // (w / sigma)^2
+    if (rc == MRMD_OK && 2 * (ld.span + 1) <= ld.bins && ld.span <= 16 && step2 <= 6.25)
+    {
+        std::vector<double> gauss((size_t)ld.span + 1);
+        for (int32_t o = 0; o <= ld.span; ++o) gauss[o] = std::exp(-0.5 * (double)o * (double)o * step2);
+        rc = grow(ctx, d->gauss, 0, (int64_t)ld.span + 1);
+        if (rc == MRMD_OK) rc = h2d(ctx, d->gauss, gauss.data(), sizeof(double) * gauss.size());
+    }
     if (rc == MRMD_OK) rc = snapshot(ctx, d->b, d->init, true);
     if (rc == MRMD_OK) rc = check_cuda(ctx, cudaStreamSynchronize(ctx->stream), "diff create");
     if (rc != MRMD_OK)
@@ -602,7 +648,7 @@ int mrmd_diff_destroy(mrmd_ctx* ctx, mrmd_diff* d)
     if (ctx) cudaStreamSynchronize(ctx->stream);
     snap_free(d->init);
     for (auto& s : d->ckpt) snap_free(s);
-    void* ptrs[] = {d->x2, d->xbar, d->vbar, d->Fbar, d->adj, d->adjf, d->grad, d->tfGrad, d->rho, d->fold, d->coef};
+    void* ptrs[] = {d->x2, d->xbar, d->vbar, d->Fbar, d->adj, d->adjf, d->grad, d->tfGrad, d->rho, d->fold, d->gauss, d->coef};
     for (void* p : ptrs) dfree(p);
     if (d->b) mrmd_batch_destroy(ctx, d->b);
     delete d;

@@ -349,8 +349,9 @@ def test_adjoint_rows_over_chunk_edges(M, n, prec):
 
 
 # Bins wider than the kernel's reach allows for one visit each (4, 5), the
-# first count that takes the direct form (6), 32 columns a bin and one (4,097)
-@pytest.mark.parametrize("bins", [4, 5, 6, 33, 4096, 4097])
+# first count that takes the direct form (6), the Gaussian by factors (16: bins of
+# 2.5 sigma, to 100: 16 bins on a side), 32 columns a bin and one (4,097)
+@pytest.mark.parametrize("bins", [4, 5, 6, 15, 16, 17, 33, 100, 107, 4096, 4097])
 def test_density_loss_over_bin_counts(M, bins):
     """The loss of one step's smoothed density against NumPy in FP64 (a sum of
     n terms rounds to under 1e-13 of itself)."""
