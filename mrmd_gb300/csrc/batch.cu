@@ -45,13 +45,12 @@ using namespace mrmd_batch_impl;
 namespace
 {
 // ------------------------------------------------------------------ pre --
-// Ghost g of a molecule at x with derived values `own`: its position, and the
+// Ghost g, shifted by `code`, of a molecule at x with derived values `own`: its position, and the
 // derived values of the axes it is shifted along anew.
 template <bool MIXED>
-__device__ __forceinline__ void ghost_follow(const BDev& B, const RepDev& R, int32_t g, const double4& x,
-                                             const Derived& own)
+__device__ __forceinline__ void ghost_follow(const BDev& B, const RepDev& R, int32_t g, uint32_t code,
+                                             const double4& x, const Derived& own)
 {
-    const uint32_t code = B.gShift[g];
     const int64_t s = (int64_t)B.N + g;
     const double4 p = make_double4(shifted(x.x, code & 3u, R.L[0]), shifted(x.y, (code >> 2) & 3u, R.L[1]),
                                    shifted(x.z, (code >> 4) & 3u, R.L[2]), 0.0);
@@ -120,7 +119,7 @@ __device__ __forceinline__ void pre_body(const BDev& B, int rebuild, int64_t tid
             }
             m2 = fmaxf(m2, __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz))));
             const int32_t gEnd = i + 1 < B.N ? B.gCount[i + 1] : B.sc->numGhost;
-            for (int32_t g = B.gCount[i]; g < gEnd && g < B.gCap; ++g) ghost_follow<MIXED>(B, R, g, x, own);
+            for (int32_t g = B.gCount[i]; g < gEnd && g < B.gCap; ++g) ghost_follow<MIXED>(B, R, g, B.gShift[g], x, own);
             continue;
         }
         {
@@ -295,6 +294,17 @@ __global__ void k_b_ghost_write(BDev B)
         const double4 x = B.pos[i];
         int32_t k = B.gCount[i];  // exclusive offset
         int2 xImg = make_int2(-1, -1);
+        if (!flags)
+        {
+            B.xImg[i] = xImg;
+            continue;
+        }
+        // the ghosts share the molecule's derived values, anew only on the
+        // axes they are shifted along
+        Derived own;
+        derive_x<MIXED>(R, x.x, own);
+        derive_y<MIXED>(R, x.y, own);
+        derive_z<MIXED>(R, x.z, own);
         // options per axis: 0 (no shift), 2 (-L) if x >= maxInner, 1 (+L) if x < minInner
         for (int ox = 0; ox < 3; ++ox)
         {
@@ -315,21 +325,12 @@ __global__ void k_b_ghost_write(BDev B)
                         atomicOr(&B.sc->overflow, FLAG_GHOST_OVERFLOW);
                         continue;
                     }
-                    double4 p = x;
-                    const int c3[3] = {cx, cy, cz};
-#pragma unroll
-                    for (int d = 0; d < 3; ++d)
-                    {
-                        if (c3[d] == 1) set_coord(p, d, __dadd_rn(coord(p, d), R.L[d]));
-                        if (c3[d] == 2) set_coord(p, d, __dsub_rn(coord(p, d), R.L[d]));
-                    }
-                    p.w = 0.0;
                     const int64_t s = (int64_t)B.N + g;
-                    B.pos[s] = p;
+                    const uint32_t code = (uint32_t)(cx | (cy << 2) | (cz << 4));
                     B.slotRep[s] = r;
                     B.gSrc[g] = i;
-                    B.gShift[g] = (uint8_t)(cx | (cy << 2) | (cz << 4));
-                    slot_derived<MIXED>(B, R, s, p);
+                    B.gShift[g] = (uint8_t)code;
+                    ghost_follow<MIXED>(B, R, g, code, x, own);
                     if (!cy && !cz)
                     {
                         if (cx == 2) xImg.x = (int32_t)s;
@@ -356,7 +357,7 @@ __global__ void k_b_adj_state(BDev B, AdjState A)
         B.pos[i] = x;
         const Derived own = slot_derived<MIXED>(B, R, i, x);
         const int32_t gEnd = i + 1 < B.N ? B.gCount[i + 1] : B.sc->numGhost;
-        for (int32_t g = B.gCount[i]; g < gEnd && g < B.gCap; ++g) ghost_follow<MIXED>(B, R, g, x, own);
+        for (int32_t g = B.gCount[i]; g < gEnd && g < B.gCap; ++g) ghost_follow<MIXED>(B, R, g, B.gShift[g], x, own);
         const double4 a = make_double4(f.x + A.h * v.x, f.y + A.h * v.y, f.z + A.h * v.z, 0.0);
         A.a[i] = a;
         if (MIXED) A.af[i] = make_float4((float)a.x, (float)a.y, (float)a.z, (float)(a.x * own.g));
