@@ -97,7 +97,8 @@ __device__ __forceinline__ bool trim_column(const CellGrid& g, float xi, float y
 // order (c0: the cell index of (ax, ay, 0)).
 template <bool FULL, class Span>
 __device__ __forceinline__ void for_each_span(const int32_t* __restrict__ cellStart, const CellGrid& g, int32_t ci,
-                                              float xi, float yi, float zi, float reachSq, int64_t nPos, Span&& span)
+                                              float xi, float yi, float zi, float reachSq, int64_t nPos, Span&& span,
+                                              int part = 0, int parts = 1)
 {
     const int cz = ci % g.n.z;
     const int cy = (ci / g.n.z) % g.n.y;
@@ -106,10 +107,15 @@ __device__ __forceinline__ void for_each_span(const int32_t* __restrict__ cellSt
     const int axEnd = min(cx + R, g.n.x - 1);
     const int za = max(cz - R, 0), zb = min(cz + R, g.n.z - 1);
     const int ay0 = max(cy - R, 0), ay1 = min(cy + R, g.n.y - 1);
-    for (int ax = FULL ? max(cx - R, 0) : cx; ax <= axEnd; ++ax)
+    // part `part` of `parts` runs of the columns in scan order
+    const int axBegin = FULL ? max(cx - R, 0) : cx, wide = ay1 - ay0 + 1, columns = (axEnd - axBegin + 1) * wide;
+    const int first = columns * part / parts, last = columns * (part + 1) / parts;
+    for (int ax = axBegin; ax <= axEnd; ++ax)
     {
         for (int ay = ay0; ay <= ay1; ++ay)
         {
+            const int column = (ax - axBegin) * wide + ay - ay0;
+            if (parts > 1 && (column < first || column >= last)) continue;
             int z0 = za, z1 = zb;
             if (!trim_column(g, xi, yi, zi, reachSq, cx, cy, ax, ay, z0, z1)) continue;
             // cells (ax, ay, z0..z1) are adjacent in the cell order, so their

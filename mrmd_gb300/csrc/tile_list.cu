@@ -36,6 +36,7 @@ namespace
 constexpr int COL_BITS = 9;
 constexpr int COL_HT = 1 << COL_BITS;  // span table slots per tile (a sorted tile uses ~100-200)
 constexpr int ZB_BITS = 4;             // z blocks of 16 cells
+constexpr int SLICE_E = 64;            // entries of a row that one of several threads finds (an LJ fluid: 20-30)
 constexpr int CAND_CAP = 8192;         // candidate positions per tile (a sorted tile has ~2,000-3,500)
 
 __device__ __forceinline__ uint32_t col_hash(int32_t key)
@@ -74,7 +75,8 @@ __device__ __forceinline__ int col_find(const int32_t* keys, int32_t key)
     return -1;
 }
 
-// Exclusive prefix of v over the block (TILE_ROWS threads); *total: the sum.
+// Exclusive prefix of v over the block (THREADS threads); *total: the sum.
+template <int THREADS>
 __device__ __forceinline__ int32_t block_exclusive_scan(int32_t v, int32_t* warpTot, int32_t* total)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -89,17 +91,17 @@ __device__ __forceinline__ int32_t block_exclusive_scan(int32_t v, int32_t* warp
     __syncthreads();
     if (warp == 0)
     {
-        int32_t w = lane < TILE_ROWS / 32 ? warpTot[lane] : 0;
+        int32_t w = lane < THREADS / 32 ? warpTot[lane] : 0;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1)
         {
             const int32_t t = __shfl_up_sync(0xffffffffu, w, o);
             if (lane >= o) w += t;
         }
-        if (lane < TILE_ROWS / 32) warpTot[lane] = w;
+        if (lane < THREADS / 32) warpTot[lane] = w;
     }
     __syncthreads();
-    *total = warpTot[TILE_ROWS / 32 - 1];
+    *total = warpTot[THREADS / 32 - 1];
     const int32_t base = (warp > 0 ? warpTot[warp - 1] : 0) + incl - v;
     __syncthreads();  // warpTot is reused by the next scan
     return base;
@@ -176,7 +178,14 @@ __device__ __forceinline__ void chunk_remap(uint4* __restrict__ out, int64_t row
 // that did not fit (their rows are incomplete), [5] members of all tiles.
 // Four blocks per SM (64 registers): the scan is bound by the latency of its
 // candidate loads; three blocks of 72 registers ran 14% slower.
-__global__ void __launch_bounds__(TILE_ROWS, 4) k_tile_list(
+//
+// H threads share a row, each one run of its stencil's columns in scan order.
+// H = 1 packs the entries in registers.  With few tiles the time is one block's,
+// that is one thread's walk: H = 4 walks a quarter each into a column of shared
+// memory (SLICE_E entries, near ones from below and far ones from above), and
+// the row's chunks are put together at the end.
+template <int H>
+__global__ void __launch_bounds__(TILE_ROWS * H, H == 1 ? 4 : 1) k_tile_list(
     const double4* __restrict__ pos, const int32_t* __restrict__ cellOf, const int32_t* __restrict__ cellStart,
     const float4* __restrict__ spos, CellGrid g, int64_t rows, int64_t nPos, double rsq,
     float rsqLo, float rsqHi, float nearSqF, int64_t capN, int64_t capF, int32_t* __restrict__ countsN,
@@ -186,18 +195,22 @@ __global__ void __launch_bounds__(TILE_ROWS, 4) k_tile_list(
 {
     __shared__ int32_t colKey[COL_HT], colLo[COL_HT], colHi[COL_HT], colDelta[COL_HT];
     __shared__ int32_t used[CAND_CAP];  // candidate position -> particle (-1: unused), then -> member slot
-    __shared__ int32_t warpTot[TILE_ROWS / 32];
-    __shared__ int32_t badS;
+    constexpr int THREADS = TILE_ROWS * H;
+    __shared__ int32_t warpTot[32];
+    __shared__ int32_t badS, longS;  // a table that did not fit, a slice that did not
+    __shared__ uint32_t sliceCount[H == 1 ? 1 : H][TILE_ROWS];  // near entries, far ones << 16
+    extern __shared__ uint16_t sliceBuf[];                      // H > 1: [SLICE_E][THREADS]
     const int tid = threadIdx.x, lane = tid & 31;
+    const int rowInTile = tid % TILE_ROWS, slice = tid / TILE_ROWS;
     const int64_t tile = blockIdx.x;
-    const int64_t row = tile * TILE_ROWS + tid;
-    for (int h = tid; h < COL_HT; h += TILE_ROWS)
+    const int64_t row = tile * TILE_ROWS + rowInTile;
+    for (int h = tid; h < COL_HT; h += THREADS)
     {
         colKey[h] = -1;
         colLo[h] = INT_MAX;
         colHi[h] = -1;
     }
-    if (tid == 0) badS = 0;
+    if (tid == 0) badS = longS = 0;
     __syncthreads();
 
     // ---- span table: one insertion per distinct cell of a warp's rows
@@ -211,7 +224,7 @@ __global__ void __launch_bounds__(TILE_ROWS, 4) k_tile_list(
         const int cz = ci % g.n.z, cy = (ci / g.n.z) % g.n.y, cx = ci / (g.n.z * g.n.y);
         const int R = g.reach;
         const int z0 = max(cz - R, 0), z1 = min(cz + R, g.n.z - 1);
-        for (int ax = max(cx - R, 0); ax <= min(cx + R, g.n.x - 1); ++ax)
+        for (int ax = max(cx - R, 0) + slice; ax <= min(cx + R, g.n.x - 1); ax += H)
             for (int ay = max(cy - R, 0); ay <= min(cy + R, g.n.y - 1); ++ay)
             {
                 const int h = col_insert(colKey, (ax * g.n.y + ay) * nzb + (cz >> ZB_BITS));
@@ -227,14 +240,14 @@ __global__ void __launch_bounds__(TILE_ROWS, 4) k_tile_list(
     __syncthreads();
 
     // ---- candidate positions: the entries' spans numbered one after another
-    constexpr int PER = COL_HT / TILE_ROWS;
+    constexpr int PER = COL_HT > THREADS ? COL_HT / THREADS : 1;
     int32_t cnt[PER], start[PER];
     int32_t local = 0;
 #pragma unroll
     for (int q = 0; q < PER; ++q)
     {
         const int h = tid * PER + q;
-        const int32_t key = colKey[h];
+        const int32_t key = h < COL_HT ? colKey[h] : -1;
         cnt[q] = 0;
         start[q] = 0;
         if (key >= 0)
@@ -250,14 +263,14 @@ __global__ void __launch_bounds__(TILE_ROWS, 4) k_tile_list(
         local += cnt[q];
     }
     int32_t nCand;
-    int32_t base = block_exclusive_scan(local, warpTot, &nCand);
+    int32_t base = block_exclusive_scan<THREADS>(local, warpTot, &nCand);
 #pragma unroll
     for (int q = 0; q < PER; ++q)
     {
-        colDelta[tid * PER + q] = base - start[q];
+        if (tid * PER + q < COL_HT) colDelta[tid * PER + q] = base - start[q];
         base += cnt[q];
     }
-    for (int32_t p = tid; p < nCand && p < CAND_CAP; p += TILE_ROWS) used[p] = -1;
+    for (int32_t p = tid; p < nCand && p < CAND_CAP; p += THREADS) used[p] = -1;
     __syncthreads();
     if (badS || nCand > CAND_CAP)
     {
@@ -266,7 +279,7 @@ __global__ void __launch_bounds__(TILE_ROWS, 4) k_tile_list(
     }
 
     // ---- scan: the rows' neighbours as candidate positions
-    ChunkAcc an, af;
+    ChunkAcc an, af;  // H > 1: only their counts
     if (live)
     {
         const double4 pi = pos[row];
@@ -276,13 +289,21 @@ __global__ void __launch_bounds__(TILE_ROWS, 4) k_tile_list(
             if (!candidate_kept<true>(pos, pi, row, xi, yi, zi, q, rsq, rsqLo, rsqHi, nPos, d2f)) return;
             if ((uint32_t)slot >= (uint32_t)nCand) return;  // unreachable: the span lies in its entry's hull
             used[slot] = __float_as_int(q.w);
-            if (d2f >= nearSqF)
+            if (H > 1)
+            {
+                const bool far = d2f >= nearSqF;
+                if (an.cnt + af.cnt < SLICE_E)
+                    sliceBuf[(far ? SLICE_E - 1 - af.cnt : an.cnt) * THREADS + tid] = (uint16_t)slot;
+                an.cnt += far ? 0 : 1;
+                af.cnt += far ? 1 : 0;
+            }
+            else if (d2f >= nearSqF)
                 chunk_push(af, (uint32_t)slot, farChunks, row, chF);
             else
                 chunk_push(an, (uint32_t)slot, nearChunks, row, chN);
         };
         const int zbRow = (ci % g.n.z) >> ZB_BITS;
-        for_each_span<true>(cellStart, g, ci, xi, yi, zi, rsqHi, nPos, [&](int ax, int ay, int32_t, int, int, int32_t s0, int32_t s1) {
+        auto walk = [&](int ax, int ay, int32_t, int, int, int32_t s0, int32_t s1) {
             const int h = col_find(colKey, (ax * g.n.y + ay) * nzb + zbRow);
             if (h < 0) return;  // unreachable: the table holds every entry of the row's stencil
             const int32_t delta = colDelta[h];
@@ -296,24 +317,48 @@ __global__ void __launch_bounds__(TILE_ROWS, 4) k_tile_list(
                 candidate(q3, s + 3 + delta);
             }
             for (; s < s1; ++s) candidate(spos[s], s + delta);
-        });
-        chunk_flush(an, nearChunks, row, chN);
-        chunk_flush(af, farChunks, row, chF);
+        };
+        for_each_span<true>(cellStart, g, ci, xi, yi, zi, rsqHi, nPos, walk, slice, H);
+        if (H == 1)
+        {
+            chunk_flush(an, nearChunks, row, chN);
+            chunk_flush(af, farChunks, row, chF);
+        }
+    }
+    add_totals((uint32_t)an.cnt, (uint32_t)af.cnt, list_totals(flags));
+    int32_t preN[H] = {0}, preF[H] = {0};  // H > 1: entries of the slices before
+    if (H > 1)
+    {
+        sliceCount[H == 1 ? 0 : slice][rowInTile] = (uint32_t)an.cnt | ((uint32_t)af.cnt << 16);
+        if (an.cnt + af.cnt > SLICE_E) longS = 1;
+        __syncthreads();
+        an.cnt = af.cnt = 0;
+#pragma unroll
+        for (int h = 0; h < H; ++h)
+        {
+            const uint32_t c = sliceCount[H == 1 ? 0 : h][rowInTile];
+            preN[h] = an.cnt;
+            preF[h] = af.cnt;
+            an.cnt += (int32_t)(c & 0xffffu);
+            af.cnt += (int32_t)(c >> 16);
+        }
+    }
+    if (live && slice == 0)
+    {
         countsN[row] = an.cnt < capN ? an.cnt : (int32_t)capN;
         countsF[row] = af.cnt < capF ? af.cnt : (int32_t)capF;
         if (an.cnt > capN) atomicMax(&flags[0], an.cnt);
         if (af.cnt > capF) atomicMax(&flags[1], af.cnt);
     }
-    add_totals((uint32_t)an.cnt, (uint32_t)af.cnt, list_totals(flags));
     __syncthreads();
 
     // ---- members: the used positions in order
-    const int32_t per = (nCand + TILE_ROWS - 1) / TILE_ROWS;
+    const int32_t per = (nCand + THREADS - 1) / THREADS;
     const int32_t p0 = tid * per, p1 = min(p0 + per, nCand);
     local = 0;
     for (int32_t p = p0; p < p1; ++p) local += used[p] >= 0;
     int32_t total;
-    int32_t m = block_exclusive_scan(local, warpTot, &total);
+    int32_t m = block_exclusive_scan<THREADS>(local, warpTot, &total);
     int32_t* mem = members + tile * TILE_CAP;
     for (int32_t p = p0; p < p1; ++p)
     {
@@ -327,14 +372,44 @@ __global__ void __launch_bounds__(TILE_ROWS, 4) k_tile_list(
         memberCount[tile] = total < TILE_CAP ? total : TILE_CAP;
         atomicMax(&flags[3], total);
         atomicAdd(&flags[5], total);
-        if (total > TILE_CAP) atomicAdd(&flags[4], 1);
+        if (total > TILE_CAP || longS) atomicAdd(&flags[4], 1);
     }
     __syncthreads();
-    if (total > TILE_CAP || !live) return;
+    if (total > TILE_CAP || longS || !live) return;
 
     // ---- each row's entries: candidate positions -> member slots
-    chunk_remap(nearChunks, row, chN, an.cnt < capN ? an.cnt : (int32_t)capN, used, nCand);
-    chunk_remap(farChunks, row, chF, af.cnt < capF ? af.cnt : (int32_t)capF, used, nCand);
+    const int32_t cntN = an.cnt < capN ? an.cnt : (int32_t)capN, cntF = af.cnt < capF ? af.cnt : (int32_t)capF;
+    if (H == 1)
+    {
+        chunk_remap(nearChunks, row, chN, cntN, used, nCand);
+        chunk_remap(farChunks, row, chF, cntF, used, nCand);
+        return;
+    }
+    // every H-th chunk a slice's thread
+    auto chunks = [&](uint4* __restrict__ out, int64_t perRow, int32_t cnt, const int32_t (&pre)[H], bool far) {
+        for (int32_t g0 = 8 * slice; g0 < cnt; g0 += 8 * H)
+        {
+            uint32_t v[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+            {
+                const int32_t e = g0 + q;
+                if (e >= cnt) continue;
+                int h = 0;
+#pragma unroll
+                for (int t = 1; t < H; ++t) h += e >= pre[t] ? 1 : 0;
+                int32_t first = 0;
+#pragma unroll
+                for (int t = 1; t < H; ++t) first = h == t ? pre[t] : first;
+                const int32_t k = far ? SLICE_E - 1 - (e - first) : e - first;
+                const uint32_t p = sliceBuf[k * THREADS + h * TILE_ROWS + rowInTile];
+                v[q >> 1] |= ((uint32_t)used[p < CAND_CAP ? p : 0] & 0xffffu) << (16 * (q & 1));
+            }
+            out[chunk_word(row, g0 >> 3, perRow)] = make_uint4(v[0], v[1], v[2], v[3]);
+        }
+    };
+    chunks(nearChunks, chN, cntN, preN, false);
+    chunks(farChunks, chF, cntF, preF, true);
 }
 }  // namespace
 
@@ -346,10 +421,26 @@ int tile_list_launch(mrmd_ctx* ctx, TileList* tl, int64_t rows, int64_t nPos, co
 {
     MRMD_TRY(tile_storage(ctx, tl, rows, nearList->maxNeighbors, farList->maxNeighbors));
     if (rows == 0) return MRMD_OK;
-    k_tile_list<<<(unsigned)tl->tiles, TILE_ROWS, 0, ctx->stream>>>(
-        reinterpret_cast<const double4*>(pos4), cl.cellOf, cl.cellStart, cl.spos, cl.g, rows, nPos, rsq, rsqLo, rsqHi,
-        nearSqF, nearList->maxNeighbors, farList->maxNeighbors, nearList->counts, farList->counts, flags, tl->members,
-        tl->memberCount, tl->nearChunks, tl->nearChunksPerRow, tl->farChunks, tl->farChunksPerRow);
+    // a row's threads: four up to two tiles per SM, unless a slice has
+    // overflowed before.  us per launch with 1 / 4 on 152 SMs: 8 tiles 110 / 43,
+    // 125 tiles 117 / 50, 245 tiles 131 / 94, 308 tiles 143 / 136, 422 tiles
+    // 145 / 144, 1,000 tiles 304 / 357
+    tl->sliced = tl->tiles <= 2 * ctx->numSMs && !tl->longSlices;
+    auto launch = [&](auto kernel, int threads, size_t smem) {
+        kernel<<<(unsigned)tl->tiles, threads, smem, ctx->stream>>>(
+            reinterpret_cast<const double4*>(pos4), cl.cellOf, cl.cellStart, cl.spos, cl.g, rows, nPos, rsq, rsqLo,
+            rsqHi, nearSqF, nearList->maxNeighbors, farList->maxNeighbors, nearList->counts, farList->counts, flags,
+            tl->members, tl->memberCount, tl->nearChunks, tl->nearChunksPerRow, tl->farChunks, tl->farChunksPerRow);
+    };
+    if (tl->sliced)
+    {
+        constexpr int H = 4;
+        constexpr size_t smem = sizeof(uint16_t) * SLICE_E * TILE_ROWS * H;
+        MRMD_CUDA(ctx, cudaFuncSetAttribute(k_tile_list<H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        launch(k_tile_list<H>, TILE_ROWS * H, smem);
+    }
+    else
+        launch(k_tile_list<1>, TILE_ROWS, 0);
     return after_launch(ctx, "tile_list");
 }
 }  // namespace mrmd_impl

@@ -431,3 +431,27 @@ def test_list_keeps_every_pair_when_cells_are_cut(M, n, box, origin, out):
     assert len(got) == counts.sum()
     tree = spatial.cKDTree(pos)
     np.testing.assert_array_equal(got, np.unique(np.sort(tree.query_pairs(1.3, output_type="ndarray"), 1), axis=0))
+
+
+# Tiles of 256 rows with four threads a row up to two tiles per SM (304 on 152
+# SMs, 77,824 rows), one above; a row more than a tile, less than a warp; rows
+# whose quarter of the columns holds more than 64 entries (r_list 4.0: one
+# thread a row from then on).
+@pytest.mark.parametrize("cells,atoms,rc", [(8, 2048, 2.5), (8, 2031, 2.5), (10, 3841, 2.5), (27, 77824, 2.5),
+                                            (27, 77825, 2.5), (10, 4000, 3.7)])
+def test_tile_list_threads_per_row(M, cells, atoms, rc):
+    """The one-pass tile list has the rows, and in them the order, of the one
+    made from the int32 rows: bitwise equal forces after a few rebuilds."""
+    from test_gpu_md import fcc, mb_velocities
+
+    pos, L = fcc(cells)
+    keep = np.sort(np.random.default_rng(atoms).permutation(len(pos))[:atoms])
+    pos, vel = pos[keep], mb_velocities(len(pos), 0.728, 9)[keep]
+    a, b = (M.LJSystem(pos, vel, [0, 0, 0], [L] * 3, rc=rc, precision=M.PREC_MIXED, tile_build=t)
+            for t in ("one_pass", "two_kernel"))
+    a.run(25)
+    b.run(25)
+    assert a.tile_stats()["tiled"] and b.tile_stats()["tiled"]
+    for x, y in zip(a.state(), b.state()):
+        np.testing.assert_array_equal(x, y)
+    np.testing.assert_array_equal(a.pair_keys(), b.pair_keys())
