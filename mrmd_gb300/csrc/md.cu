@@ -762,6 +762,7 @@ const mrmd_nlist* mrmd_md_nlist(const mrmd_md* md) { return md ? &md->list : nul
 
 int mrmd_md_tile_stats(const mrmd_md* md, int64_t* out6)
 {
+const mrmd_ghost_layer* mrmd_md_ghosts(const mrmd_md* md) { return md ? &md->ghosts : nullptr; }
     if (!md || !out6) return MRMD_ERR_ARG;
     const bool mixed = md->cfg.precision == MRMD_PREC_MIXED;
     out6[0] = mixed ? md->tiles.tiles : 0;
