@@ -792,6 +792,9 @@ int mrmd_multires_ghost_create(mrmd_ctx* ctx, mrmd_ghost_layer* g, mrmd_molecule
     MRMD_TRY(ensure_layer(ctx, g, a->capacity > nLocal + 1 ? a->capacity : nLocal + 1, nLocal + 1));
     MRMD_CUDA(ctx, cudaMemsetAsync(g->correspondingRealAtom, 0xff, sizeof(int32_t) * (size_t)g->capacity, ctx->stream));
     if (addM > 0)
+    // molecules, atoms and their places among the images are 32-bit indices
+    if (nMol + addM > INT32_MAX || nLocal + addA > INT32_MAX)
+        return set_error(ctx, MRMD_ERR_CAPACITY, "more than 2^31 molecules or atoms");
     {
         // sources and first atoms of the images behind the counts (which a
         // larger scratch buffer would lose: they are counted again then)
