@@ -569,7 +569,12 @@ int ensure_layer(mrmd_ctx* ctx, mrmd_ghost_layer* g, int64_t capacity, int64_t l
             MRMD_CUDA(ctx, cudaMemcpyAsync(nc, g->correspondingRealAtom, sizeof(int32_t) * (size_t)g->capacity,
                                            cudaMemcpyDeviceToDevice, ctx->stream));
         int32_t* nl = nullptr;
-        MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&nl), sizeof(int32_t) * (size_t)capacity));
+        if (const int rc = dmalloc(ctx, reinterpret_cast<void**>(&nl), sizeof(int32_t) * (size_t)capacity))
+        {
+            cudaStreamSynchronize(ctx->stream);
+            dfree(nc);
+            return rc;
+        }
         MRMD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         dfree(g->correspondingRealAtom);
         dfree(g->ghostList);
@@ -581,6 +586,7 @@ int ensure_layer(mrmd_ctx* ctx, mrmd_ghost_layer* g, int64_t capacity, int64_t l
     {
         dfree(g->ghostStart);
         g->ghostStart = nullptr;
+        g->localCapacity = g->numLocal = g->numGhost = 0;
         MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&g->ghostStart), sizeof(int32_t) * (size_t)(localCapacity + 1)));
         g->localCapacity = localCapacity;
     }
@@ -786,15 +792,15 @@ int mrmd_multires_ghost_create(mrmd_ctx* ctx, mrmd_ghost_layer* g, mrmd_molecule
     MRMD_CUDA(ctx, cudaMemcpyAsync(h, mem, head, cudaMemcpyDeviceToHost, ctx->stream));
     MRMD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     const int64_t addM = h[KINDS], addA = h[2 * KINDS + 1];
+    // molecules, atoms and their places among the images are 32-bit indices
+    if (nMol + addM > INT32_MAX || nLocal + addA > INT32_MAX)
+        return set_error(ctx, MRMD_ERR_CAPACITY, "more than 2^31 molecules or atoms");
     if (nMol + addM > m->capacity) MRMD_TRY(mrmd_molecules_reserve(ctx, m, nMol + addM + (nMol + addM) / 8 + 64));
     if (nLocal + addA > a->capacity)
         MRMD_TRY(mrmd_atoms_reserve(ctx, a, nLocal + addA + (nLocal + addA) / 8 + 64));
     MRMD_TRY(ensure_layer(ctx, g, a->capacity > nLocal + 1 ? a->capacity : nLocal + 1, nLocal + 1));
     MRMD_CUDA(ctx, cudaMemsetAsync(g->correspondingRealAtom, 0xff, sizeof(int32_t) * (size_t)g->capacity, ctx->stream));
     if (addM > 0)
-    // molecules, atoms and their places among the images are 32-bit indices
-    if (nMol + addM > INT32_MAX || nLocal + addA > INT32_MAX)
-        return set_error(ctx, MRMD_ERR_CAPACITY, "more than 2^31 molecules or atoms");
     {
         // sources and first atoms of the images behind the counts (which a
         // larger scratch buffer would lose: they are counted again then)

@@ -320,6 +320,7 @@ int CellList::build(mrmd_ctx* ctx, const double* pos4, int64_t n, const CellGrid
         dfree(sorted);
         dfree(spos);
         dfree(unordered);
+        capN = 0;  // until all four are there
         cellOf = sorted = unordered = nullptr;
         spos = nullptr;
         const int64_t c = n + n / 4 + 64;
@@ -332,6 +333,7 @@ int CellList::build(mrmd_ctx* ctx, const double* pos4, int64_t n, const CellGrid
     if (nkeys + 1 > capCells)
     {
         // one allocation: cell starts, then the scatter's cursors
+        capCells = 0;
         dfree(cellStart);
         cellStart = nullptr;
         const int64_t c = nkeys + 1;
@@ -371,6 +373,7 @@ void CellList::release()
     cellOf = sorted = unordered = cellStart = nullptr;
     spos = nullptr;
     capN = capCells = 0;
+// (A failed allocation leaves an empty list: no rows, no capacity.)
 }
 
 static int ensure_list_storage(mrmd_ctx* ctx, mrmd_nlist* nl, int64_t rows, int64_t maxNeighbors)
@@ -378,6 +381,7 @@ static int ensure_list_storage(mrmd_ctx* ctx, mrmd_nlist* nl, int64_t rows, int6
     const int64_t stride = div_up(rows > 0 ? rows : 1, 32) * 32;
     if (rows + 1 > nl->rowsCapacity)
     {
+        nl->rows = nl->rowsCapacity = nl->totalPairs = 0;
         dfree(nl->counts);
         nl->counts = nullptr;
         const int64_t c = rows + rows / 8 + 64;
@@ -387,6 +391,7 @@ static int ensure_list_storage(mrmd_ctx* ctx, mrmd_nlist* nl, int64_t rows, int6
     const int64_t need = stride * maxNeighbors;
     if (need > nl->nbrsCapacity)
     {
+        nl->rows = nl->nbrsCapacity = nl->totalPairs = 0;
         dfree(nl->nbrs);
         nl->nbrs = nullptr;
         MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&nl->nbrs), sizeof(int32_t) * (size_t)need));
