@@ -542,7 +542,6 @@ __global__ void __launch_bounds__(IMG_TB) k_image_molecules(mrmd_molecules m, mr
     const int64_t g = blockIdx.x * (int64_t)IMG_TB + threadIdx.x;
     if (g >= nGhost || !MRMD_IN_BOUNDS(nMol + g, m.capacity)) return;
     const int64_t src = source[g];
-    if (!MRMD_IN_BOUNDS(src, nMol)) return;
     const uint32_t kf = flags_of_image<true>(first, g);
     const int64_t s = m.atomsOffset[src], size = m.numAtoms[src], dst = nAtoms + atom0[g];
     copy_molecule(m, nMol + g, src);
@@ -552,7 +551,7 @@ __global__ void __launch_bounds__(IMG_TB) k_image_molecules(mrmd_molecules m, mr
     pos = reinterpret_cast<double4*>(a.pos);
     for (int64_t k = 0; k < size; ++k)
     {
-        if (!MRMD_IN_BOUNDS(dst + k, a.capacity) || !MRMD_IN_BOUNDS(s + k, nAtoms)) break;
+        if (!MRMD_IN_BOUNDS(dst + k, a.capacity)) break;
         copy_atom(a, dst + k, s + k);
         pos[dst + k] = image_position(pos[s + k], kf, box);
         corr[dst + k] = (int32_t)(s + k);
@@ -569,12 +568,7 @@ int ensure_layer(mrmd_ctx* ctx, mrmd_ghost_layer* g, int64_t capacity, int64_t l
             MRMD_CUDA(ctx, cudaMemcpyAsync(nc, g->correspondingRealAtom, sizeof(int32_t) * (size_t)g->capacity,
                                            cudaMemcpyDeviceToDevice, ctx->stream));
         int32_t* nl = nullptr;
-        if (const int rc = dmalloc(ctx, reinterpret_cast<void**>(&nl), sizeof(int32_t) * (size_t)capacity))
-        {
-            cudaStreamSynchronize(ctx->stream);
-            dfree(nc);
-            return rc;
-        }
+        MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&nl), sizeof(int32_t) * (size_t)capacity));
         MRMD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         dfree(g->correspondingRealAtom);
         dfree(g->ghostList);
@@ -586,7 +580,6 @@ int ensure_layer(mrmd_ctx* ctx, mrmd_ghost_layer* g, int64_t capacity, int64_t l
     {
         dfree(g->ghostStart);
         g->ghostStart = nullptr;
-        g->localCapacity = g->numLocal = g->numGhost = 0;
         MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&g->ghostStart), sizeof(int32_t) * (size_t)(localCapacity + 1)));
         g->localCapacity = localCapacity;
     }
@@ -792,9 +785,6 @@ int mrmd_multires_ghost_create(mrmd_ctx* ctx, mrmd_ghost_layer* g, mrmd_molecule
     MRMD_CUDA(ctx, cudaMemcpyAsync(h, mem, head, cudaMemcpyDeviceToHost, ctx->stream));
     MRMD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     const int64_t addM = h[KINDS], addA = h[2 * KINDS + 1];
-    // molecules, atoms and their places among the images are 32-bit indices
-    if (nMol + addM > INT32_MAX || nLocal + addA > INT32_MAX)
-        return set_error(ctx, MRMD_ERR_CAPACITY, "more than 2^31 molecules or atoms");
     if (nMol + addM > m->capacity) MRMD_TRY(mrmd_molecules_reserve(ctx, m, nMol + addM + (nMol + addM) / 8 + 64));
     if (nLocal + addA > a->capacity)
         MRMD_TRY(mrmd_atoms_reserve(ctx, a, nLocal + addA + (nLocal + addA) / 8 + 64));

@@ -243,7 +243,6 @@ int kick_factors(mrmd_ctx* ctx, mrmd_md* md)
 int md_rebuild(mrmd_ctx* ctx, mrmd_md* md)
 {
     mrmd_atoms* a = &md->atoms;
-    md->needRebuild = true;  // until it is through
     MRMD_TRY(mrmd_ghost_exchange_real_atoms(ctx, a, &md->sd));
     if (md->cfg.sortAtoms > 0 && md->rebuilds % md->cfg.sortAtoms == 0)
     {
@@ -289,7 +288,6 @@ int md_rebuild(mrmd_ctx* ctx, mrmd_md* md)
     {
         dfree(md->rec);
         md->rec = nullptr;
-        md->splitCap = 0;
         const int64_t c = nAll + nAll / 8 + 64;
         MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&md->rec), 2 * sizeof(float4) * (size_t)c));
         md->splitCap = c;
@@ -375,17 +373,16 @@ int ensure_energy(mrmd_ctx* ctx, mrmd_md* md, int64_t nsteps)
     if (md->hEnergy) cudaFreeHost(md->hEnergy);
     md->dEnergy = nullptr;
     md->hEnergy = nullptr;
-    md->energyCap = 0;
+    const int64_t c = nsteps + 64;
+    MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&md->dEnergy), sizeof(double) * REC * (size_t)c));
+    MRMD_CUDA(ctx, cudaMallocHost(reinterpret_cast<void**>(&md->hEnergy), sizeof(double) * REC * (size_t)c));
+    md->energyCap = c;
     // any captured graph referenced the old buffer
     if (md->exec)
     {
         cudaGraphExecDestroy(md->exec);
         md->exec = nullptr;
     }
-    const int64_t c = nsteps + 64;
-    MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&md->dEnergy), sizeof(double) * REC * (size_t)c));
-    MRMD_CUDA(ctx, cudaMallocHost(reinterpret_cast<void**>(&md->hEnergy), sizeof(double) * REC * (size_t)c));
-    md->energyCap = c;
     return MRMD_OK;
 }
 
@@ -571,7 +568,7 @@ int md_run(mrmd_ctx* ctx, mrmd_md* md, int64_t nsteps, double* out, int cols)
         rc = md_rebuild(ctx, md);
         if (rc == MRMD_OK) rc = mrmd_atoms_set_force(ctx, a, a->numLocal + a->numGhost, 0.0);
         if (rc == MRMD_OK) rc = md_forces(ctx, md, rec + REC * nsteps);  // scratch slot
-        md->forceValid = rc == MRMD_OK;
+        md->forceValid = true;
     }
     // the previous step's record, for the kinetic energy its post-kick yields;
     // none for the first step of a run (the last run's end recorded it)
@@ -762,7 +759,6 @@ int mrmd_md_eval(mrmd_ctx* ctx, mrmd_md* md, int what, double* ev2)
 
 const mrmd_atoms* mrmd_md_atoms(const mrmd_md* md) { return md ? &md->atoms : nullptr; }
 const mrmd_nlist* mrmd_md_nlist(const mrmd_md* md) { return md ? &md->list : nullptr; }
-const mrmd_ghost_layer* mrmd_md_ghosts(const mrmd_md* md) { return md ? &md->ghosts : nullptr; }
 
 int mrmd_md_tile_stats(const mrmd_md* md, int64_t* out6)
 {
