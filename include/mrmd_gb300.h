@@ -504,10 +504,11 @@ int mrmd_md_stats(const mrmd_md* md, int64_t* out5);
  * what = 1: launch only the pair-force kernel on the current list and split
  * coordinates, asynchronously (for timing the kernel alone). */
 int mrmd_md_eval(mrmd_ctx* ctx, mrmd_md* md, int what, double* ev2);
-/* Access to the internal atoms / list for profiling and tests (the mixed
+/* Access to the internal atoms / list / ghosts for profiling and tests (the mixed
  * form's list is split by distance; this is its near part). */
 const mrmd_atoms* mrmd_md_atoms(const mrmd_md* md);
 const mrmd_nlist* mrmd_md_nlist(const mrmd_md* md);
+const mrmd_ghost_layer* mrmd_md_ghosts(const mrmd_md* md);
 /* Mixed form's tile list: [0] tiles, [1] members of the largest tile,
  * [2] 1 when the pair kernel reads shared-memory tiles, 0 when it gathers
  * through the int32 lists (a tile over capacity, or gatherNeighbours),

@@ -542,6 +542,7 @@ __global__ void __launch_bounds__(IMG_TB) k_image_molecules(mrmd_molecules m, mr
     const int64_t g = blockIdx.x * (int64_t)IMG_TB + threadIdx.x;
     if (g >= nGhost || !MRMD_IN_BOUNDS(nMol + g, m.capacity)) return;
     const int64_t src = source[g];
+    if (!MRMD_IN_BOUNDS(src, nMol)) return;
     const uint32_t kf = flags_of_image<true>(first, g);
     const int64_t s = m.atomsOffset[src], size = m.numAtoms[src], dst = nAtoms + atom0[g];
     copy_molecule(m, nMol + g, src);
@@ -551,7 +552,7 @@ __global__ void __launch_bounds__(IMG_TB) k_image_molecules(mrmd_molecules m, mr
     pos = reinterpret_cast<double4*>(a.pos);
     for (int64_t k = 0; k < size; ++k)
     {
-        if (!MRMD_IN_BOUNDS(dst + k, a.capacity)) break;
+        if (!MRMD_IN_BOUNDS(dst + k, a.capacity) || !MRMD_IN_BOUNDS(s + k, nAtoms)) break;
         copy_atom(a, dst + k, s + k);
         pos[dst + k] = image_position(pos[s + k], kf, box);
         corr[dst + k] = (int32_t)(s + k);

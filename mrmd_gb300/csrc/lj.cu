@@ -252,7 +252,9 @@ __global__ void __launch_bounds__(LJ_TB, LJ_BLOCKS) k_lj_fp64(
                     fx -= gx;
                     fy -= gy;
                     fz -= gz;
-                    double* fj = force + 4 * (realOf && j >= nLocal ? (int64_t)realOf[j] : j);
+                    const int64_t to = realOf && j >= nLocal ? (int64_t)realOf[j] : j;
+                    if (!MRMD_IN_BOUNDS(to, realOf ? nLocal : nAll)) continue;
+                    double* fj = force + 4 * to;
                     atomicAdd(fj + 0, gx);
                     atomicAdd(fj + 1, gy);
                     atomicAdd(fj + 2, gz);

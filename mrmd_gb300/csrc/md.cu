@@ -759,6 +759,7 @@ int mrmd_md_eval(mrmd_ctx* ctx, mrmd_md* md, int what, double* ev2)
 
 const mrmd_atoms* mrmd_md_atoms(const mrmd_md* md) { return md ? &md->atoms : nullptr; }
 const mrmd_nlist* mrmd_md_nlist(const mrmd_md* md) { return md ? &md->list : nullptr; }
+const mrmd_ghost_layer* mrmd_md_ghosts(const mrmd_md* md) { return md ? &md->ghosts : nullptr; }
 
 int mrmd_md_tile_stats(const mrmd_md* md, int64_t* out6)
 {

@@ -1,0 +1,89 @@
+"""Calls at the limits of indices and buffers: refused with an error, or
+reported by the bounds-checked build, and the objects stay usable."""
+import os
+import subprocess
+import sys
+import textwrap
+
+import numpy as np
+import pytest
+
+from conftest import ROOT
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def M():
+    import mrmd_gb300 as m
+
+    return m
+
+
+# Runs with the bounds-checked library alone, where an index outside its array
+# is recorded and the access is skipped.
+CHILD = textwrap.dedent(r"""
+    import ctypes, sys
+    import numpy as np
+    sys.path.insert(0, ROOT)
+    sys.path.insert(0, ROOT + "/tests")
+    import mrmd_gb300 as M
+    from test_gpu_md import fcc, mb_velocities
+    ctx = M.default_context()
+    if ctx.lib.mrmd_bounds_checked() != 1:
+        print("not the bounds-checked library")
+        sys.exit(3)
+    cudart = None
+    for name in ("libcudart.so.13", "libcudart.so.12", "libcudart.so"):
+        try:
+            cudart = ctypes.CDLL(name)
+            break
+        except OSError:
+            pass
+    clean = M.Atoms.from_arrays(np.ones((4, 3)), capacity=64)
+
+    def reported(f, source, value):
+        try:
+            f()
+            clean.setForce(0.0)  # the next synchronisation
+        except M.MrmdError as e:
+            assert e.code == -9 and source in str(e) and str(value) in str(e), e
+            print("reported:", e)
+        else:
+            print("no violation reported for", source)
+            sys.exit(4)
+
+    # the FP64 stepper's real atoms of its ghosts, from the host
+    pos, L = fcc(6)
+    s = M.LJSystem(pos, mb_velocities(len(pos), 0.728, 3), [0, 0, 0], [L] * 3, precision=M.PREC_FP64)
+    s.run(5)
+    g = ctx.lib.mrmd_md_ghosts(s.h).contents
+    real = ctypes.c_void_p(ctypes.cast(g.correspondingRealAtom, ctypes.c_void_p).value + 4 * g.numLocal)
+    for bad in (1 << 30, -1):
+        entries = np.full(g.numGhost, bad, dtype=np.int32)
+        assert cudart.cudaMemcpy(real, entries.ctypes.data_as(ctypes.c_void_p), ctypes.c_size_t(4 * g.numGhost), 1) == 0
+        reported(s.launch_pair_kernel, "lj.cu", bad)
+    s.close()
+    # a molecule whose atoms are not there
+    a = M.Atoms.from_arrays([[0.5, 5.0, 5.0], [5.0, 5.0, 5.0]], capacity=64)
+    m = M.Molecules(16)
+    up = dict(pos=np.array([[0.5, 5.0, 5.0], [5.0, 5.0, 5.0]]), force=np.zeros((2, 3)), lambda_=np.zeros(2),
+              modulated_lambda=np.zeros(2), grad_lambda=np.zeros((2, 3)), num_atoms=[1, 1])
+    box, gl = M.Subdomain([0, 0, 0], [10.0] * 3, 2.8), M.MultiResGhostLayer()
+    m.upload(2, 0, atoms_offset=[1 << 30, 1], **up)
+    reported(lambda: gl.createGhostAtoms(m, a, box), "ghost.cu", 1 << 30)
+    m.upload(2, 0, atoms_offset=[0, 1], **up)
+    gl.createGhostAtoms(m, a, box)
+    print("ok")
+""")
+
+
+def test_bounds_build_reports_bad_real_atoms_and_molecules():
+    from mrmd_gb300 import build as B
+
+    B.build(bounds_check=True)
+    env = dict(os.environ, MRMD_GB300_BOUNDS_CHECK="1")
+    r = subprocess.run([sys.executable, "-c", f"ROOT = {ROOT!r}\n" + CHILD], env=env, capture_output=True,
+                       text=True, timeout=600)
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert r.stdout.count("reported: MRMD_ERR_BOUNDS") == 3 and r.stdout.strip().endswith("ok"), r.stdout
