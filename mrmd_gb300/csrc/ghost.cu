@@ -786,6 +786,9 @@ int mrmd_multires_ghost_create(mrmd_ctx* ctx, mrmd_ghost_layer* g, mrmd_molecule
     MRMD_CUDA(ctx, cudaMemcpyAsync(h, mem, head, cudaMemcpyDeviceToHost, ctx->stream));
     MRMD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     const int64_t addM = h[KINDS], addA = h[2 * KINDS + 1];
+    // molecules, atoms and their places among the images are 32-bit indices
+    if (nMol + addM > INT32_MAX || nLocal + addA > INT32_MAX)
+        return set_error(ctx, MRMD_ERR_CAPACITY, "more than 2^31 molecules or atoms");
     if (nMol + addM > m->capacity) MRMD_TRY(mrmd_molecules_reserve(ctx, m, nMol + addM + (nMol + addM) / 8 + 64));
     if (nLocal + addA > a->capacity)
         MRMD_TRY(mrmd_atoms_reserve(ctx, a, nLocal + addA + (nLocal + addA) / 8 + 64));

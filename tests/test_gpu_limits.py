@@ -20,6 +20,25 @@ def M():
     return m
 
 
+def test_molecule_images_beyond_31_bits_are_refused(M):
+    """A molecule in a corner has seven images; 7 x 2^29 atoms have no 32-bit
+    index.  Refused before anything is reserved or written."""
+    box = M.Subdomain([0, 0, 0], [10.0] * 3, 2.8)
+    a = M.Atoms.from_arrays([[0.5, 0.5, 0.5]], capacity=64)
+    m = M.Molecules(16)
+    up = dict(pos=np.array([[0.5, 0.5, 0.5]]), force=np.zeros((1, 3)), lambda_=np.zeros(1),
+              modulated_lambda=np.zeros(1), grad_lambda=np.zeros((1, 3)), atoms_offset=[0])
+    m.upload(1, 0, num_atoms=[1 << 29], **up)
+    gl = M.MultiResGhostLayer()
+    with pytest.raises(M.MrmdError) as e:
+        gl.createGhostAtoms(m, a, box)
+    assert e.value.code == -8  # MRMD_ERR_CAPACITY
+    assert (m.numGhostMolecules, a.numGhostAtoms) == (0, 0)
+    m.upload(1, 0, num_atoms=[1], **up)
+    gl.createGhostAtoms(m, a, box)
+    assert (m.numGhostMolecules, a.numGhostAtoms) == (7, 7)
+
+
 # Runs with the bounds-checked library alone, where an index outside its array
 # is recorded and the access is skipped.
 CHILD = textwrap.dedent(r"""
