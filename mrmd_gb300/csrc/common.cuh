@@ -55,7 +55,6 @@ void dfree(void* p);
 // not be ordered with its kernels).
 int h2d(mrmd_ctx* ctx, void* dst, const void* src, size_t bytes);
 int d2h(mrmd_ctx* ctx, void* dst, const void* src, size_t bytes);
-void touch_pages(void* dst, size_t bytes);
 int dzero(mrmd_ctx* ctx, void* p, size_t bytes);
 
 inline int64_t div_up(int64_t a, int64_t b) { return (a + b - 1) / b; }

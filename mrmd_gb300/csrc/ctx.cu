@@ -1,11 +1,10 @@
 // Context, error reporting, scratch memory and exclusive scans.
-#include <unistd.h>
-
 #include <cstdarg>
 #include <cstring>
 #include <vector>
 
 #include "common.cuh"
+#include "host_pages.cuh"
 
 namespace mrmd_impl
 {
@@ -111,20 +110,10 @@ int h2d(mrmd_ctx* ctx, void* dst, const void* src, size_t bytes)
     return check_cuda(ctx, cudaStreamSynchronize(ctx->stream), "h2d");
 }
 
-// Fresh host pages are faulted in here, by the host: left to the copy, the
-// GPU faults them one by one (3 x 25 MB into new arrays 54 ms, 0.5 ms into
-// pages that exist).  The bytes written are overwritten by the copy.
-void touch_pages(void* dst, size_t bytes)
-{
-    static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-    volatile char* p = static_cast<volatile char*>(dst);
-    for (size_t b = 0; b < bytes; b += page) p[b] = 0;
-}
-
 int d2h(mrmd_ctx* ctx, void* dst, const void* src, size_t bytes)
 {
     if (bytes == 0) return MRMD_OK;
-    touch_pages(dst, bytes);
+    populate_pages(dst, bytes);
     MRMD_CUDA(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
     return check_cuda(ctx, cudaStreamSynchronize(ctx->stream), "d2h");
 }
