@@ -61,6 +61,7 @@ int ad_rebuild(mrmd_ctx* ctx, mrmd_adress* s)
 {
     mrmd_atoms* a = &s->atoms;
     mrmd_molecules* m = &s->mol;
+    s->needRebuild = true;  // until it is through
     a->numGhost = 0;
     m->numGhost = 0;
     MRMD_TRY(mrmd_update_molecules(ctx, m, a, &s->slab));
@@ -76,6 +77,7 @@ int ad_rebuild(mrmd_ctx* ctx, mrmd_adress* s)
         cudaStreamSynchronize(ctx->stream);
         dfree(s->split);
         s->split = nullptr;
+        s->splitCap = 0;
         const int64_t c = nA + nA / 8 + 64;
         MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&s->split), sizeof(float4) * 2 * (size_t)c));
         s->splitCap = c;
@@ -342,6 +344,7 @@ int mrmd_adress_run(mrmd_ctx* ctx, mrmd_adress* s, int64_t nsteps, double* energ
         cudaStreamSynchronize(ctx->stream);
         dfree(s->dEnergy);
         s->dEnergy = nullptr;
+        s->energyCap = 0;
         ad_drop_graph(s);  // graphs reference the old buffer
         MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&s->dEnergy), sizeof(double) * (size_t)(nsteps + 64)));
         s->energyCap = nsteps + 64;

@@ -2012,15 +2012,16 @@ int ensure_ring(mrmd_ctx* ctx, mrmd_batch* b)
     const int32_t need = (int32_t)std::max<int64_t>(b->cfg.tuning.graphSteps, 64);
     if (need <= b->B.ring) return MRMD_OK;
     MRMD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    drop_graph(b);
     dfree(b->B.energyRing);
     b->B.energyRing = nullptr;
+    b->B.ring = 0;
     if (b->hRing) cudaFreeHost(b->hRing);
     b->hRing = nullptr;
     MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&b->B.energyRing), sizeof(double) * (size_t)need * b->R));
     MRMD_TRY(dzero(ctx, b->B.energyRing, sizeof(double) * (size_t)need * b->R));
     MRMD_CUDA(ctx, cudaMallocHost(reinterpret_cast<void**>(&b->hRing), sizeof(double) * (size_t)need * b->R));
     b->B.ring = need;
-    drop_graph(b);
     return MRMD_OK;
 }
 
@@ -2363,6 +2364,7 @@ int mrmd_batch_destroy(mrmd_ctx* ctx, mrmd_batch* b)
 int mrmd_batch_run(mrmd_ctx* ctx, mrmd_batch* b, int64_t nsteps, double* energies)
 {
     if (!ctx || !b || nsteps < 0) return MRMD_ERR_ARG;
+    MRMD_TRY(ensure_ring(ctx, b));  // gone when it could not grow
     const int oldSync = ctx->sync;
     ctx->sync = 0;
     const int64_t P = b->cfg.tuning.graphSteps;

@@ -569,7 +569,12 @@ int ensure_layer(mrmd_ctx* ctx, mrmd_ghost_layer* g, int64_t capacity, int64_t l
             MRMD_CUDA(ctx, cudaMemcpyAsync(nc, g->correspondingRealAtom, sizeof(int32_t) * (size_t)g->capacity,
                                            cudaMemcpyDeviceToDevice, ctx->stream));
         int32_t* nl = nullptr;
-        MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&nl), sizeof(int32_t) * (size_t)capacity));
+        if (const int rc = dmalloc(ctx, reinterpret_cast<void**>(&nl), sizeof(int32_t) * (size_t)capacity))
+        {
+            cudaStreamSynchronize(ctx->stream);
+            dfree(nc);
+            return rc;
+        }
         MRMD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         dfree(g->correspondingRealAtom);
         dfree(g->ghostList);
@@ -581,6 +586,7 @@ int ensure_layer(mrmd_ctx* ctx, mrmd_ghost_layer* g, int64_t capacity, int64_t l
     {
         dfree(g->ghostStart);
         g->ghostStart = nullptr;
+        g->localCapacity = g->numLocal = g->numGhost = 0;
         MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&g->ghostStart), sizeof(int32_t) * (size_t)(localCapacity + 1)));
         g->localCapacity = localCapacity;
     }

@@ -639,6 +639,7 @@ int tile_storage(mrmd_ctx* ctx, TileList* tl, int64_t rows, int64_t capN, int64_
         dfree(tl->members);
         dfree(tl->memberCount);
         tl->members = tl->memberCount = nullptr;
+        tl->tilesCap = 0;
         const int64_t c = tl->tiles + tl->tiles / 8 + 4;
         MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&tl->members), sizeof(int32_t) * (size_t)c * TILE_CAP));
         MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&tl->memberCount), sizeof(int32_t) * (size_t)c));
@@ -651,6 +652,7 @@ int tile_storage(mrmd_ctx* ctx, TileList* tl, int64_t rows, int64_t capN, int64_
     {
         dfree(tl->nearChunks);
         tl->nearChunks = nullptr;
+        tl->nearWords = 0;
         const int64_t w = rows32 * tl->nearChunksPerRow + rows32 * tl->nearChunksPerRow / 8;
         MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&tl->nearChunks), sizeof(uint4) * (size_t)w));
         tl->nearWords = w;
@@ -659,6 +661,7 @@ int tile_storage(mrmd_ctx* ctx, TileList* tl, int64_t rows, int64_t capN, int64_
     {
         dfree(tl->farChunks);
         tl->farChunks = nullptr;
+        tl->farWords = 0;
         const int64_t w = rows32 * tl->farChunksPerRow + rows32 * tl->farChunksPerRow / 8;
         MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&tl->farChunks), sizeof(uint4) * (size_t)w));
         tl->farWords = w;

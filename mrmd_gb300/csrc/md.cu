@@ -243,6 +243,7 @@ int kick_factors(mrmd_ctx* ctx, mrmd_md* md)
 int md_rebuild(mrmd_ctx* ctx, mrmd_md* md)
 {
     mrmd_atoms* a = &md->atoms;
+    md->needRebuild = true;  // until it is through
     MRMD_TRY(mrmd_ghost_exchange_real_atoms(ctx, a, &md->sd));
     if (md->cfg.sortAtoms > 0 && md->rebuilds % md->cfg.sortAtoms == 0)
     {
@@ -288,6 +289,7 @@ int md_rebuild(mrmd_ctx* ctx, mrmd_md* md)
     {
         dfree(md->rec);
         md->rec = nullptr;
+        md->splitCap = 0;
         const int64_t c = nAll + nAll / 8 + 64;
         MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&md->rec), 2 * sizeof(float4) * (size_t)c));
         md->splitCap = c;
@@ -373,16 +375,17 @@ int ensure_energy(mrmd_ctx* ctx, mrmd_md* md, int64_t nsteps)
     if (md->hEnergy) cudaFreeHost(md->hEnergy);
     md->dEnergy = nullptr;
     md->hEnergy = nullptr;
-    const int64_t c = nsteps + 64;
-    MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&md->dEnergy), sizeof(double) * REC * (size_t)c));
-    MRMD_CUDA(ctx, cudaMallocHost(reinterpret_cast<void**>(&md->hEnergy), sizeof(double) * REC * (size_t)c));
-    md->energyCap = c;
+    md->energyCap = 0;
     // any captured graph referenced the old buffer
     if (md->exec)
     {
         cudaGraphExecDestroy(md->exec);
         md->exec = nullptr;
     }
+    const int64_t c = nsteps + 64;
+    MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&md->dEnergy), sizeof(double) * REC * (size_t)c));
+    MRMD_CUDA(ctx, cudaMallocHost(reinterpret_cast<void**>(&md->hEnergy), sizeof(double) * REC * (size_t)c));
+    md->energyCap = c;
     return MRMD_OK;
 }
 
@@ -568,7 +571,7 @@ int md_run(mrmd_ctx* ctx, mrmd_md* md, int64_t nsteps, double* out, int cols)
         rc = md_rebuild(ctx, md);
         if (rc == MRMD_OK) rc = mrmd_atoms_set_force(ctx, a, a->numLocal + a->numGhost, 0.0);
         if (rc == MRMD_OK) rc = md_forces(ctx, md, rec + REC * nsteps);  // scratch slot
-        md->forceValid = true;
+        md->forceValid = rc == MRMD_OK;
     }
     // the previous step's record, for the kinetic energy its post-kick yields;
     // none for the first step of a run (the last run's end recorded it)

@@ -322,6 +322,7 @@ int CellList::build(mrmd_ctx* ctx, const double* pos4, int64_t n, const CellGrid
         dfree(unordered);
         cellOf = sorted = unordered = nullptr;
         spos = nullptr;
+        capN = 0;  // until all four are there
         const int64_t c = n + n / 4 + 64;
         MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&unordered), sizeof(int32_t) * (size_t)c));
         MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&cellOf), sizeof(int32_t) * (size_t)c));
@@ -373,6 +374,7 @@ void CellList::release()
     capN = capCells = 0;
 }
 
+// (A failed allocation leaves an empty list: no rows, no capacity.)
 static int ensure_list_storage(mrmd_ctx* ctx, mrmd_nlist* nl, int64_t rows, int64_t maxNeighbors)
 {
     const int64_t stride = div_up(rows > 0 ? rows : 1, 32) * 32;
@@ -380,6 +382,7 @@ static int ensure_list_storage(mrmd_ctx* ctx, mrmd_nlist* nl, int64_t rows, int6
     {
         dfree(nl->counts);
         nl->counts = nullptr;
+        nl->rows = nl->rowsCapacity = nl->totalPairs = 0;
         const int64_t c = rows + rows / 8 + 64;
         MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&nl->counts), sizeof(int32_t) * (size_t)c));
         nl->rowsCapacity = c;
@@ -389,6 +392,7 @@ static int ensure_list_storage(mrmd_ctx* ctx, mrmd_nlist* nl, int64_t rows, int6
     {
         dfree(nl->nbrs);
         nl->nbrs = nullptr;
+        nl->rows = nl->nbrsCapacity = nl->totalPairs = 0;
         MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&nl->nbrs), sizeof(int32_t) * (size_t)need));
         nl->nbrsCapacity = need;
     }

@@ -106,3 +106,51 @@ def test_bounds_build_reports_bad_real_atoms_and_molecules():
                        text=True, timeout=600)
     assert r.returncode == 0, r.stdout + r.stderr
     assert r.stdout.count("reported: MRMD_ERR_BOUNDS") == 3 and r.stdout.strip().endswith("ok"), r.stdout
+
+
+def test_a_list_that_could_not_grow_is_empty(M):
+    """A build with room for 2^40 neighbours a row fails; the list has no rows
+    then, and the next build allocates anew."""
+    pos = np.random.default_rng(3).uniform(0, 6.0, (500, 3))
+    a = M.Atoms.from_arrays(pos)
+    vl, lj = M.HalfVerletList(), M.LennardJones(1.0, 1.0, 1.0, 0.7)
+    args = (a, 0, 500, 1.3, 1.0, [0.0] * 3, [6.0] * 3)
+    vl.build(*args, 60)
+    pairs = vl.total_pairs
+    a.setForce(0.0)
+    lj.apply(a, vl)
+    energy = lj.getEnergy()
+    with pytest.raises(M.MrmdError) as e:
+        vl.build(*args, 1 << 40)
+    assert e.value.code == -2  # MRMD_ERR_OOM
+    assert vl.total_pairs == 0 and len(vl.download()[0]) == 0
+    lj.apply(a, vl)
+    assert lj.getEnergy() == 0.0
+    vl.build(*args, 60)
+    a.setForce(0.0)
+    lj.apply(a, vl)
+    assert vl.total_pairs == pairs and abs(lj.getEnergy() - energy) <= 1e-12 * abs(energy)
+
+
+@pytest.mark.parametrize("kind", ["md", "adress"])
+def test_a_run_too_long_to_record_leaves_the_system(M, kind):
+    """2^45 steps have no room for their energies; a run after that is the one
+    of a fresh system."""
+    from test_gpu_md import fcc, mb_velocities
+
+    pos, L = fcc(6)
+    vel = mb_velocities(len(pos), 0.728, 3)
+
+    def system():
+        if kind == "md":
+            return M.LJSystem(pos, vel, [0, 0, 0], [L] * 3, precision=M.PREC_MIXED)
+        return M.AdResSSystem(pos, vel, [0, 0, 0], [L] * 3, [L / 2] * 3, 3.0, 2.0, capping_distance=0.7842,
+                              precision=M.PREC_MIXED, composed=True)
+
+    a, b = system(), system()
+    with pytest.raises(M.MrmdError) as e:
+        a.run(1 << 45, energies=False)
+    assert e.value.code == -2  # MRMD_ERR_OOM
+    ea, eb = a.run(12), b.run(12)
+    np.testing.assert_allclose(ea, eb, rtol=1e-9)
+    np.testing.assert_allclose(a.state()[0], b.state()[0], rtol=0, atol=1e-9)
