@@ -14,6 +14,7 @@
 #include <cmath>
 
 #include "common.cuh"
+#include "list_grid.cuh"
 #include "nlist_impl.cuh"
 #include "lj_tile.cuh"
 
@@ -33,8 +34,7 @@ CellGrid make_grid(const double* gridMin, const double* gridMax, double delta, i
     for (int d = 0; d < 3; ++d)
     {
         const double L = gridMax[d] - gridMin[d];
-        int64_t c = (int64_t)std::floor(L / delta);
-        if (c < 1) c = 1;
+        const int64_t c = cells_per_axis(L, delta);
         n[d] = (int)c;
         mn[d] = gridMin[d];
         rdx[d] = (double)c / L;
@@ -48,7 +48,7 @@ CellGrid make_grid(const double* gridMin, const double* gridMax, double delta, i
     g.h = make_float3((float)(1.0 / rdx[0]), (float)(1.0 / rdx[1]), (float)(1.0 / rdx[2]));
     g.margin = (float)std::ldexp(extent, -20);
     g.n = make_int3(n[0], n[1], n[2]);
-    g.ncell = (int64_t)n[0] * n[1] * n[2];
+    g.ncell = cell_count(n[0], n[1], n[2]);
     g.extent = extent;
     return g;
 }
@@ -56,9 +56,7 @@ CellGrid make_grid(const double* gridMin, const double* gridMax, double delta, i
 CellGrid make_list_grid(const double* gridMin, const double* gridMax, double delta, int64_t n)
 {
     const CellGrid g = make_grid(gridMin, gridMax, delta, 2);
-    // (per axis first: the product of three counts may pass 2^63)
-    const double cells = (double)g.n.x * (double)g.n.y * (double)g.n.z;
-    return cells <= 8.0 * (double)n + 1048576.0 ? g : make_grid(gridMin, gridMax, delta, 1);
+    return half_radius_cells(g.ncell, n) ? g : make_grid(gridMin, gridMax, delta, 1);
 }
 
 // Bits of v spread to every third position (v < 2^10).
@@ -307,13 +305,13 @@ int CellList::build(mrmd_ctx* ctx, const double* pos4, int64_t n, const CellGrid
                     int32_t* nonfinite)
 {
     g = grid;
+    if (n > INT32_MAX || g.ncell > INT32_MAX) return set_error(ctx, MRMD_ERR_CAPACITY, "too many particles or cells");
     // Morton keys need at most 10 bits per axis; the key range is then a
     // power-of-two cube covering the grid
     int bits = 0;
     while ((1 << bits) < std::max(g.n.x, std::max(g.n.y, g.n.z))) ++bits;
     if (bits > 10) morton = false;
     const int64_t nkeys = morton ? (int64_t)1 << (3 * bits) : g.ncell;
-    if (n > INT32_MAX || g.ncell > INT32_MAX) return set_error(ctx, MRMD_ERR_CAPACITY, "too many particles or cells");
     if (n + 1 > capN)
     {
         dfree(cellOf);
@@ -335,6 +333,7 @@ int CellList::build(mrmd_ctx* ctx, const double* pos4, int64_t n, const CellGrid
         // one allocation: cell starts, then the scatter's cursors
         dfree(cellStart);
         cellStart = nullptr;
+        capCells = 0;
         const int64_t c = nkeys + 1;
         MRMD_TRY(dmalloc(ctx, reinterpret_cast<void**>(&cellStart), 2 * sizeof(int32_t) * (size_t)c));
         capCells = c;
