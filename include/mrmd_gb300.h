@@ -516,6 +516,9 @@ const mrmd_ghost_layer* mrmd_md_ghosts(const mrmd_md* md);
  * tile build could not fit (the rebuild then made the int32 rows and their
  * tile form), [5] rebuilds so far that needed that second path. */
 int mrmd_md_tile_stats(const mrmd_md* md, int64_t* out6);
+/* Threads that shared a row in the last one-pass tile build (1 or 4); 0 when
+ * the last rebuild made the int32 rows. */
+int mrmd_md_tile_row_threads(const mrmd_md* md, int64_t* out);
 /* The stepper's current neighbour pairs as canonical keys a * 2^32 + b of
  * unordered pairs of original atom indices (a < b; ghosts mapped to their
  * real atom), one key per list entry as the pair kernel reads it (the mixed

@@ -799,11 +799,13 @@ class LJSystem:
         """Mixed form: tiles, members of the largest tile, whether the pair
         kernel reads shared-memory tiles (True) or gathers through the cache,
         members of all tiles, the tiles the last rebuild's one-pass build could
-        not fit, and the rebuilds so far that needed the int32 rows."""
-        out = np.zeros(6, dtype=np.int64)
+        not fit, the rebuilds so far that needed the int32 rows, and the threads
+        that shared a row in the last one-pass build (0: it made int32 rows)."""
+        out, threads = np.zeros(6, dtype=np.int64), np.zeros(1, dtype=np.int64)
         self.ctx.lib.mrmd_md_tile_stats(self.h, _ip(out))
+        self.ctx.lib.mrmd_md_tile_row_threads(self.h, _ip(threads))
         return dict(tiles=int(out[0]), max_members=int(out[1]), tiled=bool(out[2]), members=int(out[3]),
-                    unfit_tiles=int(out[4]), two_pass_builds=int(out[5]))
+                    unfit_tiles=int(out[4]), two_pass_builds=int(out[5]), row_threads=int(threads[0]))
 
     def pair_keys(self):
         """Sorted canonical keys a * 2^32 + b (a < b, original atom indices) of

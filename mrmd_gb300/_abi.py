@@ -279,6 +279,7 @@ SIGNATURES = {
     "mrmd_md_nlist": (P(NListS), [_v]),
     "mrmd_md_ghosts": (P(GhostLayerS), [_v]),
     "mrmd_md_tile_stats": (_i, [_v, c_int64_p]),
+    "mrmd_md_tile_row_threads": (_i, [_v, c_int64_p]),
     "mrmd_md_pair_keys": (_i, [_v, _v, c_int64_p, _i64, c_int64_p]),
     "mrmd_batch_pair_keys": (_i, [_v, _v, _i64, c_int64_p, _i64, c_int64_p]),
     "mrmd_grid_sync_selftest": (_i, [_v, C.c_int32, C.c_int32, C.c_double]),

@@ -83,7 +83,7 @@ struct TileList
     int64_t totalMembers = 0;  // members of all tiles after the last build
     bool valid = false;      // every tile fits TILE_CAP
     bool sliced = false;      // the last one-pass build had several threads a row
-    bool longSlices = false;  // such a build did not fit once: one thread a row from then on
+    bool longSlices = false;  // rows were too long for that once: one thread a row from then on
     int64_t unfitTiles = 0;     // tiles the last one-pass build could not fit
     int64_t twoPassBuilds = 0;  // builds that made the int32 rows and their tile form
     void release();

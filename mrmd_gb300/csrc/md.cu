@@ -777,6 +777,14 @@ int mrmd_md_tile_stats(const mrmd_md* md, int64_t* out6)
     return MRMD_OK;
 }
 
+int mrmd_md_tile_row_threads(const mrmd_md* md, int64_t* out)
+{
+    if (!md || !out) return MRMD_ERR_ARG;
+    const TileList& t = md->tiles;
+    *out = md->cfg.precision != MRMD_PREC_MIXED || !t.valid || t.unfitTiles || md->cfg.tileBuild ? 0 : t.sliced ? 4 : 1;
+    return MRMD_OK;
+}
+
 }  // extern "C"
 
 namespace

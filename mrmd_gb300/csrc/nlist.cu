@@ -495,12 +495,14 @@ int build_split_list(mrmd_ctx* ctx, mrmd_nlist* nearList, mrmd_nlist* farList, c
         MRMD_TRY(read_flags(ctx, maxCount, &h));
         if (hMax[2]) return set_error(ctx, MRMD_ERR_NONFINITE, "non-finite particle position at the list build");
         if (tiles) tiles->unfitTiles = 0;
-        if (tiles && onePass && rows > 0 && hMax[4] != 0 && tiles->sliced)
+        if (tiles && rows > 0 && hMax[6] != 0)
         {
+            // rows too long for the slices of several threads (a tile that did
+            // not fit its tables, hMax[4], is left to the int32 rows below)
             tiles->longSlices = true;
             if (hMax[0] <= capN && hMax[1] <= capF && attempt < 3) continue;
         }
-        if (tiles && rows > 0 && hMax[4] != 0 && hMax[0] <= capN && hMax[1] <= capF)
+        if (tiles && rows > 0 && (hMax[4] != 0 || hMax[6] != 0) && hMax[0] <= capN && hMax[1] <= capF)
         {
             // a tile did not fit the one-pass build: the int32 rows, then
             // their tile form

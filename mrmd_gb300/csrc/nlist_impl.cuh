@@ -157,13 +157,15 @@ __device__ __forceinline__ bool candidate_kept(const double4* __restrict__ pos, 
 // with one copy.
 struct ListFlags
 {
-    int32_t i[6];  // longest near and far rows, non-finite position, largest tile, tiles that did not fit, members
+    // longest near and far rows, non-finite position, largest tile, tiles that
+    // did not fit, members, tiles with a slice that did not fit
+    int32_t i[8];
     unsigned long long totals[2];  // entries of all near and all far rows
 };
 
 __host__ __device__ inline unsigned long long* list_totals(int32_t* flags)
 {
-    return reinterpret_cast<unsigned long long*>(flags + 6);
+    return reinterpret_cast<unsigned long long*>(flags + 8);
 }
 
 // The warps' entry counts into totals[0] (near or only rows) and [1] (far).

@@ -175,7 +175,8 @@ __device__ __forceinline__ void chunk_remap(uint4* __restrict__ out, int64_t row
 }
 
 // flags: [0], [1] longest near / far row, [3] largest member count, [4] tiles
-// that did not fit (their rows are incomplete), [5] members of all tiles.
+// that did not fit (their rows are incomplete), [5] members of all tiles, [6]
+// tiles with a row too long for its slices.
 // Four blocks per SM (64 registers): the scan is bound by the latency of its
 // candidate loads; three blocks of 72 registers ran 14% slower.
 //
@@ -372,7 +373,8 @@ __global__ void __launch_bounds__(TILE_ROWS * H, H == 1 ? 4 : 1) k_tile_list(
         memberCount[tile] = total < TILE_CAP ? total : TILE_CAP;
         atomicMax(&flags[3], total);
         atomicAdd(&flags[5], total);
-        if (total > TILE_CAP || longS) atomicAdd(&flags[4], 1);
+        if (total > TILE_CAP) atomicAdd(&flags[4], 1);
+        if (longS) atomicAdd(&flags[6], 1);
     }
     __syncthreads();
     if (total > TILE_CAP || longS || !live) return;
