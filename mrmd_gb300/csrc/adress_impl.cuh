@@ -4,6 +4,7 @@
 #pragma once
 
 #include <cmath>
+#include <limits>
 
 #include "common.cuh"
 #include "lj_impl.cuh"
@@ -41,8 +42,9 @@ __device__ __forceinline__ void slab_eval(const SlabDev& s, double x, double& la
     // weighting_function/Slab.hpp:161-187 (+ setSmoothWeightInHY :96-120).
     // Outside the hybrid regions this is one FP64 operation: the comparisons
     // are integer ones on the bits of |dx| (a NaN's lie above infinity's and
-    // go on to the weights, like the FP64 comparisons'), and k and outer are
-    // the host's, of the same roundings.  The gradient's dx / |dx| is a sign.
+    // go on to the weights, like the FP64 comparisons'; to_slab has atHalf and
+    // outer such that those with a NaN fail too), and k and outer are the host's,
+    // of the same roundings.  The gradient's dx / |dx| is a sign.
     const double dx = x - s.cx;
     const double absDx = fabs(dx);
     const long long b = __double_as_longlong(absDx);
@@ -96,6 +98,14 @@ inline SlabDev to_slab(const mrmd_slab* s)
     d.hy = s->hybridRegionDiameter;
     d.outer = d.atHalf + d.hy;
     d.k = 3.141592653589793238462643383279502884 / (2.0 * d.hy);
+    // a NaN diameter: no |dx| lies below atHalf or above outer, and the weights
+    // are NaN (slab_eval compares bits: a positive NaN's lie above all others)
+    if (std::isnan(d.outer)) d.outer = std::numeric_limits<double>::quiet_NaN();
+    if (std::isnan(d.atHalf))
+    {
+        d.atHalf = -1.0;
+        d.k = std::numeric_limits<double>::quiet_NaN();
+    }
     d.exponent = 2 * s->nu;
     d.abrupt = s->interfaceType == 1;
     return d;

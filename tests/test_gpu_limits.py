@@ -154,3 +154,28 @@ def test_a_run_too_long_to_record_leaves_the_system(M, kind):
     ea, eb = a.run(12), b.run(12)
     np.testing.assert_allclose(ea, eb, rtol=1e-9)
     np.testing.assert_allclose(a.state()[0], b.state()[0], rtol=0, atol=1e-9)
+
+
+@pytest.mark.parametrize("interface", [0, 1])
+@pytest.mark.parametrize("at,hy", [(np.nan, 10.0), (-np.nan, 10.0), (np.nan, np.inf), (-np.inf, np.inf), (np.inf, 10.0),
+                                   (30.0, np.inf), (-5.0, 10.0)])
+def test_slab_diameters_out_of_the_ordinary(M, orc, at, hy, interface):
+    """Weights of slabs with NaN, infinite and negative diameters (a hybrid width
+    that is not positive is refused) are the reference's: NaN compares with
+    nothing, so that a smooth slab has NaN weights (not ones) and an abrupt one
+    weights of one."""
+    apos = np.random.default_rng(2).uniform(0, 120, (500, 3))
+    mo = orc.Molecules(500)
+    mo.atomsOffset[:], mo.numAtoms[:], mo.numLocal = np.arange(500), 1, 500
+    ao = orc.Atoms.from_positions(apos)
+    ao.relativeMass[:500] = 1.0
+    with np.errstate(all="ignore"):
+        orc.update_molecules(mo, ao, orc.slab([60, 12, 12], at, hy, 1, interface))
+    m, a = M.Molecules(500), M.Atoms.from_arrays(apos)
+    m.upload(500, 0, pos=apos, force=np.zeros((500, 3)), lambda_=np.zeros(500), modulated_lambda=np.zeros(500),
+             grad_lambda=np.zeros((500, 3)), atoms_offset=np.arange(500), num_atoms=np.ones(500))
+    M.UpdateMolecules.update(m, a, M.Slab([60, 12, 12], at, hy, 1, interface))
+    d = m.download(500)
+    np.testing.assert_allclose(d["lambda_"], mo.lambda_[:500], rtol=1e-13, atol=1e-15, equal_nan=True)
+    np.testing.assert_allclose(d["modulatedLambda"], mo.modulatedLambda[:500], rtol=1e-13, atol=1e-15, equal_nan=True)
+    np.testing.assert_allclose(d["gradLambda"][:, 0], mo.gradLambda[:500, 0], rtol=1e-12, atol=1e-15, equal_nan=True)
