@@ -431,14 +431,15 @@ __global__ void k_ghost_update(double4* __restrict__ pos, const int32_t* __restr
     }
 }
 
+template <int AHEAD>
 __global__ void k_ghost_reduce(double4* __restrict__ force, const int32_t* __restrict__ start,
                                const int32_t* __restrict__ list, int64_t nLocal, int64_t nGhost)
 {
     // communication/AccumulateForce.cpp:25-47, gathered per real atom in
     // ascending ghost order (the serial order of the reference loop).  Bound
-    // by its dependent loads: a few ghosts' entries, then their forces, are
-    // loaded at a time (32,000 atoms: 13.2 -> 7.3 us).
-    constexpr int AHEAD = 4;
+    // by its dependent loads in a small system: AHEAD ghosts' entries, then their
+    // forces, are loaded at a time (32,000 atoms: 13.2 -> 7.3 us).  A large one
+    // has the warps to wait, and four ghosts' registers take half of them away.
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nLocal;
          i += (int64_t)gridDim.x * blockDim.x)
     {
@@ -733,8 +734,18 @@ int mrmd_ghost_reduce_force(mrmd_ctx* ctx, const mrmd_ghost_layer* g, mrmd_atoms
     if (g->numLocal != a->numLocal || g->numGhost != a->numGhost)
         return set_error(ctx, MRMD_ERR_STATE, "ghost layer does not match atoms (recreate ghosts)");
     if (a->numGhost == 0 || a->numLocal == 0) return MRMD_OK;
-    k_ghost_reduce<<<grid_for(ctx, a->numLocal, TB), TB, 0, ctx->stream>>>(
-        reinterpret_cast<double4*>(a->force), g->ghostStart, g->ghostList, a->numLocal, a->numGhost);
+    auto launch = [&](auto kernel) {
+        kernel<<<grid_for(ctx, a->numLocal, TB), TB, 0, ctx->stream>>>(
+            reinterpret_cast<double4*>(a->force), g->ghostStart, g->ghostList, a->numLocal, a->numGhost);
+    };
+    // us of the call with four ghosts ahead / one, fluid in cell order: 4,000
+    // atoms 13.6 / 14.0, 32,000 13.5 / 13.3, 128,000 15.8 / 14.8, 1,000,000 25.2
+    // / 18.2, 4,000,000 45.4 / 22.8; gas of density 0.02 in random order: 32,000
+    // 13.1 / 13.9, 128,000 15.7 / 14.2, 1,000,000 32.5 / 19.8, 4,000,000 73.9 / 31.5
+    if (a->numLocal < 400 * (int64_t)ctx->numSMs)
+        launch(k_ghost_reduce<4>);
+    else
+        launch(k_ghost_reduce<1>);
     MRMD_TRY(after_launch(ctx, "ghost_reduce"));
     return finish(ctx, "ghost_reduce");
 }
