@@ -212,6 +212,11 @@ int lj_mixed_half(mrmd_ctx* ctx, const float4* hi, const float4* lo, const mrmd_
     //      87,808         80 /  73 /  71 /  83   (125)
     //     256,000        185 / 158 / 161 / 204   (327)
     //   4,000,000       2112 / 2030 / 2235 / 2958   (4536)
+    // With rows of a few entries (a gas) a second lane of a large system has
+    // nothing to do: us of the call with 1 / 2 lanes at random placement, 256,000
+    // atoms and 0.2 / 0.9 / 2.3 / 4.6 / 9.2 entries a row 44 / 54, 52 / 66, 66 /
+    // 66, 78 / 79, 103 / 102, 1,000,000 atoms 106 / 151, 127 / 176, 152 / 192,
+    // 191 / 217, 274 / 287 (139, 178, 238, 315, 460 before)
     const int64_t sms = ctx->numSMs;
     if (n < 40 * sms)
     {
@@ -221,9 +226,13 @@ int lj_mixed_half(mrmd_ctx* ctx, const float4* hi, const float4* lo, const mrmd_
     {
         MX_LANES(4);
     }
-    else
+    else if (nl->totalPairs >= 4 * n)
     {
         MX_LANES(2);
+    }
+    else
+    {
+        MX_LANES(1);
     }
 #undef MX_LANES
     return after_launch(ctx, "lj_mixed_half");
