@@ -432,10 +432,23 @@ int ljig_run_async(mrmd_ctx* ctx, mrmd_ljig* s, mrmd_molecules* m, const mrmd_nl
         // entry evaluated, before): 9,216 molecules 81 / 53 / 42 / 44 (103),
         // 34,560 91 / 64 / 66 / 78 (102), 117,600 103 / 102 / 114 / 164
         // (140), 460,800 533 / 485 / 545 / 795 (704), 156,800 of three sites
-        // 1088 / 644 / 594 / 610 (1260)
+        // 1088 / 644 / 594 / 610 (1260): two lanes there too, as the line is the
+        // single-site one.  A large system with less than one pair of sites a
+        // molecule (a gas) has nothing for a second lane: us of the action with
+        // 1 / 2 lanes, FP64 and mixed, 100,000 molecules and 0.2 entries a row
+        // 38 / 50 and 40 / 52 (41 and 40), 0.9 entries 57 / 56 and 53 / 54 (63
+        // and 53), 400,000 and 0.2 75 / 112 and 79 / 114 (88 and 82), 0.9 125 /
+        // 150 and 115 / 140 (149 and 127), 2.3 200 / 211 and 170 / 187 (248 and
+        // 191); with three sites 1 lane is the slower one
+        const double sites = (double)a->numLocal / (double)A.nMol;
+        const bool gas = (double)nl->totalPairs * sites * sites < (double)A.nMol;
         if (A.nMol < 130 * (int64_t)ctx->numSMs)
         {
             LJIG_LANES(4);
+        }
+        else if (gas && A.nMol >= 400 * (int64_t)ctx->numSMs)
+        {
+            LJIG_LANES(1);
         }
         else
         {

@@ -33,3 +33,42 @@ def test_mixed_half_short_rows(M, orc, n, rho, pred):
     rms = np.sqrt((Fo ** 2).sum(1).mean())
     assert np.linalg.norm(F - Fo, axis=1).max() <= 1e-6 * rms
     assert abs(E - Eo) <= 1e-7 * abs(Eo)
+
+
+# One lane a molecule from 60,800 of them (400 per SM on 152) with less than
+# one pair of sites each up: 0.9 entries a row, and 8 pairs of sites with three.
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("n,sites", [(60799, 1), (60801, 1), (60801, 3)])
+def test_lj_ideal_gas_short_rows(M, orc, n, sites, prec):
+    """Forces before the fold-back and the energy against the oracle, by the
+    bars of the FP64 and the mixed form."""
+    from conftest import assert_fp64_forces
+    from test_gpu_adress import adress_system, upload_molecules
+
+    mo, ao, corr, sd, slab, (rc, skin, _) = adress_system(orc, n, (310.0, 100.0, 100.0), 17, sites)
+    co, no = orc.build_half_list(mo.pos, mo.numLocal + mo.numGhost, 0, mo.numLocal, rc + skin, sd.minGhostCorner,
+                                 sd.maxGhostCorner, 1.0, 64)
+    assert 0.5 * n < co.sum() < n
+    ao.force[:] = 0
+    mo.force[:] = 0
+    Eo = orc.LJIdealGas(0.8, rc, 1.0, 1.0, True).run(mo, co, no, ao)
+    na, nm = ao.n, mo.numLocal + mo.numGhost
+    a = M.Atoms.from_arrays(ao.pos[:na], relative_mass=ao.relativeMass[:na], capacity=ao.capacity)
+    a.numLocalAtoms, a.numGhostAtoms = ao.numLocal, ao.numGhost
+    m = upload_molecules(M, mo, mo.numLocal, mo.numGhost)
+    m.setForce(0.0)
+    a.setForce(0.0)
+    vl = M.HalfVerletList()
+    vl.build(m, 0, mo.numLocal, rc + skin, 1.0, sd.minGhostCorner[:], sd.maxGhostCorner[:], 60)
+    ig = M.LJ_IdealGas(0.8, rc, 1.0, 1.0, True)
+    E = ig.run(m, vl, a, M.PREC_FP64 if prec == "fp64" else M.PREC_MIXED)
+    F, Fm = a.getForce(), m.download()["force"]
+    Fo, Fmo = ao.force[:na], mo.force[:nm]
+    if prec == "fp64":
+        assert_fp64_forces(F, Fo)
+        assert_fp64_forces(Fm, Fmo)
+        assert abs(E - Eo) <= 1e-10 * abs(Eo)
+    else:
+        rms = np.sqrt((Fo ** 2).sum(1).mean())
+        assert np.linalg.norm(F - Fo, axis=1).max() <= 1e-6 * rms
+        assert abs(E - Eo) <= 1e-7 * abs(Eo)
