@@ -127,16 +127,13 @@ __device__ __forceinline__ void pre_body(const BDev& B, int rebuild, int64_t tid
                         dz = (float)(x.z - R.gmn[2]) - r0.z;
             m2 = fmaxf(m2, __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz))));
         }
-        if (rebuild)
-        {
 #pragma unroll
-            for (int d = 0; d < 3; ++d)
-            {
-                double c = coord(x, d);
-                if (R.mx[d] <= c) c = __dsub_rn(c, R.L[d]);
-                if (c < R.lo[d]) c = __dadd_rn(c, R.L[d]);
-                set_coord(x, d, c);
-            }
+        for (int d = 0; d < 3; ++d)
+        {
+            double c = coord(x, d);
+            if (R.mx[d] <= c) c = __dsub_rn(c, R.L[d]);
+            if (c < R.lo[d]) c = __dadd_rn(c, R.L[d]);
+            set_coord(x, d, c);
         }
         B.pos[i] = x;
         B.vel[i] = v;

@@ -68,9 +68,8 @@ inline unsigned grid_for(const mrmd_ctx* ctx, int64_t n, int block, int ctasPerS
     return (unsigned)(need < cap ? need : cap);
 }
 
-// Exclusive scan of int64 values (in and out may alias).  total (device,
-// may be null) receives the sum.  Uses ctx scratch.
-int scan_exclusive_i64(mrmd_ctx* ctx, const int64_t* in, int64_t* out, int64_t n, int64_t* total);
+// Exclusive scan (in and out may alias).  total (device, may be null) receives
+// the sum.  Uses ctx scratch.
 int scan_exclusive_i32(mrmd_ctx* ctx, const int32_t* in, int32_t* out, int64_t n, int32_t* total);
 }  // namespace mrmd_impl
 

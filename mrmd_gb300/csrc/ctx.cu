@@ -270,14 +270,6 @@ static size_t scan_scratch_bytes(int64_t n)
     return b + 1024;
 }
 
-int scan_exclusive_i64(mrmd_ctx* ctx, const int64_t* in, int64_t* out, int64_t n, int64_t* total)
-{
-    char* s = static_cast<char*>(
-        grow_buffer(ctx, ctx->scanScratch, ctx->scanScratchBytes, scan_scratch_bytes<int64_t>(n)));
-    if (!s) return MRMD_ERR_OOM;
-    return scan_rec<int64_t>(ctx, in, out, n, total, s);
-}
-
 int scan_exclusive_i32(mrmd_ctx* ctx, const int32_t* in, int32_t* out, int64_t n, int32_t* total)
 {
     char* s = static_cast<char*>(
