@@ -1143,7 +1143,18 @@ class DiffSystem:
         c.tfSmoothingSigma, c.tfSmoothingRange = 1.0, 1.0
         c.tfSampleInterval, c.tfUpdateInterval = 1, int(steps) + 1
         # several lanes per row where one would leave the GPU with few warps
-        # (the rows of the coarse-grained region are empty)
+        # (the rows of the coarse-grained region are empty); a caller of
+        # mrmd_diff_create chooses them itself.  ms of a gradient over 20 steps
+        # with 1 / 2 / 4 / 8 lanes on 152 SMs (slab 0.3 of the box):
+        #               FP64                        mixed
+        #   5,000    6.6 /  5.2 /  4.5 /  4.3    5.8 /  4.9 /  4.4 /  4.3
+        #  20,000    6.6 /  5.2 /  4.8 /  4.7    5.8 /  4.9 /  4.5 /  4.4
+        #  40,000    7.9 /  6.9 /  6.8 /  7.3    6.5 /  5.8 /  5.5 /  5.7
+        #  65,000    9.6 /  8.4 /  8.5 /  9.1    7.5 /  6.8 /  6.6 /  6.9
+        # 130,000   13.1 / 12.9 / 12.6 / 14.4    9.6 /  9.2 /  9.3 /  9.9
+        # 200,000   19.2 / 16.9 / 17.1 / 20.0   12.4 / 12.0 / 12.0 / 13.1
+        # 300,000   23.4 / 22.2 / 23.5 / 28.0   15.5 / 15.7 / 16.0 / 18.0
+        # 600,000   39.8 / 39.9 / 42.8 / 51.9   26.4 / 26.7 / 27.9 / 31.9
         self.threads_per_row = 8 if self.n < 20000 else 4 if self.n < 200000 else 1
         c.tuning = _tuning_struct(dict(threads_per_row=self.threads_per_row, block_size=128,
                                        rebuild_interval=rebuild_interval, sort_every=0, graph_steps=0))

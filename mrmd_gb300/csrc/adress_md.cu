@@ -166,16 +166,17 @@ int ad_capture(mrmd_ctx* ctx, mrmd_adress* s, int64_t st0, int64_t count, int64_
 }
 // Lanes per row of the one-replica engine: several where one lane per row
 // would leave the GPU with few warps and long serial rows (rows outside the
-// slab are empty), one where there are rows enough.  us per step with
-// 1 / 2 / 4 / 8 lanes (slab half the box, fluid after 300 steps):
-//                 FP64                       mixed
-//      5,184   211 / 141 / 102 /  82     143 / 104 /  80 /  69
-//     12,960   186 / 133 / 104 /  98     141 / 106 /  85 /  75
-//     34,560   169 / 123 / 107 / 117     133 / 100 /  86 /  90
-//    129,600   235 / 217 / 206 / 248     154 / 128 / 135 / 170
-//    276,480   377 / 323 / 340 / 448     195 / 198 / 206 / 287
-//    504,600   569 / 537 / 584 / 764
-//    985,680   944 / 969 / 1060 / 1417   582 / 581 / 642 / 934
+// slab are empty), one where there are rows enough (the lines are those of 152
+// SMs).  us per step with 1 / 2 / 4 / 8 lanes (slab half the box, fluid after
+// 300 steps):
+//                 FP64                          mixed
+//      5,184    131 /   77 /   52 /   42     85 /  59 /  44 /  37
+//     12,960    128 /   87 /   65 /   65     85 /  59 /  45 /  41
+//     34,560    151 /  105 /   98 /  104     92 /  65 /  56 /  58
+//    129,600    280 /  245 /  237 /  273    122 / 113 / 109 / 123
+//    276,480    493 /  443 /  457 /  545    235 / 201 / 207 / 251
+//    491,144    756 /  717 /  756 /  923    344 / 325 / 349 / 425
+//    996,632   1377 / 1373 / 1475 / 1808    619 / 622 / 684 / 829
 int row_lanes_for(int64_t n, bool mixed)
 {
     if (n < 20000) return 8;
@@ -224,8 +225,10 @@ int mrmd_adress_create(mrmd_ctx* ctx, mrmd_adress** out, const mrmd_adress_confi
         bc.initialMaxNeighbors = cfg->maxNeighbors > 0 ? cfg->maxNeighbors : 0;
         // cell sort every 5th rebuild; graphs of 5 rebuild intervals; from a
         // million molecules the steps between rebuilds as one persistent
-        // launch (4,000,000 molecules: 2.01 against 2.33 ms per step mixed,
-        // 5.13 against 5.25 FP64; 34,560: 6% slower)
+        // launch.  us per step, persistent / launches, mixed and FP64 (slab a
+        // quarter of the box, after 300 steps): 504,600 molecules 320 / 288 and
+        // 525 / 511, 985,680 441 / 478 and 865 / 861, 2,000,000 856 / 990 and
+        // 1622 / 1760, 4,000,000 1636 / 1922 and 3107 / 3442
         const int lanes = row_lanes_for(n, cfg->precision == MRMD_PREC_MIXED);
         bc.tuning.threadsPerRow = lanes;
         bc.tuning.blockSize = lanes == 8 ? 256 : 128;  // blocks of a multiple of 32 rows (rowOrderEnergy)

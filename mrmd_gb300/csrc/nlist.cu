@@ -289,10 +289,15 @@ int build_rows(mrmd_ctx* ctx, const CellList& cl, const double* pos4, int64_t be
     };
     // lanes per row: several where one lane per row leaves the SMs with few
     // warps that wait for their loads; one for large systems, where the
-    // ballots cost more than the idle lanes.  us per launch of the half list
-    // with 1 / 2 / 4 / 8 / 16 lanes: 32,000 atoms 56 / 43 / 28 / 35 / 46,
-    // 256,000 atoms 126 / 154 / 159 / 198 / 284 (before the cells out of reach
-    // were skipped)
+    // ballots cost more than the idle lanes.  us of the whole half-list call
+    // (binning and read-back are 57 of them) with 1 / 4 / 8 / 16 lanes:
+    //                density 0.8442               density 0.05
+    //     4,000   110 /  74 /  62 /   62     62 /  60 /  59 /   59
+    //     9,728    99 /  73 /  64 /   63     63 /  61 /  60 /   60
+    //    32,000   103 /  74 /  84 /   97     64 /  61 /  71 /   85
+    //    97,280   113 / 113 / 125 /  172     72 /  85 / 101 /  146
+    //   256,000   159 / 198 / 246 /  359     95 / 134 / 189 /  291
+    // 1,000,000   381 / 580 / 788 / 1311    210 / 381 / 606 / 1028
     const int64_t rows = end - begin, sms = ctx->numSMs;
     if (rows < 64 * sms) launch(k_build_list<FULL, SPLIT, 8>, 8);
     else if (rows < 640 * sms) launch(k_build_list<FULL, SPLIT, 4>, 4);
